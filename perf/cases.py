@@ -3,7 +3,8 @@ Model.run_with_tensors(), and the eager kernels of aitemplate_b200.kernels, over
 that inference programs call them with. (There is no training here: the library runs forward passes only.)
 
 listed() names a fixed set, draw() gives more of the same ranges; prepare() makes what a program holds before the call,
-run() is one call, work() what it cannot do without, tolerance() how far two correct results may lie apart.
+run() is one call, work() what it cannot do without, tolerance() how far two correct results may lie apart, exact()
+what the call returns when all of it is computed in 64 bits.
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ import math
 import tempfile
 
 import torch
+import torch.nn.functional as F
 
 from aitemplate_b200 import kernels
 from aitemplate_b200.compiler import compile_model
@@ -112,7 +114,7 @@ def _model(output, name):
         return compile_model(output, detect_target(), workdir, name)
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
     gen = torch.Generator(device="cuda").manual_seed(seed)
     kind = case["kind"]
     dtype = _DTYPES[case.get("dtype", "fp16")]
@@ -132,11 +134,7 @@ def prepare(case, seed):
         for ln in ("ln1", "ln2"):
             params[ln + "_gamma"] = uniform(_HIDDEN, lo=0.5, hi=1.5)
             params[ln + "_beta"] = normal(_HIDDEN, scale=0.1)
-        _, y = workloads.build_bert_layer(batch, seq)
-        model = _model(y, "bert_layer")
-        model.set_many_constants_with_tensors({n: params[k] for n, k in workloads.BERT_PARAM_NAMES.items()})
-        return {"case": case, "model": model, "params": params, "inputs": {"hidden_states": normal(batch, seq, _HIDDEN)},
-                "outputs": {"output_0": torch.empty((batch, seq, _HIDDEN), dtype=dtype, device="cuda")}}
+        return {"params": params, "inputs": {"hidden_states": normal(batch, seq, _HIDDEN)}}
     if kind == "sd":
         batch, tokens, dim = case["batch"], case["tokens"], _SD["dim"]
         params = {}
@@ -154,31 +152,42 @@ def prepare(case, seed):
             params[f"{name}_bias"] = normal(4 * dim, scale=0.02)
         params["ff_out_weight"] = normal(dim, 4 * dim, scale=0.02)
         params["ff_out_bias"] = normal(dim, scale=0.02)
-        model = _model(workloads.build_sd_block(batch, tokens=tokens), "sd_block")
-        model.set_many_constants_with_tensors(params)
-        inputs = {"latent": normal(batch, tokens, dim),
-                  "context": normal(batch, _SD["context_tokens"], _SD["context_dim"])}
-        return {"case": case, "model": model, "params": params, "inputs": inputs,
-                "outputs": {"output_0": torch.empty((batch, tokens, dim), dtype=dtype, device="cuda")}}
+        return {"params": params, "inputs": {"latent": normal(batch, tokens, dim),
+                                             "context": normal(batch, _SD["context_tokens"], _SD["context_dim"])}}
     if kind == "gemm":
         m, n, k = case["m"], case["n"], case["k"]
-        return {"case": case, "x": uniform(m, k), "w": normal(n, k, scale=0.01), "bias": normal(n, scale=0.01),
+        return {"x": uniform(m, k), "w": normal(n, k, scale=0.01), "bias": normal(n, scale=0.01),
                 "d0": normal(m, n) if case["epilogue"] in _RESIDUAL else None}
     if kind == "attention":
         lengths, heads, dim = _lengths(case), case["heads"], case["dim"]
         if case["packed"]:
             starts = torch.tensor([0] + lengths, device="cuda").cumsum(0).to(torch.int32)
-            return {"case": case, "qkv": normal(sum(lengths), 3, heads, dim), "cu_seqlens": starts}
+            return {"qkv": normal(sum(lengths), 3, heads, dim), "cu_seqlens": starts}
         q, k, v = (normal(case["seqs"], heads, case["longest"], dim) for _ in range(3))
-        return {"case": case, "q": q, "k": k, "v": v,
+        return {"q": q, "k": k, "v": v,
                 "lengths_kv": torch.tensor(lengths, dtype=torch.int32, device="cuda")}
     if kind == "bmm":
         batch, m, n, k = case["batch"], case["m"], case["n"], case["k"]
-        return {"case": case, "a": uniform(batch, m, k),
+        return {"a": uniform(batch, m, k),
                 "b": uniform(batch, k, n) if case["b_row_major"] else uniform(batch, n, k)}
     n = case["n"]
-    return {"case": case, "x": normal(case["batch"], case["seq"], n, scale=2.0), "gamma": uniform(n, lo=0.5, hi=1.5),
+    return {"x": normal(case["batch"], case["seq"], n, scale=2.0), "gamma": uniform(n, lo=0.5, hi=1.5),
             "beta": normal(n, scale=0.1)}
+
+
+def prepare(case, seed):
+    state = {"case": case, **_inputs(case, seed)}
+    if case["kind"] == "bert":
+        _, y = workloads.build_bert_layer(case["batch"], case["seq"])
+        state["model"] = _model(y, "bert_layer")
+        state["model"].set_many_constants_with_tensors(
+            {n: state["params"][k] for n, k in workloads.BERT_PARAM_NAMES.items()})
+        state["outputs"] = {"output_0": torch.empty_like(state["inputs"]["hidden_states"])}
+    elif case["kind"] == "sd":
+        state["model"] = _model(workloads.build_sd_block(case["batch"], tokens=case["tokens"]), "sd_block")
+        state["model"].set_many_constants_with_tensors(state["params"])
+        state["outputs"] = {"output_0": torch.empty_like(state["inputs"]["latent"])}
+    return state
 
 
 # ------------------------------------------------------------------------------------------------------------ one call
@@ -252,3 +261,86 @@ def tolerance(case):
     # layer 4.2e-4 and 2.4e-3, one product 2.1e-4 and 5e-4; bf16: attention 2.3e-3 and 3.4e-2, one product 1.7e-3 and 4e-3)
     half = case.get("dtype", "fp16") == "fp16"
     return {"rel": 1.7e-3 if half else 9e-3, "max": 1e-2 if half else 0.14}
+
+
+# --------------------------------------------------------------------------------------- the same expressions in 64 bits
+
+
+def _attend(q, k, v, causal=False, length=None):
+    """softmax(q k^T / sqrt(d)) v of one sequence, [heads, rows, d] -> [rows, heads, d], 1024 query rows at a time."""
+    out, keys = [], torch.arange(k.shape[1], device=q.device)
+    for r0 in range(0, q.shape[1], 1024):
+        s = q[:, r0:r0 + 1024] @ k.transpose(1, 2) / math.sqrt(q.shape[2])
+        if length is not None:
+            s = s.masked_fill(keys >= length, -math.inf)
+        if causal:
+            rows = torch.arange(r0, r0 + s.shape[1], device=q.device)
+            s = s.masked_fill(keys > rows[:, None], -math.inf)
+        out.append((torch.softmax(s, dim=-1) @ v).transpose(0, 1))
+    return torch.cat(out)
+
+
+def _heads(x, heads):
+    return x.reshape(x.shape[0], heads, -1).transpose(0, 1)
+
+
+def _encoder_layer(x, p):
+    def one(h):  # [seq, hidden]
+        q, k, v = (_heads(t, 12) for t in F.linear(h, p["qkv_weight"], p["qkv_bias"]).chunk(3, dim=1))
+        a = F.linear(_attend(q, k, v).reshape(h.shape), p["proj_weight"], p["proj_bias"]) + h
+        a = F.layer_norm(a, a.shape[1:], p["ln1_gamma"], p["ln1_beta"], workloads.BERT_BASE["eps"])
+        f = F.gelu(F.linear(a, p["fc1_weight"], p["fc1_bias"]), approximate="tanh")
+        f = F.linear(f, p["fc2_weight"], p["fc2_bias"]) + a
+        return F.layer_norm(f, f.shape[1:], p["ln2_gamma"], p["ln2_beta"], workloads.BERT_BASE["eps"])
+
+    return torch.stack([one(h) for h in x])
+
+
+def _unet_block(x, context, p):
+    def norm(name, t):
+        return F.layer_norm(t, t.shape[1:], p[name + "_weight"], p[name + "_bias"], _SD["eps"])
+
+    def attention(name, h, ctx):
+        q, k, v = (_heads(F.linear(t, p[f"{name}_to_{n}_weight"]), _SD["heads"]) for n, t in (("q", h), ("k", ctx), ("v", ctx)))
+        return F.linear(_attend(q, k, v).reshape(h.shape), p[name + "_to_out_weight"], p[name + "_to_out_bias"])
+
+    def one(t, ctx):
+        h = norm("norm1", t)
+        t = t + attention("attn1", h, h)
+        t = t + attention("attn2", norm("norm2", t), ctx)
+        h = norm("norm3", t)
+        gate = F.gelu(F.linear(h, p["ff_gate_weight"], p["ff_gate_bias"]), approximate="tanh")
+        h = F.linear(h, p["ff_proj_weight"], p["ff_proj_bias"]) * gate
+        return t + F.linear(h, p["ff_out_weight"], p["ff_out_bias"])
+
+    return torch.stack([one(*pair) for pair in zip(x, context)])
+
+
+def exact(case, seed):
+    def wide(v):
+        if isinstance(v, dict):
+            return {name: wide(t) for name, t in v.items()}
+        return v.double() if torch.is_tensor(v) and v.is_floating_point() else v
+
+    given, kind = wide(_inputs(case, seed)), case["kind"]
+    if kind == "bert":
+        return {"output_0": _encoder_layer(given["inputs"]["hidden_states"], given["params"])}
+    if kind == "sd":
+        return {"output_0": _unet_block(given["inputs"]["latent"], given["inputs"]["context"], given["params"])}
+    if kind == "gemm":
+        y, d0 = F.linear(given["x"], given["w"], given["bias"]), given["d0"]
+        return {"": lambda: y, "relu": lambda: torch.relu(y), "gelu": lambda: F.gelu(y), "tanh": lambda: torch.tanh(y),
+                "fast_gelu": lambda: F.gelu(y, approximate="tanh"), "add": lambda: y + d0,
+                "add_relu": lambda: torch.relu(y + d0), "mul": lambda: y * d0}[case["epilogue"]]()
+    if kind == "attention":
+        causal, lengths = case["causal"], _lengths(case)
+        if case["packed"]:
+            return torch.cat([_attend(*t.permute(1, 2, 0, 3), causal) for t in given["qkv"].split(lengths)])
+        return torch.stack([_attend(q, k, v, causal, length)
+                            for q, k, v, length in zip(given["q"], given["k"], given["v"], lengths)])
+    if kind == "bmm":
+        return given["a"] @ (given["b"] if case["b_row_major"] else given["b"].transpose(1, 2))
+    x, n = given["x"], case["n"]
+    parts = list(x.split((n + 3) // 4, dim=2))
+    return {"layernorm": F.layer_norm(x, (n,), given["gamma"], given["beta"], 1e-5), "softmax": torch.softmax(x, dim=-1),
+            "parts": parts, "joined": torch.cat(parts[::-1], dim=2), "turned": x.transpose(1, 2)}
