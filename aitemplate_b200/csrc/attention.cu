@@ -9,7 +9,7 @@
 // and divided by the row sum at the end. S is never written to global memory.
 //
 // Persistent CTAs walk work items of 128 query rows of one (batch, head):
-//   warp 0      TMA producer: the item's Q tile, then K/V blocks of kBlockN keys into a 3-stage ring;
+//   warp 0      TMA producer: the item's Q tile, then K/V blocks of kBlockN keys into a ring (AttnCfg);
 //               the next item's Q streams in while the current item drains
 //   warp 6      MMA issuer:   S = Q K^T  (tcgen05.mma, fp32 accumulator in TMEM)
 //   warp 1      MMA issuer:   O += P V   (P read from TMEM, where the softmax threads put it over the S columns
@@ -21,7 +21,7 @@
 //               reference max / row sum, exp2, P (16-bit pairs) -> TMEM; O is touched only when a row's
 //               maximum outgrows the reference by more than 2^8 (then O and the row sum are rescaled in
 //               TMEM) and once at the end of the item (O / row sum -> global memory)
-// Two CTAs share an SM (head dim <= 64) so one CTA's softmax also overlaps the other's MMAs.
+// Two CTAs share an SM so one CTA's softmax also overlaps the other's MMAs.
 // Shared-memory bandwidth is what the MMAs of this kernel run into (a 128 x 64 x 16 MMA with both operands in
 // shared memory reads 6 KB and issues every 48 cycles = 128 B / clk, the whole bandwidth of an SM), which is why P
 // never goes through shared memory: that removed a 16 KB write and a 16 KB read per key block.
@@ -140,18 +140,26 @@ template <int DCH>
 struct AttnCfg {
   static constexpr int kQBytes = DCH * kBlockM * 128;
   static constexpr int kKBytes = DCH * kBlockN * 128;  // one K (or V) block
-  // K/V ring. A block's load is issued when the block kKvStages before it has been consumed and is needed two block
-  // periods before its own P V, so the ring gives (kKvStages - 2) block periods of lead (six stages measured the
-  // same as four, also on short sequences whose K / V come from DRAM).
-  static constexpr int kKvStages = 4;
+  // Two CTAs share an SM whatever the head's width: they have 113 KB of shared memory and 256 TMEM columns each. What
+  // the wide heads give up for it is the second Q tile, the second O and half of the K / V stages; what they gain is
+  // eight softmax warps per SM instead of four (16 heads of 128, bf16: 8 packed causal sequences of 512 .. 4096 rows,
+  // one CTA with four stages and two O buffers 421 us, two CTAs 292; 4 sequences of 2048 rows 186 -> 136 us).
+  // K/V ring. With four stages a block's load is issued when the block four before it has been consumed and is needed
+  // two block periods before its own P V: two block periods of lead (six stages measured the same, also on short
+  // sequences whose K / V come from DRAM). With two stages K and V have barriers of their own, and K is loaded again as
+  // soon as S of the block two before it is complete, a block period before its stage's V is free.
+  static constexpr int kKvStages = (DCH == 1) ? 4 : 2;
+  static constexpr bool kSplitKv = kKvStages == 2;
   static constexpr int kQBufs = (DCH == 1) ? 2 : 1;   // Q tiles in shared memory: the next item's Q loads an item ahead
+  static constexpr int kOBufs = (DCH == 1) ? 2 : 1;
   static constexpr int kDataBytes = kQBufs * kQBytes + kKvStages * 2 * kKBytes;
   // the dynamic shared-memory window is declared 1024-byte aligned, so no slack is reserved:
-  // two CTAs of the 64-wide configuration (96 KB each) must fit one SM
-  static constexpr int kBarrierBytes = 256;  // 19 mbarriers + the TMEM slot + the abort flag (160 bytes), padded
+  // two CTAs (96 KB each) must fit one SM
+  static constexpr int kBarrierBytes = 256;  // up to 20 mbarriers + the TMEM slot + the abort flag (168 bytes), padded
   static constexpr int kSmemBytes = kDataBytes + kBarrierBytes;
   static constexpr int kTWidth = DCH * 64;                       // columns of one O accumulator
-  static constexpr int kTmemCols = (DCH == 1) ? 256 : 512;       // S x2 (64 each) then O x2 (item parity)
+  static constexpr int kTmemCols = 2 * kBlockN + kOBufs * kTWidth;  // S x2, then O (x2: item parity)
+  static_assert(kTmemCols == 256 && 2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs share an SM");
 };
 
 // Persistent CTAs: each walks work items (one item = 128 query rows of one (batch, head)) with stride
@@ -170,7 +178,7 @@ struct AttnCfg {
 // NOMASK: no causal mask and a key length that is a multiple of the block: every key block is "plain", and the
 // kernel is compiled without the masked softmax body (the lean variant is measurably faster than a run-time test).
 template <int DCH, bool BF16, bool NOMASK>
-__global__ void __launch_bounds__(kAttnThreads, (DCH == 1) ? 2 : 1)
+__global__ void __launch_bounds__(kAttnThreads, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                     const __grid_constant__ CUtensorMap tma_v, const AttnParams p) {
   using Cfg = AttnCfg<DCH>;
@@ -192,9 +200,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   uint64_t* o_empty = p_full + 2;           // [2] the softmax threads have read the item's O out of TMEM
   uint64_t* drain_bar = o_empty + 2;         // [2] one per issuing thread, used only when a wait has given up
   uint64_t* q_empty = drain_bar + 2;          // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_empty + 2);
+  uint64_t* v_full = q_empty + 2;              // [kKvStages] with kSplitKv only: kv_full is K's alone then
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_full + (Cfg::kSplitKv ? Cfg::kKvStages : 0));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 + 2 * Cfg::kKvStages + 2 * 3 + 4) * 8 + 8 <= Cfg::kBarrierBytes, "barrier block overflows its shared memory");
+  static_assert((2 + 3 * Cfg::kKvStages + 2 * 3 + 4) * 8 + 8 <= Cfg::kBarrierBytes, "barrier block overflows its shared memory");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // work item -> where its rows live and how many key blocks it walks. n_blocks == 0 (a query tile past the end of
@@ -253,6 +262,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     for (int s = 0; s < Cfg::kKvStages; ++s) {
       mbar_init(&kv_full[s], 1);
       mbar_init(&kv_empty[s], 1);
+      if (Cfg::kSplitKv) mbar_init(&v_full[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
@@ -279,7 +289,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_s = tmem_base;        // S(j) at + (j & 1) * 64; P(j) as 16-bit pairs over its first 32 columns
-  const uint32_t tmem_o = tmem_base + 128;  // O of item it at + (it & 1) * kTWidth
+  const uint32_t tmem_o = tmem_base + 128;  // O of item it at + o_buf(it) * kTWidth
+  auto o_buf = [](int it) { return Cfg::kOBufs == 2 ? (it & 1) : 0; };
+  auto o_phase = [](int it) { return static_cast<uint32_t>(Cfg::kOBufs == 2 ? (it >> 1) & 1 : it & 1); };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -301,10 +313,26 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         for (int j = 0; j < w.n_blocks; ++j, ++g) {
           const int st = g % Cfg::kKvStages;
           const uint32_t ph = (g / Cfg::kKvStages) & 1;
-          ok = mbar_wait(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
-          if (!ok) break;
           uint8_t* sK = sKV + st * 2 * Cfg::kKBytes;
           uint8_t* sV = sK + Cfg::kKBytes;
+          if constexpr (Cfg::kSplitKv) {
+            // the block that had this stage before is g - 2: K is free when its S is complete, V when its P V is
+            ok = mbar_wait(&s_full[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&kv_full[st], Cfg::kKBytes);
+#pragma unroll
+            for (int c = 0; c < DCH; ++c)
+              load_rows(sK + c * kBlockN * 128, &tma_k, &kv_full[st], c * 64, w.row0 + j * kBlockN, w, p.k_order);
+            ok = mbar_wait(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&v_full[st], Cfg::kKBytes);
+#pragma unroll
+            for (int c = 0; c < DCH; ++c)
+              load_rows(sV + c * kBlockN * 128, &tma_v, &v_full[st], c * 64, w.row0 + j * kBlockN, w, p.v_order);
+            continue;
+          }
+          ok = mbar_wait(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+          if (!ok) break;
           mbar_arrive_expect_tx(&kv_full[st], 2 * Cfg::kKBytes);
 #pragma unroll
           for (int c = 0; c < DCH; ++c) {
@@ -335,13 +363,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         const Item w = decode_item(item);
         const int n_blocks = w.n_blocks;
         if (n_blocks == 0) continue;
-        // this item's O buffer was last used by item it - 2: its rows must have been read out
-        ok = mbar_wait(&o_empty[it & 1], ((it >> 1) & 1) ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
-        const uint32_t o_addr = tmem_o + static_cast<uint32_t>((it & 1) * Cfg::kTWidth);
+        // this item's O buffer was last used by item it - kOBufs: its rows must have been read out
+        ok = mbar_wait(&o_empty[o_buf(it)], o_phase(it) ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
+        const uint32_t o_addr = tmem_o + static_cast<uint32_t>(o_buf(it) * Cfg::kTWidth);
         for (int j = 0; ok && j < n_blocks; ++j) {
           const int g = gb + j;
           ATTN_PROBE(1)  // loop bookkeeping
           ok = mbar_wait(&p_full[g & 1], (g >> 1) & 1, abort_flag, p.status, kDevWaitOtherTimeout);
+          if (Cfg::kSplitKv && ok)
+            ok = mbar_wait(&v_full[g % Cfg::kKvStages], (g / Cfg::kKvStages) & 1, abort_flag, p.status, kDevWaitFullTimeout);
           if (!ok) break;
           tc_fence_after();
           ATTN_PROBE(2)  // wait for P
@@ -454,7 +484,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
                      kDevWaitAccFullTimeout))
         return false;
       tc_fence_after();
-      const uint32_t o_prev = tmem_o + lane_addr + static_cast<uint32_t>((pend.it & 1) * Cfg::kTWidth);
+      const uint32_t o_prev = tmem_o + lane_addr + static_cast<uint32_t>(o_buf(pend.it) * Cfg::kTWidth);
 #pragma unroll
       for (int c = 0; c < DCH * 2; ++c) {
         if (c * 32 < p.Dv) {  // warp-uniform
@@ -475,7 +505,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         }
       }
       tc_fence_before();
-      mbar_arrive(&o_empty[pend.it & 1]);
+      mbar_arrive(&o_empty[o_buf(pend.it)]);
       return true;
     };
     for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
@@ -491,7 +521,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         continue;
       }
       const int q_idx = w.q0 + r;
-      const uint32_t o_addr = tmem_o + lane_addr + static_cast<uint32_t>((it & 1) * Cfg::kTWidth);
+      const uint32_t o_addr = tmem_o + lane_addr + static_cast<uint32_t>(o_buf(it) * Cfg::kTWidth);
       float m_ref = -INFINITY, l_run = 0.f;
       for (int j = 0; ok && j < n_blocks; ++j) {
         const int g = gb + j;
@@ -761,11 +791,7 @@ void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnO
   AttnParams pp = p;
   pp.num_items = static_cast<int>(items);
   pp.q_order = attn_map_order(q), pp.k_order = attn_map_order(k), pp.v_order = attn_map_order(v);
-#ifdef B200AIT_ATTN_ONE_CTA  // tuning experiment: one CTA per SM
-  const long long grid = std::min<long long>(items, static_cast<long long>(sm_count()));
-#else
-  const long long grid = std::min<long long>(items, static_cast<long long>(sm_count()) * (DCH == 1 ? 2 : 1));
-#endif
+  const long long grid = std::min<long long>(items, static_cast<long long>(sm_count()) * 2);
   ::b200ait::count_launch(), attention_tc_kernel<DCH, BF16, NOMASK><<<static_cast<unsigned>(grid), kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv,
                                                                                                                  pp);
   B200AIT_CUDA_CHECK(cudaGetLastError());
