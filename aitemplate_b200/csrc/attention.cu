@@ -143,7 +143,8 @@ struct AttnCfg {
   // Two CTAs share an SM whatever the head's width: they have 113 KB of shared memory and 256 TMEM columns each. What
   // the wide heads give up for it is the second Q tile, the second O and half of the K / V stages; what they gain is
   // eight softmax warps per SM instead of four (16 heads of 128, bf16: 8 packed causal sequences of 512 .. 4096 rows,
-  // one CTA with four stages and two O buffers 421 us, two CTAs 292; 4 sequences of 2048 rows 186 -> 136 us).
+  // one CTA with four stages and two O buffers 421 us, two CTAs 292 and with a CTA per work item 276; 4 sequences of
+  // 2048 rows 186 -> 136 us).
   // K/V ring. With four stages a block's load is issued when the block four before it has been consumed and is needed
   // two block periods before its own P V: two block periods of lead (six stages measured the same, also on short
   // sequences whose K / V come from DRAM). With two stages K and V have barriers of their own, and K is loaded again as
@@ -791,7 +792,16 @@ void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnO
   AttnParams pp = p;
   pp.num_items = static_cast<int>(items);
   pp.q_order = attn_map_order(q), pp.k_order = attn_map_order(k), pp.v_order = attn_map_order(v);
-  const long long grid = std::min<long long>(items, static_cast<long long>(sm_count()) * 2);
+  // Normally every CTA walks its share of the items. From 64 key blocks on an item is long enough to pay for a CTA of
+  // its own, and the hardware hands the items out as SMs fall free: taken where the items differ in length (packed
+  // causal sequences of 512 .. 4096 rows: 64-wide heads 241 -> 224 us, 128-wide 295 -> 280) and where the fixed shares
+  // would be one item or two (2 x 8 heads x 4096 rows of 40: 130 -> 119 us). With 16 or 32 key blocks it loses (2 x 12
+  // heads x 2048 rows: 52 -> 54 us; packed causal up to 1024 rows: 33 -> 36), and so it does where equal items fill many
+  // rounds (4 x 12 heads x 4096 rows: 288 -> 301).
+  const long long resident = 2ll * sm_count();
+  const bool uneven = p.causal || p.cu_seqlens || p.lengths_kv || p.lengths_q;
+  const bool item_per_cta = p.Skv >= 64 * kBlockN && (uneven || items < 2 * resident);
+  const long long grid = item_per_cta ? items : std::min(items, resident);
   ::b200ait::count_launch(), attention_tc_kernel<DCH, BF16, NOMASK><<<static_cast<unsigned>(grid), kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv,
                                                                                                                  pp);
   B200AIT_CUDA_CHECK(cudaGetLastError());
