@@ -95,7 +95,7 @@ struct TileCfg {
   static constexpr int kStages = PAIR ? (D0BOX ? 5 : 6) : (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
   static constexpr int kTmemCols = 2 * BN;  // two accumulators
   static constexpr int kBoxesPerWarp = D0BOX ? 2 : 1;  // 32 rows x 64 columns x 16 bit = 4 KB each
-  static constexpr int kStagingBytes = (BN >= 128) ? kEpiWarps * kBoxesPerWarp * 4096 : 0;
+  static constexpr int kStagingBytes = kEpiWarps * kBoxesPerWarp * 4096;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes +
                                     2 * BN * 4 /*bias tile, fp32, one per accumulator*/;
@@ -228,7 +228,7 @@ __device__ __forceinline__ void epilogue_chunk32(const GemmParams& p, float (&v)
 
 
 // EPI >= 0 fixes the epilogue code at compile time (straight-line code for the common epilogues);
-// EPI == -1 reads it from the parameters.
+// EPI < 0 reads it from the parameters.
 template <int EPI>
 __device__ __forceinline__ int epilogue_code_of(const GemmParams& p) {
   return EPI >= 0 ? EPI : p.epilogue;
@@ -312,6 +312,95 @@ __device__ __forceinline__ void epilogue_direct_store32(const GemmParams& p, con
       if (col0 + j < p.N) out[col_offset(p, col0 + j)] = E::from_float(v[j]);
   }
 }
+
+// One warp moves a staged box (32 rows of 64 16-bit columns, 16-byte units swizzled by row) from or to rows that TMA
+// cannot describe: N or a stride that is not a multiple of 8, or a permuted output whose runs are not multiples of the
+// box. The lanes of an access lie side by side in one row (or in four rows, with 16-byte units), so it touches full
+// sectors; a thread that writes its own row makes 32 partial ones of every access. Per-thread rows -> here: 1294 x 4711 x
+// 2424 bf16 116 .. 176 -> 50 us; 4138 x 756 x 768 bf16 51 -> 19 us; 2000 x 3333 x 1024 with a multiplied residual 162 ->
+// 60 us; 8000 x 2304 x 768 into [3, 8, 12, 1000, 64] 50 -> 45 us.
+template <bool BF16>
+__device__ __forceinline__ void load_box_rows(uint8_t* box, const typename Elem16<BF16>::T* src, long long ld, int rows,
+                                              int width, int lane) {
+  using T = typename Elem16<BF16>::T;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += 8) {
+    T x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {  // every load of eight rows in flight before the first is stored
+      const int r = r0 + (i >> 1), col = (i & 1) * 32 + lane;
+      if (r < rows && col < width) x[i] = src[r * ld + col];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int r = r0 + (i >> 1), col = (i & 1) * 32 + lane;
+      if (r < rows && col < width) *reinterpret_cast<T*>(box + r * 128 + (((col >> 3) ^ (r & 7)) * 16) + (col & 7) * 2) = x[i];
+    }
+  }
+}
+template <bool BF16>
+__device__ __forceinline__ void store_box_rows(const GemmParams& p, const uint8_t* box, int b, int row0, int gcol,
+                                               int rows, int width, int lane) {
+  using T = typename Elem16<BF16>::T;
+  T* out = static_cast<T*>(p.out) + batch_offset(p, b);
+  if (p.vec_ok) {  // 16-byte units stay whole in the output
+    const int u = lane & 7;
+    if (u * 8 < width) {
+      T* dst = out + col_offset(p, gcol + u * 8);
+#pragma unroll 4
+      for (int r = lane >> 3; r < rows; r += 4)
+        *reinterpret_cast<uint4*>(dst + row_offset(p, row0 + r)) =
+            *reinterpret_cast<const uint4*>(box + r * 128 + ((u ^ (r & 7)) * 16));
+    }
+    return;
+  }
+  if (p.store_mode == 0) {
+    // Pairs of columns from the first 4-byte boundary of a row on (with an odd pitch every second row starts off one);
+    // eight rows are read from the box before the first is stored.
+    out += static_cast<long long>(row0) * p.ldc + gcol;
+    auto at = [&](int r, int k) { return *reinterpret_cast<const uint16_t*>(box + r * 128 + (((k >> 3) ^ (r & 7)) * 16) + (k & 7) * 2); };
+#pragma unroll 1
+    for (int r0 = 0; r0 < rows; r0 += 8) {
+      uint32_t x[8];
+      uint16_t* dst0 = reinterpret_cast<uint16_t*>(out + static_cast<long long>(r0) * p.ldc);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int off = static_cast<int>(reinterpret_cast<uintptr_t>(dst0 + i * p.ldc) >> 1) & 1;
+        const int col = 2 * lane - off;  // off = 1: lane 0 has column 0 (in the upper half), and column 63 below
+        x[i] = static_cast<uint32_t>(at(r0 + i, col + 1)) << 16;
+        x[i] |= at(r0 + i, col < 0 ? 63 : col);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (r0 + i >= rows) break;
+        uint16_t* dst = dst0 + i * p.ldc;
+        const int off = static_cast<int>(reinterpret_cast<uintptr_t>(dst) >> 1) & 1;
+        const int col = 2 * lane - off;
+        if (col >= 0 && col + 1 < width) {
+          *reinterpret_cast<uint32_t*>(dst + col) = x[i];
+        } else if (col < 0) {
+          dst[0] = static_cast<uint16_t>(x[i] >> 16);
+          if (width == 64) dst[63] = static_cast<uint16_t>(x[i]);
+        } else if (col < width) {
+          dst[col] = static_cast<uint16_t>(x[i]);
+        }
+      }
+    }
+    return;
+  }
+  for (int h = 0; h < 64; h += 32) {
+    const int col = h + lane;
+    if (col >= width) continue;
+    T* dst = out + col_offset(p, gcol + col);
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r)
+      dst[row_offset(p, row0 + r)] = *reinterpret_cast<const T*>(box + r * 128 + (((col >> 3) ^ (r & 7)) * 16) + (col & 7) * 2);
+  }
+}
+
+// EPI of the instantiations that read the epilogue from the parameters and write the output row by row (the plain
+// generic ones do not carry that path: it cost them 5 to 10 % on outputs that never take it).
+constexpr int kRowsEpilogue = -2;
 
 // BMN: B is stored [K, N]. MULTI: the staged store goes to p.num_out destinations. Both are compile-time, so that
 // the plain [N, K] single-destination kernels carry no trace of them (a run-time flag cost the BERT-layer GEMMs
@@ -563,7 +652,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     const bool has_d0 = epi_b1(code) != kBinaryNone;
     const bool has_bias = p.bias != nullptr && splits == 1;
     const bool chunk_contig = p.store_mode == 0 || (p.d % 32 == 0);
-    const bool use_tma = kLean || ((BN >= 128) && p.tma_store != 0);
+    const bool use_tma = kLean || (EPI != kRowsEpilogue && (BN >= 128) && p.tma_store != 0);
     // residual through staging boxes: needs the TMA store path and a tensor map over d0
     const bool box_d0 = D0BOX && (kLean || (use_tma && p.tma_d0 != 0));
     uint8_t* my_staging = staging + ew * (Cfg::kBoxesPerWarp * 4096);
@@ -733,6 +822,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
               bulk_commit_group();
             }
           }
+        } else if constexpr (EPI == kRowsEpilogue) {
+          // An output that TMA cannot describe: the warp's box goes through the same staging buffer and is written row
+          // by row.
+          uint8_t* row_base = my_staging + lane * 128;
+          const int gcol = colh + (c & ~1) * 32;
+          const int width = min(64, min(BN / 2 - (c & ~1) * 32, p.N - gcol)), rows = min(32, p.M - row0);
+          const bool row_d0 = has_d0 && !p.vec_ok && epi_b2(code) == kBinaryNone;
+          if (row_d0) {
+            if ((c & 1) == 0) {
+              load_box_rows<BF16>(my_staging, static_cast<const T*>(p.d0) + static_cast<long long>(b) * p.d_bs +
+                                                  static_cast<long long>(row0) * p.ldd + gcol, p.ldd, rows, width, lane);
+              __syncwarp();
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              d0c[u] = *reinterpret_cast<const uint4*>(row_base + ((((c & 1) * 4 + u) ^ (lane & 7)) * 16));
+          }
+          epilogue_math32<BF16, EPI>(p, v, d0c, b, row, col0, full || row_d0, row_ok);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            *reinterpret_cast<uint4*>(row_base + ((((c & 1) * 4 + u) ^ (lane & 7)) * 16)) = pack8<BF16>(&v[u * 8]);
+          if ((c & 1) != 0 || c + 1 == kChunksPerWarp || col0 + 32 >= p.N) {
+            __syncwarp();
+            store_box_rows<BF16>(p, my_staging, b, row0, gcol, rows, width, lane);
+            __syncwarp();
+          }
         } else if (row_ok) {
           epilogue_math32<BF16, EPI>(p, v, d0c, b, row, col0, full, true);
           epilogue_direct_store32<BF16>(p, v, b, row, col0, full, chunk_contig);
@@ -860,6 +975,14 @@ void launch_tc_pair256_bf16_lean(const CUtensorMap& ta, const CUtensorMap& tb, c
         launch_tc<BN_, true, -1, true>(ta, tb, tout, p, grid, stream);                                         \
       else                                                                                                     \
         launch_tc<BN_, false, -1, true>(ta, tb, tout, p, grid, stream);                                        \
+      return;                                                                                                  \
+    }                                                                                                          \
+    /* outputs that TMA cannot describe (64-wide tiles store 16-byte vectors per thread where they can) */     \
+    if (p.splits == 1 && (BN_ < 128 ? p.vec_ok == 0 : p.tma_store == 0)) {                                     \
+      if (bf16)                                                                                                \
+        launch_tc<BN_, true, kRowsEpilogue>(ta, tb, tout, p, grid, stream);                                    \
+      else                                                                                                     \
+        launch_tc<BN_, false, kRowsEpilogue>(ta, tb, tout, p, grid, stream);                                   \
       return;                                                                                                  \
     }                                                                                                          \
     if (bf16) {                                                                                                \

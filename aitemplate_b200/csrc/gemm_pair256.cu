@@ -24,6 +24,13 @@ void launch_tc_pair256(bool bf16, const CUtensorMap& ta, const CUtensorMap& tb, 
       launch_tc_pair<256, false, -1, true>(ta, tb, tout, td0, p, grid, stream);
     return;
   }
+  if (p.tma_store == 0) {  // written row by row
+    if (bf16)
+      launch_tc_pair<256, true, kRowsEpilogue>(ta, tb, tout, td0, p, grid, stream);
+    else
+      launch_tc_pair<256, false, kRowsEpilogue>(ta, tb, tout, td0, p, grid, stream);
+    return;
+  }
   // the compile-time-epilogue kernels are lean: alpha = 1, staged TMA store, residual (if any) through staged boxes
   const bool lean_ok = p.alpha == 1.f && p.tma_store != 0 && (epi_b1(p.epilogue) == kBinaryNone || p.tma_d0 != 0);
   if (!lean_ok) {
