@@ -203,6 +203,88 @@ __global__ void __launch_bounds__(kRowDotThreads, 1) gemm_rowdot_kernel(const vo
   }
 }
 
+// The same for K <= 1024, where a row of W is so short that one row per warp leaves too little in flight and the
+// launch's latencies are most of the time: a warp takes up to 8 / KV rows at once (KV 16-byte vectors per lane and row,
+// eight loads in flight), its first rows are on their way before the block stages X, and all its sums are reduced
+// together. M = 1 .. 4 on the tile kernels -> here: K = 1016, N = 512: 8.2 -> 2.8 us, N = 3176: 10.6 -> 3.2 .. 4.0;
+// K = 512, N = 3176: 8.2 -> 2.9 .. 4.7; K = 256, N = 100: 7.4 -> 2.6 .. 3.9.
+constexpr int kRowDotShortThreads = 512;
+template <bool BF16, int MR, int KV>
+__global__ void __launch_bounds__(kRowDotShortThreads, 1) gemm_rowdot_short_kernel(const void* a_, const void* b_,
+                                                                                   const GemmParams p) {
+  using T = typename Elem16<BF16>::T;
+  constexpr int kRows = MR == 4 && KV == 1 ? 4 : 8 / KV;  // (32 sums do not fit the registers beside the loads)
+  __shared__ uint4 xs[MR * KV * 32];  // [MR][KV * 32], zero past K
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kRowDotShortThreads / 32;
+  const int nvec = p.K >> 3;
+  // rows [n_begin, n_end) of W belong to this block, row n_begin + i to warp i % kWarps
+  const int per = (p.N + gridDim.x - 1) / gridDim.x;
+  const int n_begin = blockIdx.x * per, n_end = min(p.N, n_begin + per);
+  uint4 wq[kRows][KV];
+  auto fetch = [&](int n0) {
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int n = n0 + r * kWarps;
+      const uint4* w = reinterpret_cast<const uint4*>(static_cast<const T*>(b_) + static_cast<long long>(n) * p.ldb);
+#pragma unroll
+      for (int u = 0; u < KV; ++u)
+        wq[r][u] = (n < n_end && lane + 32 * u < nvec) ? __ldcs(w + lane + 32 * u) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  fetch(n_begin + warp);
+  for (int i = threadIdx.x; i < MR * KV * 32; i += kRowDotShortThreads) {
+    const int m = i / (KV * 32), v = i - m * (KV * 32);
+    xs[i] = (m < p.M && v < nvec) ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a_) + static_cast<long long>(m) * p.lda) + v)
+                                  : make_uint4(0, 0, 0, 0);
+  }
+  __syncthreads();
+  for (int n0 = n_begin + warp; n0 < n_end; n0 += kWarps * kRows) {
+    float acc[kRows][MR];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int m = 0; m < MR; ++m) acc[r][m] = 0.f;
+#pragma unroll
+    for (int u = 0; u < KV; ++u)
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        float xf[8];
+        unpack8<BF16>(xs[m * KV * 32 + u * 32 + lane], xf);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          float wf[8];
+          unpack8<BF16>(wq[r][u], wf);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[r][m] = fmaf(xf[j], wf[j], acc[r][m]);
+        }
+      }
+    if (n0 + kWarps * kRows < n_end) fetch(n0 + kWarps * kRows);
+    // Sums over the lanes, all of them at once: at every step a lane keeps one half of its values and hands over the
+    // other (31 shuffles for 32 values instead of 160), and ends with value lane / (32 / kValues).
+    constexpr int kValues = kRows * MR;
+    float val[kValues];
+#pragma unroll
+    for (int i = 0; i < kValues; ++i) val[i] = acc[i / MR][i % MR];
+#pragma unroll
+    for (int o = 16, left = kValues; o > 0; o >>= 1) {
+      if (left > 1) {
+        left >>= 1;
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < left; ++i) {
+          const float keep = upper ? val[i + left] : val[i], give = upper ? val[i] : val[i + left];
+          val[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      } else {
+        val[0] += __shfl_xor_sync(0xffffffffu, val[0], o);
+      }
+    }
+    const int i = lane / (32 / kValues), n = n0 + (i / MR) * kWarps;
+    if (lane % (32 / kValues) == 0 && n < n_end && i % MR < p.M) epilogue_scalar_store<BF16>(p, val[0], 0, i % MR, n);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 // Weight-streaming tensor-core kernel with the operands swapped: Y^T = W X^T.
 // The run time of a GEMM with few rows of X is the time to read W once. Here the rows of W sit on the 128 MMA rows
@@ -1071,6 +1153,30 @@ void gemm_run(const GemmArgs& g_in) {
     } else {
       if (g.m <= 1) B200AIT_ROWDOT(false, 1); else if (g.m <= 2) B200AIT_ROWDOT(false, 2); else B200AIT_ROWDOT(false, 4);
     }
+#undef B200AIT_ROWDOT
+    B200AIT_CUDA_CHECK(cudaGetLastError());
+    return;
+  }
+  // the same for shorter rows; below K = 256 the tile kernels are level or ahead (K = 128, N = 8192: 4.8 against 3.1 .. 6.0 us)
+  if (tma_ok && g.batch == 1 && g.m <= kRowDotMaxM && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0 &&
+      g.k >= 256 && g.k < 1024 && g.n >= 64) {
+    const unsigned grid = static_cast<unsigned>(std::min<long long>(sm_count(), (g.n + 3) / 4));
+#define B200AIT_ROWDOT(MR, KV)                                                                                    \
+  do {                                                                                                            \
+    ::b200ait::count_launch();                                                                                    \
+    if (bf16)                                                                                                     \
+      gemm_rowdot_short_kernel<true, MR, KV><<<grid, kRowDotShortThreads, 0, g.stream>>>(g.a, g.b, p);            \
+    else                                                                                                          \
+      gemm_rowdot_short_kernel<false, MR, KV><<<grid, kRowDotShortThreads, 0, g.stream>>>(g.a, g.b, p);           \
+  } while (0)
+#define B200AIT_ROWDOT_K(MR)                       \
+  do {                                             \
+    if (g.k <= 256) B200AIT_ROWDOT(MR, 1);         \
+    else if (g.k <= 512) B200AIT_ROWDOT(MR, 2);    \
+    else B200AIT_ROWDOT(MR, 4);                    \
+  } while (0)
+    if (g.m <= 1) B200AIT_ROWDOT_K(1); else if (g.m <= 2) B200AIT_ROWDOT_K(2); else B200AIT_ROWDOT_K(4);
+#undef B200AIT_ROWDOT_K
 #undef B200AIT_ROWDOT
     B200AIT_CUDA_CHECK(cudaGetLastError());
     return;
