@@ -116,6 +116,8 @@ def exported_symbols():
 def load() -> ctypes.CDLL:
     """Loads libb200ait.so; raises if it has not been built (there is no fallback path)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

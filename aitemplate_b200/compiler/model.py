@@ -79,6 +79,8 @@ def _reshape_tensor(tensor, shape: List[int]):
     assert tensor.ndim == len(shape), (
         f"Expected output tensor's ndim to match the length of Run()'s return value: {tensor.ndim=} != {len(shape)=}")
     numel = math.prod(shape)
+    if numel == tensor.numel() and tensor.is_contiguous():
+        return tensor.view(shape)
     return tensor.flatten()[:numel].reshape(shape)
 
 
@@ -93,6 +95,8 @@ class Model:
 
         def close(self) -> None:
             self.is_open = False
+            for name in [n for n, f in self.__dict__.items() if callable(f) and n != "DLL"]:
+                del self.__dict__[name]  # from here on every call ends in __getattr__
 
         def __getattr__(self, name):
             if not self.is_open:
@@ -105,6 +109,7 @@ class Model:
                 if err:
                     raise RuntimeError(f"Error in function: {name}: {_lib.last_error()}")
 
+            self.__dict__[name] = _wrapped
             return _wrapped
 
     def __init__(self, lib_path: str, num_runtimes: int = AIT_DEFAULT_NUM_RUNTIMES,
@@ -179,8 +184,7 @@ class Model:
         c_stream = ctypes.c_void_p() if stream_ptr is None else ctypes.c_void_p(stream_ptr)
         num_outputs = len(self._output_ndims)
         c_shapes = [(ctypes.c_longlong * n)() for n in self._output_ndims]
-        c_shape_ptrs = (ctypes.POINTER(ctypes.c_longlong) * num_outputs)(
-            *[ctypes.cast(s, ctypes.POINTER(ctypes.c_longlong)) for s in c_shapes])
+        c_shape_ptrs = (ctypes.POINTER(ctypes.c_longlong) * num_outputs)(*c_shapes)
         return c_inputs, c_outputs, c_stream, ctypes.c_bool(sync), ctypes.c_bool(graph_mode), c_shapes, c_shape_ptrs
 
     def _dict_to_ordered_list(self, params, is_inputs: bool):
@@ -233,7 +237,7 @@ class Model:
         if stream_ptr is None:
             import torch
 
-            stream_ptr = torch.cuda.current_stream().cuda_stream
+            stream_ptr = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
         outputs_ait = self.run(_convert_tensor_args(inputs), _convert_tensor_args(outputs), stream_ptr=stream_ptr,
                                sync=sync, graph_mode=graph_mode)
         return self._interpret_tensors_as_shapes(outputs, outputs_ait)
@@ -291,7 +295,7 @@ class Model:
         if stream_ptr is None:
             import torch
 
-            stream_ptr = torch.cuda.current_stream().cuda_stream
+            stream_ptr = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
         mean, std, out = self.benchmark(_convert_tensor_args(inputs), _convert_tensor_args(outputs), stream_ptr,
                                         graph_mode, count, repeat, num_threads, use_unique_stream_per_thread)
         return mean, std, self._interpret_tensors_as_shapes(outputs, out)

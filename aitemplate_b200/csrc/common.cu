@@ -1,6 +1,7 @@
 // Library-wide host state: last-error text, per-device status word, device properties.
 #include "common.h"
 
+#include <atomic>
 #include <cstring>
 #include <mutex>
 
@@ -12,8 +13,9 @@ namespace {
 thread_local std::string g_last_error;
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
-int* g_status_word[kMaxDevices] = {};
-int g_sm_count[kMaxDevices] = {};
+// set once per device under g_mutex, read without it (a planner asks for the SM count a dozen times per call)
+std::atomic<int*> g_status_word[kMaxDevices] = {};
+std::atomic<int> g_sm_count[kMaxDevices] = {};
 
 int current_device() {
   int dev = 0;
@@ -28,25 +30,24 @@ const std::string& last_error() { return g_last_error; }
 
 int* device_status_word() {
   const int dev = current_device();
+  if (int* p = g_status_word[dev].load(std::memory_order_acquire)) return p;
   std::lock_guard<std::mutex> lock(g_mutex);
-  if (!g_status_word[dev]) {
-    int* p = nullptr;
-    B200AIT_CUDA_CHECK(cudaMalloc(&p, sizeof(int)));
-    B200AIT_CUDA_CHECK(cudaMemset(p, 0, sizeof(int)));
-    g_status_word[dev] = p;
-  }
-  return g_status_word[dev];
+  if (int* p = g_status_word[dev].load(std::memory_order_relaxed)) return p;
+  int* p = nullptr;
+  B200AIT_CUDA_CHECK(cudaMalloc(&p, sizeof(int)));
+  B200AIT_CUDA_CHECK(cudaMemset(p, 0, sizeof(int)));
+  g_status_word[dev].store(p, std::memory_order_release);
+  return p;
 }
 
 int sm_count() {
   const int dev = current_device();
-  std::lock_guard<std::mutex> lock(g_mutex);
-  if (!g_sm_count[dev]) {
-    int n = 0;
-    B200AIT_CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    g_sm_count[dev] = n > 0 ? n : 1;
-  }
-  return g_sm_count[dev];
+  if (const int known = g_sm_count[dev].load(std::memory_order_relaxed)) return known;
+  int n = 0;
+  B200AIT_CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  n = n > 0 ? n : 1;
+  g_sm_count[dev].store(n, std::memory_order_relaxed);  // (threads that race here store the same value)
+  return n;
 }
 
 void opt_in_smem_once(std::atomic<uint64_t>& done, const void* kernel, int bytes) {

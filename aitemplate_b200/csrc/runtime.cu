@@ -1060,9 +1060,11 @@ class ModelContainer {
     }
     release(ex);
     if (sync) {
-      B200AIT_CUDA_CHECK(cudaStreamSynchronize(stream));
+      // The status word is read behind the run on its own stream, so that one wait covers both: a blocking copy after
+      // the wait is a second round trip to the GPU, and one on the default stream.
       int status = 0;
-      B200AIT_CUDA_CHECK(cudaMemcpy(&status, device_status_word(), sizeof(int), cudaMemcpyDeviceToHost));
+      B200AIT_CUDA_CHECK(cudaMemcpyAsync(&status, device_status_word(), sizeof(int), cudaMemcpyDeviceToHost, stream));
+      B200AIT_CUDA_CHECK(cudaStreamSynchronize(stream));
       if (status != 0) {
         B200AIT_CUDA_CHECK(cudaMemset(device_status_word(), 0, sizeof(int)));
         throw Error("a kernel gave up waiting (device status " + std::to_string(status) + "); outputs are invalid");
