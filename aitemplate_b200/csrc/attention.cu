@@ -143,7 +143,7 @@ struct AttnCfg {
   // Two CTAs share an SM whatever the head's width: they have 113 KB of shared memory and 256 TMEM columns each. What
   // the wide heads give up for it is the second Q tile, the second O and half of the K / V stages; what they gain is
   // eight softmax warps per SM instead of four (16 heads of 128, bf16: 8 packed causal sequences of 512 .. 4096 rows,
-  // one CTA with four stages and two O buffers 421 us, two CTAs 292 and with a CTA per work item 276; 4 sequences of
+  // one CTA with four stages and two O buffers 421 us, two CTAs 292, with a CTA per work item 280; 4 sequences of
   // 2048 rows 186 -> 136 us).
   // K/V ring. With four stages a block's load is issued when the block four before it has been consumed and is needed
   // two block periods before its own P V: two block periods of lead (six stages measured the same, also on short
