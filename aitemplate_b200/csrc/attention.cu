@@ -36,6 +36,7 @@
 #include "common.h"
 #include "epilogue.cuh"
 #include "ptx.cuh"
+#include "rules.h"
 
 namespace b200ait {
 
@@ -136,8 +137,10 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
   p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(r1) << 23));
 }
 
-template <int DCH>
+// LONE: the problem has at most one work item per SM, so that no two CTAs share one and no CTA has a second item.
+template <int DCH, bool LONE>
 struct AttnCfg {
+  static_assert(DCH == 2 || !LONE, "narrow heads have four stages with two CTAs on an SM as well");
   static constexpr int kQBytes = DCH * kBlockM * 128;
   static constexpr int kKBytes = DCH * kBlockN * 128;  // one K (or V) block
   // Two CTAs share an SM whatever the head's width: they have 113 KB of shared memory and 256 TMEM columns each. What
@@ -145,11 +148,13 @@ struct AttnCfg {
   // eight softmax warps per SM instead of four (16 heads of 128, bf16: 8 packed causal sequences of 512 .. 4096 rows,
   // one CTA with four stages and two O buffers 421 us, two CTAs 292, with a CTA per work item 280; 4 sequences of
   // 2048 rows 186 -> 136 us).
+  // A lone CTA on its SM has the shared memory of two and keeps four stages: a decode step reads K and V at the pace of
+  // the loads in flight (attn_lone).
   // K/V ring. With four stages a block's load is issued when the block four before it has been consumed and is needed
   // two block periods before its own P V: two block periods of lead (six stages measured the same, also on short
   // sequences whose K / V come from DRAM). With two stages K and V have barriers of their own, and K is loaded again as
   // soon as S of the block two before it is complete, a block period before its stage's V is free.
-  static constexpr int kKvStages = (DCH == 1) ? 4 : 2;
+  static constexpr int kKvStages = (DCH == 1 || LONE) ? 4 : 2;
   static constexpr bool kSplitKv = kKvStages == 2;
   static constexpr int kQBufs = (DCH == 1) ? 2 : 1;   // Q tiles in shared memory: the next item's Q loads an item ahead
   static constexpr int kOBufs = (DCH == 1) ? 2 : 1;
@@ -158,9 +163,10 @@ struct AttnCfg {
   // two CTAs (96 KB each) must fit one SM
   static constexpr int kBarrierBytes = 256;  // up to 20 mbarriers + the TMEM slot + the abort flag (168 bytes), padded
   static constexpr int kSmemBytes = kDataBytes + kBarrierBytes;
+  static constexpr int kCtasPerSm = LONE ? 1 : 2;
   static constexpr int kTWidth = DCH * 64;                       // columns of one O accumulator
   static constexpr int kTmemCols = 2 * kBlockN + kOBufs * kTWidth;  // S x2, then O (x2: item parity)
-  static_assert(kTmemCols == 256 && 2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs share an SM");
+  static_assert(kTmemCols == 256 && kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "the CTAs of an SM fit it");
 };
 
 // Persistent CTAs: each walks work items (one item = 128 query rows of one (batch, head)) with stride
@@ -178,11 +184,11 @@ struct AttnCfg {
 // (attention_scaling_coefs_updater.h:85-165), up to the rounding of P at a different power-of-two-ish scale.
 // NOMASK: no causal mask and a key length that is a multiple of the block: every key block is "plain", and the
 // kernel is compiled without the masked softmax body (the lean variant is measurably faster than a run-time test).
-template <int DCH, bool BF16, bool NOMASK>
+template <int DCH, bool BF16, bool NOMASK, bool LONE>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                     const __grid_constant__ CUtensorMap tma_v, const AttnParams p) {
-  using Cfg = AttnCfg<DCH>;
+  using Cfg = AttnCfg<DCH, LONE>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {  // swizzled tiles need 1024-byte alignment
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kDevBadSmemAlignment);
@@ -777,17 +783,23 @@ static CUtensorMap make_attn_map(const AttnOperand& op, bool bf16, int d, long l
   return m;
 }
 
-template <int DCH, bool BF16, bool NOMASK>
+template <int DCH, bool BF16, bool NOMASK, bool LONE = false>
 void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const AttnParams& p,
                          long long q_rows, long long kv_rows, cudaStream_t stream) {
-  using Cfg = AttnCfg<DCH>;
+  const long long items = static_cast<long long>(p.B) * p.H * p.q_blocks;
+  if constexpr (DCH == 2 && !LONE) {
+    if (attn_lone(items, sm_count())) {
+      launch_attn_variant<DCH, BF16, NOMASK, true>(q, k, v, p, q_rows, kv_rows, stream);
+      return;
+    }
+  }
+  using Cfg = AttnCfg<DCH, LONE>;
   static std::atomic<uint64_t> configured{0};
-  opt_in_smem_once(configured, reinterpret_cast<const void*>(&attention_tc_kernel<DCH, BF16, NOMASK>), Cfg::kSmemBytes);
+  opt_in_smem_once(configured, reinterpret_cast<const void*>(&attention_tc_kernel<DCH, BF16, NOMASK, LONE>), Cfg::kSmemBytes);
   const int map_batches = p.cu_seqlens ? 1 : p.B;
   CUtensorMap tq = make_attn_map(q, BF16, p.D, q_rows, p.H, map_batches, kBlockM);
   CUtensorMap tk = make_attn_map(k, BF16, p.D, kv_rows, p.H, map_batches, kBlockN);
   CUtensorMap tv = make_attn_map(v, BF16, p.Dv, kv_rows, p.H, map_batches, kBlockN);
-  const long long items = static_cast<long long>(p.B) * p.H * p.q_blocks;
   B200AIT_REQUIRE(items < (1ll << 31), "attention: too many work items");
   AttnParams pp = p;
   pp.num_items = static_cast<int>(items);
@@ -802,7 +814,7 @@ void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnO
   const bool uneven = p.causal || p.cu_seqlens || p.lengths_kv || p.lengths_q;
   const bool item_per_cta = p.Skv >= 64 * kBlockN && (uneven || items < 2 * resident);
   const long long grid = item_per_cta ? items : std::min(items, resident);
-  ::b200ait::count_launch(), attention_tc_kernel<DCH, BF16, NOMASK><<<static_cast<unsigned>(grid), kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv,
+  ::b200ait::count_launch(), attention_tc_kernel<DCH, BF16, NOMASK, LONE><<<static_cast<unsigned>(grid), kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv,
                                                                                                                  pp);
   B200AIT_CUDA_CHECK(cudaGetLastError());
 }

@@ -53,3 +53,19 @@ def test_packed_sequences(causal):
             q, k, v = (t.permute(1, 0, 2)[None] for t in qkv[lo:hi].unbind(1))
             want = oracle.mem_eff_attention(q, k, v, causal=causal)[0]
             assert float((got[lo:hi] - want).abs().max()) < 4e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize(
+    "b,h,sq,skv,d,causal,lengths",
+    [
+        (1, 1, 1, 40, 128, False, False),     # one row, one ragged key block
+        (2, 8, 1, 1000, 72, False, False),    # a decode step: the ring of four stages goes round several times
+        (4, 37, 1, 320, 96, False, False),    # an item for every SM (148), no masks, five key blocks
+        (1, 9, 129, 576, 128, True, False),
+        (4, 5, 200, 700, 128, False, True),   # items of no, one and several key blocks
+    ],
+)
+def test_an_item_per_sm(b, h, sq, skv, d, causal, lengths, dtype):
+    """At most one work item per SM: the form with four K / V stages and one CTA per SM."""
+    test_items_follow_one_another(b, h, sq, skv, d, causal, lengths, dtype)
