@@ -96,6 +96,9 @@ struct AttnParams {
   // coordinate order of each tensor map: 0 = (channel, row, head, batch), 1 = (channel, head, row, batch); the host
   // picks whichever keeps the map's strides ascending
   int q_order, k_order, v_order;
+  // packed mode with a CTA per work item: a tile past the end of its sequence ends its CTA before the set-up (64 sequences
+  // of 128 rows under a bound of 4096, 12 heads: 144 -> 134 us; 8 of 512 .. 4096 rows, 16 heads of 128: 283 -> 277)
+  int skip_empty;
 };
 
 // One operand (q, k or v) as the kernel addresses it: element strides of a [batch, head, row, channel] view with
@@ -261,6 +264,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     else
       tma_load_4d(dst, map, bar, c0, w.h, row, w.b4);
   };
+  if (p.skip_empty && decode_item(blockIdx.x).n_blocks == 0) return;
   const int dsteps = (p.D + 15) / 16;  // k-steps of Q K^T
 
   if (threadIdx.x == 0) {
@@ -804,15 +808,11 @@ void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnO
   AttnParams pp = p;
   pp.num_items = static_cast<int>(items);
   pp.q_order = attn_map_order(q), pp.k_order = attn_map_order(k), pp.v_order = attn_map_order(v);
-  // Normally every CTA walks its share of the items. From 64 key blocks on an item is long enough to pay for a CTA of
-  // its own, and the hardware hands the items out as SMs fall free: taken where the items differ in length (packed
-  // causal sequences of 512 .. 4096 rows: 64-wide heads 241 -> 224 us, 128-wide 295 -> 280) and where the fixed shares
-  // would be one item or two (2 x 8 heads x 4096 rows of 40: 130 -> 119 us). With 16 or 32 key blocks it loses (2 x 12
-  // heads x 2048 rows: 52 -> 54 us; packed causal up to 1024 rows: 33 -> 36), and so it does where equal items fill many
-  // rounds (4 x 12 heads x 4096 rows: 288 -> 301).
-  const long long resident = 2ll * sm_count();
-  const bool uneven = p.causal || p.cu_seqlens || p.lengths_kv || p.lengths_q;
-  const bool item_per_cta = p.Skv >= 64 * kBlockN && (uneven || items < 2 * resident);
+  const long long resident = static_cast<long long>(Cfg::kCtasPerSm) * sm_count();
+  const AttnItems work{items, p.q_blocks, (p.Skv + kBlockN - 1) / kBlockN, p.causal != 0, p.lengths_kv || p.lengths_q,
+                       p.cu_seqlens ? kv_rows / p.B : p.Skv, p.Skv, std::max(p.D, p.Dv)};
+  const bool item_per_cta = attn_item_per_cta(work, sm_count());
+  pp.skip_empty = item_per_cta && p.cu_seqlens != nullptr;
   const long long grid = item_per_cta ? items : std::min(items, resident);
   ::b200ait::count_launch(), attention_tc_kernel<DCH, BF16, NOMASK, LONE><<<static_cast<unsigned>(grid), kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv,
                                                                                                                  pp);

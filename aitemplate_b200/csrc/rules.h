@@ -2,11 +2,75 @@
 // its result. Plain functions of sizes, so that they can be checked without a GPU. Times: B200, fp16 unless stated.
 #pragma once
 
+#include <algorithm>
+
 namespace b200ait {
 
 // Attention, heads above 64 channels: one CTA per SM with four K / V stages instead of two CTAs with two each. Taken
 // where a second CTA would find nothing to do. One query row against 4096 keys of 96 channels, two CTAs' form -> lone:
 // 16 heads 49 -> 46 us, 64 heads 55 -> 48, 148 heads 57 -> 49; with 160 heads two CTAs on some SMs are ahead (92 -> 68).
 inline bool attn_lone(long long items, int sms) { return items <= sms; }
+
+// Attention: how the work items (128 query rows of one head of one sequence) reach the CTAs. Two CTAs per SM either walk
+// fixed shares of the items, which pays the set-up of a CTA once, or every item gets a CTA of its own, which pays it per
+// item (2 x 16 heads x 2048 rows of 64, all items alike: 57.6 us in fixed shares, 59.2) and lets the hardware hand the
+// items out as SMs fall free.
+struct AttnItems {
+  long long items;  // all of them, with the empty tiles past the end of shorter sequences
+  int q_blocks;     // tiles of a head in the longest sequence
+  int kv_blocks;    // key blocks (of 64) of the longest sequence
+  bool causal;
+  bool lengths;           // the sequences' lengths are known to the device alone (lengths_kv / lengths_q)
+  long long mean, bound;  // rows of a sequence on average, and of the longest one as the caller states it; equal if not packed
+  int d;                  // channels of a head (of q and k or of v, whichever are more)
+};
+
+// The longest fixed share of a causal problem whose sequences are all alike, in key blocks: CTA c walks items c, c + slots,
+// c + 2 slots, .., and its length depends on how slots falls on the tiles of a head.
+inline long long attn_longest_share(const AttnItems& a, int slots) {
+  long long longest = 0;
+  const long long starts = std::min<long long>(std::min(a.q_blocks, slots), a.items);  // CTAs further on start on the same tiles, with no more items
+  for (long long c = 0; c < starts; ++c) {
+    long long share = 0;
+    for (long long i = c; i < a.items; i += slots) share += std::min<long long>(a.kv_blocks, 2 * (a.q_blocks - i % a.q_blocks));
+    longest = std::max(longest, share);
+  }
+  return longest;
+}
+
+inline bool attn_item_per_cta(const AttnItems& a, int sms) {
+  const int slots = 2 * sms;
+  if (a.items <= slots) return false;  // (one and the same)
+  // Lengths the host cannot see may be short, and then the set-up is most of the time (8 x 16 heads x 4096 rows of 64 with
+  // 128 keys each: 45 us in fixed shares, 79).
+  if (a.lengths) return false;
+  if (a.mean >= a.bound) {  // every sequence is as long as the bound
+    // Equal items gain nothing (heads of 16, 32, 48, 64, 80 and 128 channels, 297 .. 591 items of 4096 rows: 0 .. 2 %
+    // slower). The exception are narrow heads whose rows are not whole 32-byte sectors: the time of their fixed shares
+    // varies with where the operands lie (512 items of 4096 rows of 40: 113 .. 134 us, handed out 111 .. 117), and with a
+    // second round of items that is not nearly empty a CTA per item is 4 % faster on average from 3072 rows on (14 % at
+    // best; 432 items of 6144 rows 8 % slower), level at 2048.
+    if (!a.causal)
+      return a.d < 48 && a.d % 16 != 0 && a.kv_blocks >= 48 && 4 * a.items >= 5ll * slots && a.items < 2ll * slots;
+    // Causal: a tile's length grows with its position, and fixed shares are as uneven as the stride falls on the heads.
+    // Handed out, the shares end about 0.6 of the longest item after their mean. Measured over 24 problems of 1024 .. 6144
+    // rows and two head widths: above 1.15 times that a CTA per item is 2 .. 27 % faster (16 heads x 2560 rows: 53.7 ->
+    // 41.1 us), below it 6 % faster .. 5 % slower (32 heads x 2048 rows: 47.1 -> 49.1).
+    long long blocks = 0;
+    for (int t = 0; t < a.q_blocks; ++t) blocks += std::min(a.kv_blocks, 2 * (t + 1));
+    const double mean_share = static_cast<double>(blocks) * (a.items / a.q_blocks) / slots;
+    const double handed_out = mean_share + 0.6 * std::min(a.kv_blocks, 2 * a.q_blocks);
+    return attn_longest_share(a, slots) > 1.15 * handed_out;
+  }
+  // Packed sequences of different lengths (or a bound above all of them, which the host cannot tell apart). An empty tile
+  // costs a CTA launch: at most half of the tiles may be empty (64 sequences of 128 rows, 12 heads x 64, bound 4096: 99 us
+  // in fixed shares, 134; 8 x 2048 rows with a bound of 16384: 150 and 156). Short items do not pay for their set-up: over
+  // evenly and randomly spread lengths of 16 heads, causal, a mean below 2048 rows runs from 29 % faster to 14 % slower,
+  // above it from 49 % faster to 2 % slower (8 sequences of 512 .. 4096 rows, 16 heads x 128: 292 -> 277 us). Without a
+  // mask nearly equal lengths lose (8 x 2048 with a bound of 2560: 8 %); from 3072 rows and a bound of 1.5 means on it is
+  // 1 .. 27 % faster.
+  if (2 * a.mean < a.bound) return false;
+  return a.causal ? a.mean >= 2048 : a.mean >= 3072 && 2 * a.bound >= 3 * a.mean;
+}
 
 }  // namespace b200ait

@@ -12,6 +12,14 @@ SMS = 148
 _WRAPPERS = """
 #include "rules.h"
 extern "C" bool attn_lone(long long items, int sms) { return b200ait::attn_lone(items, sms); }
+extern "C" bool attn_item_per_cta(long long heads, long long seqs, long long bound, long long mean, int causal, int lengths,
+                                  int d, int sms) {
+  const int q_blocks = static_cast<int>((bound + 127) / 128), kv_blocks = static_cast<int>((bound + 63) / 64);
+  return b200ait::attn_item_per_cta({heads * seqs * q_blocks, q_blocks, kv_blocks, causal != 0, lengths != 0, mean, bound, d}, sms);
+}
+extern "C" long long attn_longest_share(long long items, int q_blocks, int kv_blocks, int slots) {
+  return b200ait::attn_longest_share({items, q_blocks, kv_blocks, true, false, 0, 0, 64}, slots);
+}
 """
 
 
@@ -23,10 +31,63 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I",
                     os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     lib = ctypes.CDLL(str(lib))
-    lib.attn_lone.restype = ctypes.c_bool
+    lib.attn_lone.restype = lib.attn_item_per_cta.restype = ctypes.c_bool
+    lib.attn_longest_share.restype = ctypes.c_longlong
     return lib
 
 
 @pytest.mark.parametrize("items,lone", [(1, True), (16, True), (128, True), (148, True), (149, False), (296, False)])
 def test_wide_heads_with_an_item_per_sm_keep_four_stages(rules, items, lone):
     assert rules.attn_lone(ctypes.c_longlong(items), SMS) == lone
+
+
+@pytest.mark.parametrize(
+    "heads,seqs,bound,mean,causal,lengths,per_item",
+    [
+        # lengths on the device: they may be short, whatever the padding
+        (16, 8, 4096, 4096, False, True, False),
+        (16, 8, 4096, 4096, True, True, False),
+        # packed: a bound far above the lengths makes nearly every CTA an empty one
+        (12, 64, 4096, 128, True, False, False),
+        (12, 16, 16384, 1024, True, False, False),
+        (12, 8, 16384, 2048, False, False, False),
+        (12, 4, 32768, 4096, True, False, False),
+        # packed: short items do not pay for a set-up each
+        (16, 8, 2048, 1152, True, False, False),
+        (16, 8, 3072, 1728, True, False, False),
+        (12, 8, 2560, 2048, False, False, False),
+        # packed: long ones of different lengths do, just below 4096 rows as well as at it
+        (16, 8, 4096, 2304, True, False, True),
+        (16, 8, 4095, 2303, True, False, True),
+        (16, 6, 3000, 2225, True, False, True),
+        (12, 4, 6144, 3072, False, False, True),
+        # equal items without a mask
+        (16, 1, 4096, 4096, False, False, False),
+        (48, 1, 4096, 4096, False, False, False),
+        # causal, all sequences alike: by how uneven the shares are, at any length
+        (32, 1, 2048, 2048, True, False, False),
+        (32, 1, 4096, 4096, True, False, False),
+        (32, 1, 3072, 3072, True, False, False),
+        (16, 1, 2560, 2560, True, False, True),
+        (16, 1, 4096, 4096, True, False, True),
+        (16, 1, 4095, 4095, True, False, True),
+        (8, 1, 6144, 6144, True, False, True),
+        (8, 1, 4096, 4096, True, False, False),  # 256 items: a slot for each anyway
+    ],
+)
+def test_attention_items_get_a_cta_each_only_where_that_was_faster(rules, heads, seqs, bound, mean, causal, lengths, per_item):
+    got = rules.attn_item_per_cta(*map(ctypes.c_longlong, (heads, seqs, bound, mean)), int(causal), int(lengths), 64, SMS)
+    assert got == per_item
+
+
+@pytest.mark.parametrize("heads,s,d,per_item", [(16, 4096, 40, True), (16, 4095, 24, True), (16, 3072, 40, True), (32, 2048, 40, False),
+                                                (10, 4096, 40, False), (48, 4096, 40, False), (16, 4096, 48, False), (16, 4096, 56, False)])
+def test_equal_items_stay_in_fixed_shares_but_for_narrow_heads_of_part_sectors(rules, heads, s, d, per_item):
+    assert rules.attn_item_per_cta(*map(ctypes.c_longlong, (heads, 1, s, s)), 0, 0, d, SMS) == per_item
+
+
+@pytest.mark.parametrize("items,q_blocks,kv_blocks,slots", [(320, 20, 40, 296), (1536, 48, 96, 296), (21, 7, 9, 4), (5, 5, 10, 296), (9, 3, 5, 2)])
+def test_longest_share_is_the_longest_of_all_shares(rules, items, q_blocks, kv_blocks, slots):
+    blocks = [min(kv_blocks, 2 * (q_blocks - i % q_blocks)) for i in range(items)]
+    assert rules.attn_longest_share(ctypes.c_longlong(items), q_blocks, kv_blocks, slots) == max(
+        sum(blocks[c::slots]) for c in range(slots))
