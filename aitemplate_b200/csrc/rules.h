@@ -55,7 +55,10 @@ inline bool attn_item_per_cta(const AttnItems& a, int sms) {
     // Causal: a tile's length grows with its position, and fixed shares are as uneven as the stride falls on the heads.
     // Handed out, the shares end about 0.6 of the longest item after their mean. Measured over 24 problems of 1024 .. 6144
     // rows and two head widths: above 1.15 times that a CTA per item is 2 .. 27 % faster (16 heads x 2560 rows: 53.7 ->
-    // 41.1 us), below it 6 % faster .. 5 % slower (32 heads x 2048 rows: 47.1 -> 49.1).
+    // 41.1 us), below it 6 % faster .. 5 % slower (32 heads x 2048 rows: 47.1 -> 49.1). Shorter sequences do not pay for
+    // the set-up of their items, however uneven the shares (768 heads x 200 rows: 39.5 us in fixed shares, 42.3; 384 x 256:
+    // 23.4 and 24.5; 256 x 512: 38.9 and 39.5).
+    if (a.kv_blocks < 16) return false;
     long long blocks = 0;
     for (int t = 0; t < a.q_blocks; ++t) blocks += std::min(a.kv_blocks, 2 * (t + 1));
     const double mean_share = static_cast<double>(blocks) * (a.items / a.q_blocks) / slots;

@@ -68,6 +68,10 @@ def test_wide_heads_with_an_item_per_sm_keep_four_stages(rules, items, lone):
         (32, 1, 2048, 2048, True, False, False),
         (32, 1, 4096, 4096, True, False, False),
         (32, 1, 3072, 3072, True, False, False),
+        (768, 1, 200, 200, True, False, False),  # uneven shares, but items too short to pay for a set-up each
+        (384, 1, 256, 256, True, False, False),
+        (256, 1, 512, 512, True, False, False),
+        (192, 1, 1024, 1024, True, False, True),
         (16, 1, 2560, 2560, True, False, True),
         (16, 1, 4096, 4096, True, False, True),
         (16, 1, 4095, 4095, True, False, True),
