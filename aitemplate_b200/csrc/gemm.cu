@@ -1157,9 +1157,10 @@ void gemm_run(const GemmArgs& g_in) {
     B200AIT_CUDA_CHECK(cudaGetLastError());
     return;
   }
-  // the same for shorter rows; below K = 256 the tile kernels are level or ahead (K = 128, N = 8192: 4.8 against 3.1 .. 6.0 us)
+  // the same for shorter rows, where they are not too many (rules.h); below K = 256 the tile kernels are level or ahead (K =
+  // 128, N = 8192: 4.8 against 3.1 .. 6.0 us)
   if (tma_ok && g.batch == 1 && g.m <= kRowDotMaxM && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0 &&
-      g.k >= 256 && g.k < 1024 && g.n >= 64) {
+      gemm_rowdot_short(g.m, g.n, g.k, p.vec_ok != 0, bf16)) {
     const unsigned grid = static_cast<unsigned>(std::min<long long>(sm_count(), (g.n + 3) / 4));
 #define B200AIT_ROWDOT(MR, KV)                                                                                    \
   do {                                                                                                            \

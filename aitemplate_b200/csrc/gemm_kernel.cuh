@@ -9,6 +9,7 @@
 #include "common.h"
 #include "epilogue.cuh"
 #include "ptx.cuh"
+#include "rules.h"
 
 namespace b200ait {
 

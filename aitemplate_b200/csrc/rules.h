@@ -76,4 +76,22 @@ inline bool attn_item_per_cta(const AttnItems& a, int sms) {
   return a.causal ? a.mean >= 2048 : a.mean >= 3072 && 2 * a.bound >= 3 * a.mean;
 }
 
+// GEMM, one to four rows of X against 256 to 1023 channels: one row of W after the other on the CUDA cores, or the tensor
+// cores. The CUDA cores do M multiplications per weight and a conversion that bfloat16
+// pays twice; the tile kernels' time goes by whole key blocks of 64 channels and jumps where W leaves the L2 cache.
+// `whole`: the rows of the output are whole 16-byte units. Others cost the tile kernels 1.5 to 2 times as much, and the
+// CUDA cores nothing (4 x 80001 x 640: 31 us, tiles 46).
+// CUDA cores -> tiles, us. M = 4, fp16: 8192 x 320: 5.0 -> 6.3, 16384 x 320: 7.9 -> 6.6, 50256 x 384: 17.8 -> 10.7, 128256 x
+// 256: 29.6 -> 15.8, 50256 x 512: 17.9 -> 19.7, 128256 x 512: 39.4 -> 36.6 .. 39.0, 24576 x 640: 12.3 -> 13.6, 50256 x 576: 20.9 -> 18.1, 50256 x 776: 21.2 ->
+// 24.9. M = 4, bf16: 20480 x 320: 9.7 -> 10.1, 30520 x 320: 12.9 -> 10.7, 50256 x 576: 24.7 -> 17.9, 50256 x 512: 19.2 ->
+// 19.5, 50256 x 768: 24.1 -> 22.3, 50256 x 832: 24.6 -> 24.5. M = 2, fp16: 50256 x 256: 9.3 -> 10.7, 80000 x 256: 13.7 -> 12.1. M = 1 always gains.
+inline bool gemm_rowdot_short(long long m, long long n, long long k, bool whole, bool bf16) {
+  if (k < 256 || k >= 1024 || n < 64) return false;
+  if (m == 1 || !whole) return true;
+  if (m == 2) return bf16 || k > 384 || n <= 56000;
+  if (k <= 448) return n <= (bf16 ? 28000 : 10000);
+  if (k <= 512) return n <= 80000;
+  return k > (bf16 ? 768 : 704) || n <= 28000;
+}
+
 }  // namespace b200ait

@@ -20,6 +20,9 @@ extern "C" bool attn_item_per_cta(long long heads, long long seqs, long long bou
 extern "C" long long attn_longest_share(long long items, int q_blocks, int kv_blocks, int slots) {
   return b200ait::attn_longest_share({items, q_blocks, kv_blocks, true, false, 0, 0, 64}, slots);
 }
+extern "C" bool gemm_rowdot_short(long long m, long long n, long long k, int whole, int bf16) {
+  return b200ait::gemm_rowdot_short(m, n, k, whole != 0, bf16 != 0);
+}
 """
 
 
@@ -31,7 +34,8 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I",
                     os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     lib = ctypes.CDLL(str(lib))
-    lib.attn_lone.restype = lib.attn_item_per_cta.restype = ctypes.c_bool
+    for f in (lib.attn_lone, lib.attn_item_per_cta, lib.gemm_rowdot_short):
+        f.restype = ctypes.c_bool
     lib.attn_longest_share.restype = ctypes.c_longlong
     return lib
 
@@ -95,3 +99,23 @@ def test_longest_share_is_the_longest_of_all_shares(rules, items, q_blocks, kv_b
     blocks = [min(kv_blocks, 2 * (q_blocks - i % q_blocks)) for i in range(items)]
     assert rules.attn_longest_share(ctypes.c_longlong(items), q_blocks, kv_blocks, slots) == max(
         sum(blocks[c::slots]) for c in range(slots))
+
+
+@pytest.mark.parametrize(
+    "m,n,k,whole,bf16,row_by_row",
+    [
+        (1, 256000, 256, True, False, True), (2, 50256, 256, True, False, True), (2, 80000, 256, True, False, False),
+        (2, 128256, 384, True, True, True), (2, 128256, 392, True, False, True),
+        (3, 8192, 256, True, False, True), (4, 16384, 320, True, False, False), (3, 128256, 256, True, False, False),
+        (4, 20480, 320, True, True, True), (4, 30520, 384, True, True, False), (4, 50256, 448, True, False, False),
+        (4, 50256, 512, True, False, True), (4, 50256, 576, True, False, False), (4, 24576, 640, True, True, True),
+        (3, 128256, 512, True, True, False), (4, 128256, 704, True, True, False), (4, 50256, 768, True, True, False),
+        (4, 50256, 768, True, False, True), (4, 128256, 776, True, True, True), (3, 128256, 1016, True, False, True),
+        # rows that are not whole 16-byte units cost the tile kernels far more
+        (4, 128257, 256, False, False, True), (3, 80001, 640, False, True, True),
+        # neither fewer channels nor fewer rows, nor the longer rows of the other row-by-row kernel
+        (1, 4096, 248, True, False, False), (1, 63, 512, True, False, False), (1, 4096, 1024, True, False, False),
+    ],
+)
+def test_few_rows_against_short_ones_run_where_they_were_faster(rules, m, n, k, whole, bf16, row_by_row):
+    assert rules.gemm_rowdot_short(*map(ctypes.c_longlong, (m, n, k)), int(whole), int(bf16)) == row_by_row

@@ -32,6 +32,12 @@ def test_sizes(m, n, k, dtype):
     _check(m, n, k, dtype)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", [(2, 56008, 320), (2, 56000, 256), (3, 28008, 264), (4, 28008, 520), (3, 10008, 448), (4, 28001, 640)])
+def test_where_the_tile_kernels_take_over(m, n, k, dtype):
+    _check(m, n, k, dtype, "add")
+
+
 @pytest.mark.parametrize("epilogue", sorted(oracle.EPILOGUES))
 def test_epilogues(epilogue):
     _check(3, 777, 328, torch.float16, epilogue)
