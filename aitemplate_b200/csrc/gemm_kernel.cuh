@@ -88,7 +88,10 @@ constexpr int kGemmThreads = 64 + 32 * kEpiWarps;  // producer warp + MMA warp +
 // single-CTA 128 x 256 tile, and keeps its own 128 x BN half of the accumulator.
 // D0BOX: the residual operand d0 is fetched by TMA into the output staging boxes (two boxes per epilogue
 // warp, one ring stage fewer) and combined in place, instead of per-thread global loads.
-template <int BN, bool PAIR = false, bool D0BOX = false>
+// ROWS: the output is written row by row from staging boxes, which 64-wide tiles do not have otherwise: their 32 KB come
+// out of the L1 cache, and the other kernels' per-thread residual loads want it (32768 x 41 x 320 with two residuals: 22.3
+// us, 24.7 beside idle boxes).
+template <int BN, bool PAIR = false, bool D0BOX = false, bool ROWS = false>
 struct TileCfg {
   static_assert(!D0BOX || PAIR, "staged residual boxes are only built for the CTA-pair tile");
   static constexpr int kBRows = PAIR ? BN / 2 : BN;  // B rows this CTA loads per stage
@@ -96,11 +99,18 @@ struct TileCfg {
   static constexpr int kStages = PAIR ? (D0BOX ? 5 : 6) : (BN == 256) ? 4 : (BN == 128) ? 6 : 8;
   static constexpr int kTmemCols = 2 * BN;  // two accumulators
   static constexpr int kBoxesPerWarp = D0BOX ? 2 : 1;  // 32 rows x 64 columns x 16 bit = 4 KB each
-  static constexpr int kStagingBytes = kEpiWarps * kBoxesPerWarp * 4096;
+  static constexpr int kStagingBytes = (BN >= 128 || ROWS) ? kEpiWarps * kBoxesPerWarp * 4096 : 0;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes +
                                     2 * BN * 4 /*bias tile, fp32, one per accumulator*/;
 };
+
+// EPI of the instantiations that read the epilogue from the parameters and write the output row by row (the plain
+// generic ones do not carry that path: it cost them 5 to 10 % on outputs that never take it).
+constexpr int kRowsEpilogue = -2;
+
+static_assert(TileCfg<64>::kStagingBytes == 0 && TileCfg<64, false, false, true>::kStagingBytes == kEpiWarps * 4096,
+              "64-wide tiles have staging boxes only where something goes through them");
 
 // whether the compile-time epilogue code EPI takes its residual through staged boxes
 template <int EPI, bool PAIR>
@@ -399,10 +409,6 @@ __device__ __forceinline__ void store_box_rows(const GemmParams& p, const uint8_
   }
 }
 
-// EPI of the instantiations that read the epilogue from the parameters and write the output row by row (the plain
-// generic ones do not carry that path: it cost them 5 to 10 % on outputs that never take it).
-constexpr int kRowsEpilogue = -2;
-
 // BMN: B is stored [K, N]. MULTI: the staged store goes to p.num_out destinations. Both are compile-time, so that
 // the plain [N, K] single-destination kernels carry no trace of them (a run-time flag cost the BERT-layer GEMMs
 // 2-3 %), and both are only instantiated with the generic epilogue (EPI == -1).
@@ -414,7 +420,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   // `tma_out` is the (first) destination; `outs.m[1..]` are the extra destinations of a multi-destination store
   // and sit at the end of the parameter space, out of the way of what every launch reads.
   constexpr bool D0BOX = d0_box_of<EPI, PAIR>();
-  using Cfg = TileCfg<BN, PAIR, D0BOX>;
+  using Cfg = TileCfg<BN, PAIR, D0BOX, EPI == kRowsEpilogue>;
   constexpr int kStages = Cfg::kStages;
   constexpr uint32_t kABytes = kBM * kBK * 2;
   constexpr uint32_t kStageBytes = Cfg::kStageBytes;
@@ -887,7 +893,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 template <int BN, bool BF16, int EPI, bool BMN = false, bool MULTI = false>
 void launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout, const GemmParams& p, int grid,
                cudaStream_t stream) {
-  using Cfg = TileCfg<BN>;
+  using Cfg = TileCfg<BN, false, false, EPI == kRowsEpilogue>;
   static std::atomic<uint64_t> configured{0};
   opt_in_smem_once(configured, reinterpret_cast<const void*>(&gemm_tc_kernel<BN, BF16, EPI, false, BMN, MULTI>),
                    Cfg::kSmemBytes);
@@ -900,7 +906,7 @@ void launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout
 template <int BN, bool BF16, int EPI, bool BMN = false, bool MULTI = false>
 void launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout, const CUtensorMap& td0,
                     const GemmParams& p, int grid, cudaStream_t stream) {
-  using Cfg = TileCfg<BN, true, d0_box_of<EPI, true>()>;
+  using Cfg = TileCfg<BN, true, d0_box_of<EPI, true>(), EPI == kRowsEpilogue>;
   static std::atomic<uint64_t> configured{0};
   auto* kernel = &gemm_tc_kernel<BN, BF16, EPI, true, BMN, MULTI>;
   opt_in_smem_once(configured, reinterpret_cast<const void*>(kernel), Cfg::kSmemBytes);
