@@ -985,7 +985,8 @@ void launch_tc_pair256_bf16_lean(const CUtensorMap& ta, const CUtensorMap& tb, c
       return;                                                                                                  \
     }                                                                                                          \
     /* outputs that TMA cannot describe (64-wide tiles store 16-byte vectors per thread where they can) */     \
-    if (p.splits == 1 && (BN_ < 128 ? p.vec_ok == 0 : p.tma_store == 0)) {                                     \
+    if (p.splits == 1 && (BN_ < 128 ? p.vec_ok == 0 : p.tma_store == 0) &&                                     \
+        gemm_rows_output(p.N, BN_, epi_b1(p.epilogue) != kBinaryNone && epi_b2(p.epilogue) == kBinaryNone)) {  \
       if (bf16)                                                                                                \
         launch_tc<BN_, true, kRowsEpilogue>(ta, tb, tout, p, grid, stream);                                    \
       else                                                                                                     \

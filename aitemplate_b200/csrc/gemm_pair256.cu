@@ -24,7 +24,7 @@ void launch_tc_pair256(bool bf16, const CUtensorMap& ta, const CUtensorMap& tb, 
       launch_tc_pair<256, false, -1, true>(ta, tb, tout, td0, p, grid, stream);
     return;
   }
-  if (p.tma_store == 0) {  // written row by row
+  if (p.tma_store == 0 && gemm_rows_output(p.N, 256, epi_b1(p.epilogue) != kBinaryNone && epi_b2(p.epilogue) == kBinaryNone)) {
     if (bf16)
       launch_tc_pair<256, true, kRowsEpilogue>(ta, tb, tout, td0, p, grid, stream);
     else

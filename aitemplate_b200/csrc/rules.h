@@ -94,4 +94,14 @@ inline bool gemm_rowdot_short(long long m, long long n, long long k, bool whole,
   return k > (bf16 ? 768 : 704) || n <= 28000;
 }
 
+// GEMM, an output that TMA cannot describe: the staging boxes written row by row, or every thread its own row. Row by row
+// fills the sectors of an output of some width, but pays for 64 columns whatever the width. Every thread its own row -> row
+// by row, 32768 x N x 320 fp16, 64-wide tiles, ratio of the times: N = 3: 1.51, 17: 1.35, 33: 1.08, 41: 0.98, 47: 0.85; 3000 x
+// N x 768: 17: 1.23, 41: 1.06, 43: 1.01, 47: 0.96; with one residual, which goes through the boxes too, 17: 1.46 and 1.30, 43:
+// 1.06 and 1.07, 47: 0.97 and 1.03, 49: 0.93 and 0.99. Wider tiles give such an output half of their warps: N = 7: 1.25 ..
+// 1.6, 31: 1.0 .. 1.4, 33: 0.63 .. 1.08.
+inline bool gemm_rows_output(int n, int tile_n, bool one_residual) {
+  return n > (tile_n > 64 ? 32 : one_residual ? 47 : 42);
+}
+
 }  // namespace b200ait

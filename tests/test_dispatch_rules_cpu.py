@@ -23,6 +23,7 @@ extern "C" long long attn_longest_share(long long items, int q_blocks, int kv_bl
 extern "C" bool gemm_rowdot_short(long long m, long long n, long long k, int whole, int bf16) {
   return b200ait::gemm_rowdot_short(m, n, k, whole != 0, bf16 != 0);
 }
+extern "C" bool gemm_rows_output(int n, int tile_n, int residual) { return b200ait::gemm_rows_output(n, tile_n, residual != 0); }
 """
 
 
@@ -34,7 +35,7 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I",
                     os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     lib = ctypes.CDLL(str(lib))
-    for f in (lib.attn_lone, lib.attn_item_per_cta, lib.gemm_rowdot_short):
+    for f in (lib.attn_lone, lib.attn_item_per_cta, lib.gemm_rowdot_short, lib.gemm_rows_output):
         f.restype = ctypes.c_bool
     lib.attn_longest_share.restype = ctypes.c_longlong
     return lib
@@ -119,3 +120,10 @@ def test_longest_share_is_the_longest_of_all_shares(rules, items, q_blocks, kv_b
 )
 def test_few_rows_against_short_ones_run_where_they_were_faster(rules, m, n, k, whole, bf16, row_by_row):
     assert rules.gemm_rowdot_short(*map(ctypes.c_longlong, (m, n, k)), int(whole), int(bf16)) == row_by_row
+
+
+@pytest.mark.parametrize("n,tile_n,residual,row_by_row", [
+    (1, 64, 0, False), (17, 64, 1, False), (41, 64, 0, False), (43, 64, 1, False), (44, 64, 0, True), (49, 64, 1, True), (63, 64, 0, True),
+    (31, 128, 0, False), (31, 256, 1, False), (33, 128, 1, True), (33, 256, 0, True), (1001, 256, 1, True)])
+def test_narrow_outputs_are_written_by_their_threads(rules, n, tile_n, residual, row_by_row):
+    assert rules.gemm_rows_output(n, tile_n, residual) == row_by_row

@@ -23,7 +23,7 @@ def _close(got, want, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("tile_n", [0, 64, 128, 256, 512])
-@pytest.mark.parametrize("m,n", [(1, 9), (31, 63), (129, 65), (300, 127), (257, 129), (260, 191), (300, 257), (513, 516), (640, 1022)])
+@pytest.mark.parametrize("m,n", [(1, 9), (31, 63), (290, 33), (290, 43), (129, 49), (129, 65), (300, 127), (257, 129), (260, 191), (300, 257), (513, 516), (640, 1022)])
 def test_odd_columns(m, n, tile_n, dtype):
     from aitemplate_b200 import kernels
 
