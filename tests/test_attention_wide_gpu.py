@@ -69,3 +69,23 @@ def test_packed_sequences(causal):
 def test_an_item_per_sm(b, h, sq, skv, d, causal, lengths, dtype):
     """At most one work item per SM: the form with four K / V stages and one CTA per SM."""
     test_items_follow_one_another(b, h, sq, skv, d, causal, lengths, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [72, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,h", [(3, 40), (1, 9)])  # more items than CTAs; an item per SM
+def test_row_maxima_that_outgrow_their_reference(b, h, causal, d, dtype):
+    """Keys four times as large from block to block: the scores' spread is 1, 4, 16, 64, 256, so nearly every row's maximum
+    outgrows its reference by more than 2^8 at every block, and O, the only accumulator, is rescaled in TMEM beside a ring of
+    two stages. Bound: outputs reach |v| = 4.5; P and the output are each rounded once (2^-12 and 2^-9 relative), and a score
+    of 256 carries fp32 sums' 1e-6 of its terms, 3e-4, in both the kernel and the oracle: 4.5 (2^-11 + 6e-4) and 4.5 (2^-8 +
+    6e-4), doubled for the row sum's rounded terms."""
+    from aitemplate_b200 import kernels
+
+    s = 300
+    q, k, v = (_rand((b, h, s, d), i, dtype) for i in range(3))
+    k = (k.float() * 4.0 ** (torch.arange(s) // 64)[:, None]).to(dtype)
+    got = kernels.mem_eff_attention(q.cuda(), k.cuda(), v.cuda(), causal=causal).float().cpu()
+    err = (got - oracle.mem_eff_attention(q, k, v, causal=causal)).abs().max()
+    assert float(err) < (1e-2 if dtype == torch.float16 else 4e-2), float(err)

@@ -67,3 +67,16 @@ def test_batches(batch, m, n, k):
     dtype = torch.bfloat16
     a, b = _rand((batch, m, k), 1, dtype, 0.3), _rand((batch, n, k), 2, dtype, 0.3)
     _close(kernels.bmm_rcr(a.cuda(), b.cuda()), oracle.bmm_rcr(a, b), dtype)
+
+
+@pytest.mark.parametrize("tile_n", [64, 128, 256, 512])
+def test_several_tiles_per_cta(tile_n):
+    """102 pair tiles on 74 pairs, 204 and more on 148 CTAs: the staging box and both accumulators serve a second tile."""
+    from aitemplate_b200 import kernels
+
+    dtype, m, n, k = torch.float16, 6500, 1021, 328
+    x, w, b, d0 = _rand((m, k), 1, dtype), _rand((n, k), 2, dtype, 0.05), _rand((n,), 3, dtype), _rand((m, n), 4, dtype)
+    c = [t.cuda() for t in (x, w, b, d0)]
+    for epilogue, extra in (("relu", 0), ("add", 1)):
+        want = oracle.gemm_rcr(x, w, b, *(d0,)[:extra], epilogue=epilogue)
+        _close(kernels.gemm_rcr(*c[:3 + extra], epilogue=epilogue, tile_n=tile_n, split_k=1), want, dtype)
