@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(kRowDotThreads, 1) gemm_rowdot_kernel(const vo
   }
 }
 
-// The same for K <= 1024, where a row of W is so short that one row per warp leaves too little in flight and the
+// The same for K < 1024, where a row of W is so short that one row per warp leaves too little in flight and the
 // launch's latencies are most of the time: a warp takes up to 8 / KV rows at once (KV 16-byte vectors per lane and row,
-// eight loads in flight), its first rows are on their way before the block stages X, and all its sums are reduced
+// eight loads in flight, four with M = 3 or 4 and K = 256), its first rows are on their way before the block stages X, and all its sums are reduced
 // together. M = 1 .. 4 on the tile kernels -> here: K = 1016, N = 512: 8.2 -> 2.8 us, N = 3176: 10.6 -> 3.2 .. 4.0;
 // K = 512, N = 3176: 8.2 -> 2.9 .. 4.7; K = 256, N = 100: 7.4 -> 2.6 .. 3.9.
 constexpr int kRowDotShortThreads = 512;
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kRowDotShortThreads, 1) gemm_rowdot_short_kern
       }
     if (n0 + kWarps * kRows < n_end) fetch(n0 + kWarps * kRows);
     // Sums over the lanes, all of them at once: at every step a lane keeps one half of its values and hands over the
-    // other (31 shuffles for 32 values instead of 160), and ends with value lane / (32 / kValues).
+    // other (16 shuffles for 16 values instead of 80), and ends with value lane / (32 / kValues).
     constexpr int kValues = kRows * MR;
     float val[kValues];
 #pragma unroll

@@ -63,7 +63,8 @@ def epilogue_code(name: str) -> int:
 # The wrappers below are paid by every eager call, and most calls take the GPU less time than the wrapper took the host
 # (256 x 3072 x 768: 8.8 us of kernel behind 24.6 us of host).
 def _stream() -> int:
-    """The current device's current stream, without the Stream object torch.cuda.current_stream() builds (3.2 us)."""
+    """The current device's current stream, without the Stream object torch.cuda.current_stream() builds (3.2 us).
+    Both calls are private to PyTorch (2.11 has them)."""
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 

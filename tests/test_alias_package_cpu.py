@@ -13,8 +13,10 @@ import sys
 
 import pytest
 
+from oracle.build_ref import DEFAULT_REFERENCE
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-REFERENCE_BERT = "/root/reference/examples/03_bert/modeling/bert.py"
+REFERENCE_BERT = os.path.join(DEFAULT_REFERENCE, "examples", "03_bert", "modeling", "bert.py")
 
 
 def test_reference_import_statements_resolve_to_this_package():
