@@ -70,10 +70,11 @@ inline bool attn_item_per_cta(const AttnItems& a, int sms) {
   // in fixed shares, 134; 8 x 2048 rows with a bound of 16384: 150 and 156). Short items do not pay for their set-up: over
   // evenly and randomly spread lengths of 16 heads, causal, a mean below 2048 rows runs from 29 % faster to 14 % slower,
   // above it from 49 % faster to 2 % slower (8 sequences of 512 .. 4096 rows, 16 heads x 128: 292 -> 277 us). Without a
-  // mask nearly equal lengths lose (8 x 2048 with a bound of 2560: 8 %); from 3072 rows and a bound of 1.5 means on it is
-  // 1 .. 27 % faster.
+  // mask, over 13 sizes of five head widths and five spreads, a mean from 2048 rows on runs from 26 % faster to 6 % slower (8
+  // sequences of 512 .. 4096 rows, 16 heads x 128 in any order: 485 -> 421 us) but for nearly equal lengths, which lose up to 10 %
+  // below 2560 rows (8 x 2048 with a bound of 2560, 24 heads x 96).
   if (2 * a.mean < a.bound) return false;
-  return a.causal ? a.mean >= 2048 : a.mean >= 3072 && 2 * a.bound >= 3 * a.mean;
+  return a.mean >= 2048 && (a.causal || a.mean >= 2560 || 2 * a.bound >= 3 * a.mean);
 }
 
 // GEMM, one to four rows of X against 256 to 1023 channels: one row of W after the other on the CUDA cores, or the tensor

@@ -66,6 +66,9 @@ def test_wide_heads_with_an_item_per_sm_keep_four_stages(rules, items, lone):
         (16, 8, 4095, 2303, True, False, True),
         (16, 6, 3000, 2225, True, False, True),
         (12, 4, 6144, 3072, False, False, True),
+        (16, 8, 4096, 2304, False, False, True),
+        (16, 8, 4096, 3276, False, False, True),
+        (16, 8, 3072, 1728, False, False, False),
         # equal items without a mask
         (16, 1, 4096, 4096, False, False, False),
         (48, 1, 4096, 4096, False, False, False),
