@@ -96,9 +96,6 @@ struct AttnParams {
   // coordinate order of each tensor map: 0 = (channel, row, head, batch), 1 = (channel, head, row, batch); the host
   // picks whichever keeps the map's strides ascending
   int q_order, k_order, v_order;
-  // packed mode with a CTA per work item: a tile past the end of its sequence ends its CTA before the set-up (64 sequences
-  // of 128 rows under a bound of 4096, 12 heads: 144 -> 134 us; 8 of 512 .. 4096 rows, 16 heads of 128: 283 -> 277)
-  int skip_empty;
 };
 
 // One operand (q, k or v) as the kernel addresses it: element strides of a [batch, head, row, channel] view with
@@ -187,7 +184,10 @@ struct AttnCfg {
 // (attention_scaling_coefs_updater.h:85-165), up to the rounding of P at a different power-of-two-ish scale.
 // NOMASK: no causal mask and a key length that is a multiple of the block: every key block is "plain", and the
 // kernel is compiled without the masked softmax body (the lean variant is measurably faster than a run-time test).
-template <int DCH, bool BF16, bool NOMASK, bool LONE>
+// SKIP: packed mode with a CTA per work item, where a tile past the end of its sequence ends its CTA before the set-up (64
+// sequences of 128 rows under a bound of 4096, 12 heads: 144 -> 134 us; 8 of 512 .. 4096 rows, 16 heads of 128: 258 -> 254).
+// Compiled apart: the test slowed fixed shares that never take it (768 causal heads x 384 rows of 64: 64.6 -> 66.7 us).
+template <int DCH, bool BF16, bool NOMASK, bool LONE, bool SKIP>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                     const __grid_constant__ CUtensorMap tma_v, const AttnParams p) {
@@ -264,7 +264,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     else
       tma_load_4d(dst, map, bar, c0, w.h, row, w.b4);
   };
-  if (p.skip_empty && decode_item(blockIdx.x).n_blocks == 0) return;
+  if constexpr (SKIP) {
+    // The condition always holds, but the compiler does not know: it would keep this decoding of the first item in registers
+    // for the roles to share (8 packed causal sequences of 512 .. 4096 rows, 16 heads of 128: 250 us; 256 .. 260 so, no skip 254).
+    if (gridDim.x == p.num_items && decode_item(blockIdx.x).n_blocks == 0) return;
+  }
   const int dsteps = (p.D + 15) / 16;  // k-steps of Q K^T
 
   if (threadIdx.x == 0) {
@@ -787,6 +791,17 @@ static CUtensorMap make_attn_map(const AttnOperand& op, bool bf16, int d, long l
   return m;
 }
 
+template <int DCH, bool BF16, bool NOMASK, bool LONE, bool SKIP>
+void launch_attn_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, unsigned grid,
+                        cudaStream_t stream) {
+  auto* kernel = &attention_tc_kernel<DCH, BF16, NOMASK, LONE, SKIP>;
+  constexpr int kSmemBytes = AttnCfg<DCH, LONE>::kSmemBytes;
+  static std::atomic<uint64_t> configured{0};
+  opt_in_smem_once(configured, reinterpret_cast<const void*>(kernel), kSmemBytes);
+  ::b200ait::count_launch(), kernel<<<grid, kAttnThreads, kSmemBytes, stream>>>(tq, tk, tv, p);
+  B200AIT_CUDA_CHECK(cudaGetLastError());
+}
+
 template <int DCH, bool BF16, bool NOMASK, bool LONE = false>
 void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const AttnParams& p,
                          long long q_rows, long long kv_rows, cudaStream_t stream) {
@@ -798,8 +813,6 @@ void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnO
     }
   }
   using Cfg = AttnCfg<DCH, LONE>;
-  static std::atomic<uint64_t> configured{0};
-  opt_in_smem_once(configured, reinterpret_cast<const void*>(&attention_tc_kernel<DCH, BF16, NOMASK, LONE>), Cfg::kSmemBytes);
   const int map_batches = p.cu_seqlens ? 1 : p.B;
   CUtensorMap tq = make_attn_map(q, BF16, p.D, q_rows, p.H, map_batches, kBlockM);
   CUtensorMap tk = make_attn_map(k, BF16, p.D, kv_rows, p.H, map_batches, kBlockN);
@@ -812,11 +825,14 @@ void launch_attn_variant(const AttnOperand& q, const AttnOperand& k, const AttnO
   const AttnItems work{items, p.q_blocks, (p.Skv + kBlockN - 1) / kBlockN, p.causal != 0, p.lengths_kv || p.lengths_q,
                        p.cu_seqlens ? kv_rows / p.B : p.Skv, p.Skv, std::max(p.D, p.Dv)};
   const bool item_per_cta = attn_item_per_cta(work, sm_count());
-  pp.skip_empty = item_per_cta && p.cu_seqlens != nullptr;
-  const long long grid = item_per_cta ? items : std::min(items, resident);
-  ::b200ait::count_launch(), attention_tc_kernel<DCH, BF16, NOMASK, LONE><<<static_cast<unsigned>(grid), kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv,
-                                                                                                                 pp);
-  B200AIT_CUDA_CHECK(cudaGetLastError());
+  const unsigned grid = static_cast<unsigned>(item_per_cta ? items : std::min(items, resident));
+  if constexpr (!NOMASK && !LONE) {
+    if (item_per_cta && p.cu_seqlens) {
+      launch_attn_kernel<DCH, BF16, false, false, true>(tq, tk, tv, pp, grid, stream);
+      return;
+    }
+  }
+  launch_attn_kernel<DCH, BF16, NOMASK, LONE, false>(tq, tk, tv, pp, grid, stream);
 }
 
 template <int DCH, bool BF16>
