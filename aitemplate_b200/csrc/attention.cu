@@ -8,20 +8,20 @@
 // row sum (attention_scaling_coefs_updater.h:85-165), P rounded to 16 bits before P.V, O kept in fp32
 // and divided by the row sum at the end. S is never written to global memory.
 //
-// Persistent CTAs walk work items of 128 query rows of one (batch, head):
+// CTAs walk work items of 128 query rows of one (batch, head), in fixed shares or one each (attn_item_per_cta in rules.h):
 //   warp 0      TMA producer: the item's Q tile, then K/V blocks of kBlockN keys into a ring (AttnCfg);
 //               the next item's Q streams in while the current item drains
 //   warp 6      MMA issuer:   S = Q K^T  (tcgen05.mma, fp32 accumulator in TMEM)
 //   warp 1      MMA issuer:   O += P V   (P read from TMEM, where the softmax threads put it over the S columns
 //                             they have consumed; V as an MN-major B operand from shared memory); O stays in
 //                             TMEM for the whole item and every key block accumulates into it
-//               S and P are double-buffered: the MMAs of key block j+1 overlap the softmax of block j; O is
-//               double-buffered across items
+//               S and P are double-buffered: the MMAs of key block j+1 overlap the softmax of block j; heads of up
+//               to 64 channels double-buffer O across items
 //   warps 2-5   one thread per query row: TMEM -> registers, mask (skipped for full, unmasked blocks),
 //               reference max / row sum, exp2, P (16-bit pairs) -> TMEM; O is touched only when a row's
 //               maximum outgrows the reference by more than 2^8 (then O and the row sum are rescaled in
 //               TMEM) and once at the end of the item (O / row sum -> global memory)
-// Two CTAs share an SM so one CTA's softmax also overlaps the other's MMAs.
+// Two CTAs share an SM so one CTA's softmax also overlaps the other's MMAs (unless there are no items for a second one).
 // Shared-memory bandwidth is what the MMAs of this kernel run into (a 128 x 64 x 16 MMA with both operands in
 // shared memory reads 6 KB and issues every 48 cycles = 128 B / clk, the whole bandwidth of an SM), which is why P
 // never goes through shared memory: that removed a 16 KB write and a 16 KB read per key block.
@@ -146,7 +146,7 @@ struct AttnCfg {
   // Two CTAs share an SM whatever the head's width: they have 113 KB of shared memory and 256 TMEM columns each. What
   // the wide heads give up for it is the second Q tile, the second O and half of the K / V stages; what they gain is
   // eight softmax warps per SM instead of four (16 heads of 128, bf16: 8 packed causal sequences of 512 .. 4096 rows,
-  // one CTA with four stages and two O buffers 421 us, two CTAs 292, with a CTA per work item 280; 4 sequences of
+  // one CTA with four stages and two O buffers 421 us, two CTAs 292, with a CTA per work item 277; 4 sequences of
   // 2048 rows 186 -> 136 us).
   // A lone CTA on its SM has the shared memory of two and keeps four stages: a decode step reads K and V at the pace of
   // the loads in flight (attn_lone).
@@ -169,11 +169,11 @@ struct AttnCfg {
   static_assert(kTmemCols == 256 && kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "the CTAs of an SM fit it");
 };
 
-// Persistent CTAs: each walks work items (one item = 128 query rows of one (batch, head)) with stride
-// gridDim.x, so barrier set-up, TMEM allocation and the load latency of the first tiles are paid once
-// and the next item's Q / K / V stream in while the current item drains.
-// Pipeline (key blocks numbered globally g = 0, 1, .. across items; S and P double-buffered on g & 1, O on the
-// item's parity):
+// Each CTA walks work items (one item = 128 query rows of one (batch, head)) with stride gridDim.x. With fewer CTAs
+// than items, barrier set-up, TMEM allocation and the load latency of the first tiles are paid once and the next
+// item's Q / K / V stream in while the current item drains; with a CTA per item the walk ends after one.
+// Pipeline (key blocks numbered globally g = 0, 1, .. across items; S and P double-buffered on g & 1, O of narrow heads
+// on the item's parity):
 //   MMA warp:      S(0), S(1); then for each j: wait P(j) -> O += P(j) V(j) -> S(j+2)
 //   softmax warps: wait S(j) -> max / exp2 / row sum -> P(j) -> signal; at the item's end O / row sum -> global
 // so the tensor core computes S(j+1), S(j+2) and P(j-1) V(j-1) while the softmax threads work on block j.
@@ -483,8 +483,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     ATTN_PROBE_DECL(blockIdx.x == 0 && threadIdx.x == 64)
     // The read-out of an item's O (wait for its last P V, O / row sum -> global memory) is deferred until this thread
     // has handed the NEXT item's first P block to the tensor core: by then the last P V has long completed, so the
-    // thread never waits for it, and its TMEM loads and stores overlap the other warps' exponentials. O is
-    // double-buffered on the item's parity, which is what makes the deferral legal.
+    // thread never waits for it, and its TMEM loads and stores overlap the other warps' exponentials. What makes
+    // the deferral legal: with two O buffers the next item accumulates into the other one. With one (wide heads) its
+    // first P V waits on o_empty, which every thread signals at the end of its read-out; so the read-out has to come
+    // before the thread's p_full arrival for block 1 and before any wait on a P V of this item (a rescale, from block 1
+    // on), or the two wait for one another.
     struct Pending {
       bool valid = false;
       int it = 0, last_g = 0;   // item counter (selects the O buffer) and global index of its last key block
