@@ -215,7 +215,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   static_assert((2 + 3 * Cfg::kKvStages + 2 * 3 + 4) * 8 + 8 <= Cfg::kBarrierBytes, "barrier block overflows its shared memory");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // work item -> where its rows live and how many key blocks it walks. n_blocks == 0 (a query tile past the end of
   // a short sequence in packed mode) means the item is skipped by every role alike.
   struct Item {
@@ -368,109 +368,88 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
 #endif
   } else if (warp == 1) {
     // P V issuer: O(item) += P(g) V(g) as soon as the softmax threads have put P(g) into TMEM
-    if (lane == 0) {
-      constexpr uint32_t idesc_t = umma_idesc_f16(kBlockM, Cfg::kTWidth, BF16, false, true);  // V is MN-major
-      bool ok = true;
-      ATTN_PROBE_DECL(blockIdx.x == 0)
-      int gb = 0;  // global index of the item's first key block
-      int it = 0;
-      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-        const Item w = decode_item(item);
-        const int n_blocks = w.n_blocks;
-        if (n_blocks == 0) continue;
-        // this item's O buffer was last used by item it - kOBufs: its rows must have been read out
-        ok = mbar_wait(&o_empty[o_buf(it)], o_phase(it) ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
-        const uint32_t o_addr = tmem_o + static_cast<uint32_t>(o_buf(it) * Cfg::kTWidth);
-        for (int j = 0; ok && j < n_blocks; ++j) {
-          const int g = gb + j;
-          ATTN_PROBE(1)  // loop bookkeeping
-          ok = mbar_wait(&p_full[g & 1], (g >> 1) & 1, abort_flag, p.status, kDevWaitOtherTimeout);
-          if (Cfg::kSplitKv && ok)
-            ok = mbar_wait(&v_full[g % Cfg::kKvStages], (g / Cfg::kKvStages) & 1, abort_flag, p.status, kDevWaitFullTimeout);
-          if (!ok) break;
-          tc_fence_after();
-          ATTN_PROBE(2)  // wait for P
-          const int st = g % Cfg::kKvStages;
-          const uint32_t p_tmem = tmem_s + static_cast<uint32_t>((g & 1) * kBlockN);
-          const uint32_t v_addr = smem_u32(sKV + st * 2 * Cfg::kKBytes + Cfg::kKBytes);
+    constexpr uint32_t idesc_t = umma_idesc_f16(kBlockM, Cfg::kTWidth, BF16, false, true);  // V is MN-major
+    const uint32_t lead = elect_one();
+    bool ok = true;
+    int gb = 0;  // global index of the item's first key block
+    int it = 0;
+    for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
+      const int n_blocks = decode_item(item).n_blocks;
+      if (n_blocks == 0) continue;
+      // this item's O buffer was last used by item it - kOBufs: its rows must have been read out
+      ok = mbar_wait_warp(&o_empty[o_buf(it)], o_phase(it) ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
+      const uint32_t o_addr = tmem_o + static_cast<uint32_t>(o_buf(it) * Cfg::kTWidth);
+      for (int j = 0; ok && j < n_blocks; ++j) {
+        const int g = gb + j, st = g % Cfg::kKvStages;
+        ok = mbar_wait_warp(&p_full[g & 1], (g >> 1) & 1, abort_flag, p.status, kDevWaitOtherTimeout);
+        if (Cfg::kSplitKv && ok)
+          ok = mbar_wait_warp(&v_full[st], (g / Cfg::kKvStages) & 1, abort_flag, p.status, kDevWaitFullTimeout);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t p_tmem = tmem_s + static_cast<uint32_t>((g & 1) * kBlockN);
+        // V block rows are keys (128 B each): 16 keys per step = 2048 B; 64-wide d chunks are kBlockN * 128 B apart
+        // (leading byte offset), 8-key groups 1024 B apart (stride byte offset)
+        const uint32_t v_lo =
+            umma_smem_desc_sw128_lo(smem_u32(sKV + st * 2 * Cfg::kKBytes + Cfg::kKBytes), kBlockN * 128);
 #pragma unroll
-          for (int k = 0; k < kBlockN / 16; ++k) {
-            // A = P from TMEM: 16 keys of a row are 8 columns of 16-bit pairs.
-            // V block rows are keys (128 B each): 16 keys per step = 2048 B; 64-wide d chunks are
-            // kBlockN*128 B apart (leading byte offset), 8-key groups 1024 B apart (stride byte offset)
-            const uint64_t bdesc = umma_smem_desc_sw128(v_addr + k * 2048, kBlockN * 128, 1024);
-            umma_f16_ts(o_addr, p_tmem + k * 8, bdesc, idesc_t, (j != 0 || k != 0) ? 1u : 0u);
-          }
-          umma_commit(&kv_empty[st]);  // K/V stage free; also "P(g) V(g) is in O" for the softmax threads and the S issuer
-          ATTN_PROBE(0)  // issue of the 4 P V MMAs + commit
-        }
-        gb += n_blocks;
-        ++it;
+        for (int k = 0; k < kBlockN / 16; ++k)  // A = P from TMEM: 16 keys of a row are 8 columns of 16-bit pairs
+          umma_f16_ts_warp(o_addr, p_tmem + k * 8, v_lo + k * (2048 >> 4), idesc_t, (j != 0 || k != 0) ? 1u : 0u, lead);
+        umma_commit_warp(&kv_empty[st], lead);  // K/V stage free; also "P(g) V(g) is in O" for the softmax threads and the S issuer
       }
-      ATTN_PROBE_FLUSH(16)
-      if (!ok) {
-        umma_commit(drain_bar);
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 1000000ull) {
-        }
+      gb += n_blocks;
+      ++it;
+    }
+    if (!ok) {
+      umma_commit_warp(drain_bar, lead);
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 1000000ull) {
       }
     }
-#ifndef B200AIT_ATTN_NO_SYNCWARP
     __syncwarp();
-#endif
   } else if (warp == 6) {
-    // S issuer: S(g) = Q K(g)^T into S buffer g & 1 (g = global key-block index). A second issuing thread, so that
-    // waiting for P and issuing P V never delays the scores of the blocks ahead (and the other way round): one
-    // thread issuing both spent as long on its own waits and commits as the softmax threads on a block.
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_f16(kBlockM, kBlockN, BF16, false, false);
-      bool ok = true;
-      int gb = 0;
-      int it = 0;
-      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-        const Item w = decode_item(item);
-        const int n_blocks = w.n_blocks;
-        if (n_blocks == 0) continue;
-        const int qb = it % Cfg::kQBufs;
-        const uint32_t q_addr = smem_u32(sQ + qb * Cfg::kQBytes);
-        ok = mbar_wait(&q_full[qb], static_cast<uint32_t>(it / Cfg::kQBufs) & 1u, abort_flag, p.status, kDevWaitFullTimeout);
-        for (int j = 0; ok && j < n_blocks; ++j) {
-          const int g = gb + j;
-          const int st = g % Cfg::kKvStages;
-          // S buffer g & 1 still holds P(g - 2) until P(g - 2) V(g - 2) has completed (un-aliasing P, so that the
-          // scores only wait for the softmax threads to have loaded S(g - 2), was measured: no faster)
-          if (g >= 2)
-            ok = mbar_wait(&kv_empty[(g - 2) % Cfg::kKvStages], ((g - 2) / Cfg::kKvStages) & 1, abort_flag, p.status,
-                           kDevWaitAccEmptyTimeout);
-          if (ok) ok = mbar_wait(&kv_full[st], (g / Cfg::kKvStages) & 1, abort_flag, p.status, kDevWaitFullTimeout);
-          if (!ok) break;
-          tc_fence_after();
-#ifdef B200AIT_ATTN_PROBE
-          if (blockIdx.x == 0) g_attn_probe[20] += 1;  // S tiles issued
-#endif
-          const uint32_t k_addr = smem_u32(sKV + st * 2 * Cfg::kKBytes);
-          for (int k = 0; k < dsteps; ++k) {
-            const int c = k >> 2, kk = k & 3;
-            const uint64_t adesc = umma_smem_desc_sw128(q_addr + c * kBlockM * 128 + kk * 32, 16, 1024);
-            const uint64_t bdesc = umma_smem_desc_sw128(k_addr + c * kBlockN * 128 + kk * 32, 16, 1024);
-            umma_f16_ss(tmem_s + static_cast<uint32_t>((g & 1) * kBlockN), adesc, bdesc, idesc_s, k != 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[g & 1]);
-          if (j + 1 == n_blocks) umma_commit(&q_empty[qb]);  // every S of this item has been issued: its Q may be replaced
-        }
-        gb += n_blocks;
-        ++it;
+    // S issuer: S(g) = Q K(g)^T into S buffer g & 1 (g = global key-block index). A second issuing warp, so that
+    // waiting for P and issuing P V never delays the scores of the blocks ahead (and the other way round).
+    constexpr uint32_t idesc_s = umma_idesc_f16(kBlockM, kBlockN, BF16, false, false);
+    const uint32_t lead = elect_one();
+    bool ok = true;
+    int gb = 0;
+    int it = 0;
+    for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
+      const int n_blocks = decode_item(item).n_blocks;
+      if (n_blocks == 0) continue;
+      const int qb = it % Cfg::kQBufs;
+      const uint32_t q_lo = umma_smem_desc_sw128_lo(smem_u32(sQ + qb * Cfg::kQBytes), 16);
+      ok = mbar_wait_warp(&q_full[qb], static_cast<uint32_t>(it / Cfg::kQBufs) & 1u, abort_flag, p.status, kDevWaitFullTimeout);
+      for (int j = 0; ok && j < n_blocks; ++j) {
+        const int g = gb + j, st = g % Cfg::kKvStages;
+        // S buffer g & 1 still holds P(g - 2) until P(g - 2) V(g - 2) has completed (un-aliasing P, so that the
+        // scores only wait for the softmax threads to have loaded S(g - 2), was measured: no faster)
+        if (g >= 2)
+          ok = mbar_wait_warp(&kv_empty[(g - 2) % Cfg::kKvStages], ((g - 2) / Cfg::kKvStages) & 1, abort_flag, p.status,
+                              kDevWaitAccEmptyTimeout);
+        if (ok) ok = mbar_wait_warp(&kv_full[st], (g / Cfg::kKvStages) & 1, abort_flag, p.status, kDevWaitFullTimeout);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t k_lo = umma_smem_desc_sw128_lo(smem_u32(sKV + st * 2 * Cfg::kKBytes), 16);
+        const uint32_t s_tmem = tmem_s + static_cast<uint32_t>((g & 1) * kBlockN);
+#pragma unroll
+        for (int k = 0; k < DCH * 4; ++k)  // unrolled, so that the offsets are constants; the count is warp-uniform
+          if (k < dsteps)
+            umma_f16_ss_warp(s_tmem, q_lo + ((k >> 2) * kBlockM * 128 + (k & 3) * 32) / 16,
+                             k_lo + ((k >> 2) * kBlockN * 128 + (k & 3) * 32) / 16, idesc_s, k != 0 ? 1u : 0u, lead);
+        umma_commit_warp(&s_full[g & 1], lead);
+        if (j + 1 == n_blocks) umma_commit_warp(&q_empty[qb], lead);  // every S of this item has been issued: its Q may be replaced
       }
-      if (!ok) {
-        umma_commit(drain_bar + 1);
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(drain_bar + 1, 0) && globaltimer_ns() - t0 < 1000000ull) {
-        }
+      gb += n_blocks;
+      ++it;
+    }
+    if (!ok) {
+      umma_commit_warp(drain_bar + 1, lead);
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(drain_bar + 1, 0) && globaltimer_ns() - t0 < 1000000ull) {
       }
     }
-#ifndef B200AIT_ATTN_NO_SYNCWARP
     __syncwarp();
-#endif
   } else {
     using E = Elem16<BF16>;
     using T = typename E::T;

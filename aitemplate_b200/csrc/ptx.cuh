@@ -204,6 +204,10 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 __device__ __forceinline__ void bulk_wait_group_read0() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
+// ... all but the latest one
+__device__ __forceinline__ void bulk_wait_group_read1() {
+  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+}
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ----------------------------------------------------------------- tcgen05
@@ -245,6 +249,102 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+// ------------------------------------------------ issue by a whole, converged warp
+// The operands of a tcgen05.mma sit in uniform registers. Code under `if (lane == 0)` cannot compute there: every descriptor
+// is worked out in ordinary registers and moved over, about 60 cycles per MMA whatever its size (four 128 x 64 x 16 MMAs
+// and a commit: 290 cycles to issue, 459 to completion). So the whole warp runs the issuing code, every wait ends in a
+// vote, and only the instruction itself is predicated on the one lane chosen by elect_one(): 67 to issue, 333 to completion
+// (P from TMEM: 326 and 497 -> 60 and 245). A commit covers the MMAs of the same lane.
+__device__ __forceinline__ uint32_t elect_one() {  // 1 in one lane of a converged warp, 0 in the others
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e;
+}
+// mbar_wait by a converged warp; one answer for all lanes
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
+// Descriptors of 128-byte-swizzled tiles as their low words; the high word is the same for every tile whose 8-row groups are
+// 1024 bytes apart. `lead`: elect_one()'s answer.
+__device__ __forceinline__ uint32_t umma_smem_desc_sw128_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return ((smem_addr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
+}
+constexpr uint32_t kUmmaDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void umma_f16_ss_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                                 uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHiSw128), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_ts_warp(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc,
+                                                 uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHiSw128), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+      "r"(lead)
+      : "memory");
+}
+
+// TMA copies take their operands from uniform registers as well.
+__device__ __forceinline__ void mbar_arrive_expect_tx_warp(uint64_t* bar, uint32_t bytes, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "r"(bytes), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_warp(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar, int c0, int c1,
+                                                 int c2, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "@e cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::
+          "r"(smem_dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_warp(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar, int c0, int c1,
+                                                 int c2, int c3, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %7, 0;\n\t"
+      "@e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
+      "[%2];\n\t}" ::"r"(smem_dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(lead)
+      : "memory");
+}
+
+// `policy`: l2_policy_store()
+__device__ __forceinline__ void tma_store_5d_warp(const CUtensorMap* m, uint32_t smem_src, int c0, int c1, int c2, int c3,
+                                                  int c4, uint64_t policy, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %8, 0;\n\t"
+      "@e cp.async.bulk.tensor.5d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3, %4, %5, %6}], [%1], %7;\n\t}" ::
+          "l"(reinterpret_cast<uint64_t>(m)),
+      "r"(smem_src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "l"(policy), "r"(lead)
+      : "memory");
+}
+// how long stored lines stay in L2: as usual, or gone first
+__device__ __forceinline__ uint64_t l2_policy_store(bool streamed) {
+  uint64_t normal, first;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+  return streamed ? first : normal;
 }
 
 // ------------------------------------------------ CTA pairs (cluster of two)
@@ -305,6 +405,35 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mas
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
           smem_u32(bar)),
       "h"(cta_mask)
+      : "memory");
+}
+
+// the same three by a converged warp (see elect_one)
+__device__ __forceinline__ void tma_load_3d_pair_warp(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
+                                                      int c0, int c1, int c2, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(smem_dst),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_ss_pair_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                                      uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHiSw128), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar, uint16_t cta_mask, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(
+          smem_u32(bar)),
+      "h"(cta_mask), "r"(lead)
       : "memory");
 }
 
