@@ -389,30 +389,6 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     tmem_alloc(tmem_slot, Cfg::kTmemCols);  // two accumulators
     tmem_relinquish();
   }
-  // The TMA producer (thread 0). Every CTA reads the same rows of X: walking the k-blocks from a different starting
-  // point in every cluster keeps the CTAs from asking L2 for the same lines of X at the same moment.
-  const int nkb = kb1 - kb0;
-  int prod_stage = 0;
-  uint32_t prod_phase = 0;
-  auto produce = [&](int unit, int i0, int i1) -> bool {
-    const int slab = unit / num_groups, grp = unit - slab * num_groups;
-    // (by slab, not by unit: every group of X rows adds its k-blocks up in the same order, so a row's result does not
-    // depend on the group it falls into)
-    const int rot = nkb > 0 ? static_cast<int>((static_cast<unsigned>(slab) * 11u) % static_cast<unsigned>(nkb)) : 0;
-    for (int i = i0; i < i1; ++i) {
-      const int kb = kb0 + (i + rot >= nkb ? i + rot - nkb : i + rot);
-      if (!mbar_wait(&empty_bar[prod_stage], prod_phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout)) return false;
-      uint8_t* sw = smem + prod_stage * Cfg::kStageBytes;
-      mbar_arrive_expect_tx(&full_bar[prod_stage], Cfg::kStageBytes);
-      tma_load_3d(sw, &tma_w, &full_bar[prod_stage], kb * kBK, slab * 128, 0);
-      tma_load_3d(sw + Cfg::kWBytes, &tma_x, &full_bar[prod_stage], kb * kBK, grp * MX, 0);
-      if (++prod_stage == Cfg::kStages) {
-        prod_stage = 0;
-        prod_phase ^= 1u;
-      }
-    }
-    return true;
-  };
   tc_fence_before();
   cluster_arrive_relaxed();
   __syncthreads();
@@ -422,59 +398,79 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   bool epi_arrived = false;  // this thread has arrived at the closing cluster barrier
 
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int unit = walker; ok && unit < my_units; unit += num_walkers)
-        ok = produce(unit, 0, nkb);
-      if (!ok) {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) {
+    // TMA producer. Every CTA reads the same rows of X: walking the k-blocks from a different starting point in every
+    // cluster keeps the CTAs from asking L2 for the same lines of X at the same moment.
+    const uint32_t lead = elect_one();
+    const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar);
+    const int nkb = kb1 - kb0;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int unit = walker; ok && unit < my_units; unit += num_walkers) {
+      const int slab = unit / num_groups, grp = unit - slab * num_groups;
+      // (by slab, not by unit: every group of X rows adds its k-blocks up in the same order, so a row's result does not
+      // depend on the group it falls into)
+      const int rot = nkb > 0 ? static_cast<int>((static_cast<unsigned>(slab) * 11u) % static_cast<unsigned>(nkb)) : 0;
+      for (int i = 0; i < nkb; ++i) {
+        const int kb = kb0 + (i + rot >= nkb ? i + rot - nkb : i + rot);
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+        if (!ok) break;
+        const uint32_t sw = smem0 + static_cast<uint32_t>(stage) * Cfg::kStageBytes, bar = full0 + static_cast<uint32_t>(stage) * 8u;
+        mbar_arrive_expect_tx_warp(&full_bar[stage], Cfg::kStageBytes, lead);
+        tma_load_3d_warp(sw, &tma_w, bar, kb * kBK, slab * 128, 0, lead);
+        tma_load_3d_warp(sw + Cfg::kWBytes, &tma_x, bar, kb * kBK, grp * MX, 0, lead);
+        if (++stage == Cfg::kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
+    if (!ok) {
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) {
+      }
+    }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_f16(128, MX, BF16, false, false);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int unit = walker; ok && unit < my_units; unit += num_walkers) {
-        ok = mbar_wait(&acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
+    constexpr uint32_t idesc = umma_idesc_f16(128, MX, BF16, false, false);
+    const uint32_t lead = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int unit = walker; ok && unit < my_units; unit += num_walkers) {
+      ok = mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * Cfg::kAccCols);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, kDevWaitFullTimeout);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * Cfg::kAccCols);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.status, kDevWaitFullTimeout);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t w_addr = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint32_t x_addr = w_addr + Cfg::kWBytes;
+        const uint32_t w_addr = smem_u32(smem + stage * Cfg::kStageBytes);
+        const uint32_t w_lo = umma_smem_desc_sw128_lo(w_addr, 16), x_lo = umma_smem_desc_sw128_lo(w_addr + Cfg::kWBytes, 16);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t adesc = umma_smem_desc_sw128(w_addr + k * 32, 16, 1024);
-            const uint64_t bdesc = umma_smem_desc_sw128(x_addr + k * 32, 16, 1024);
-            umma_f16_ss(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k != 0) ? 1u : 0u);
-          }
-          umma_commit(&empty_bar[stage]);
-          if (++stage == Cfg::kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        for (int k = 0; k < kBK / 16; ++k)
+          umma_f16_ss_warp(d_tmem, w_lo + k * (32 >> 4), x_lo + k * (32 >> 4), idesc, (kb > kb0 || k != 0) ? 1u : 0u, lead);
+        umma_commit_warp(&empty_bar[stage], lead);
+        if (++stage == Cfg::kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
-        if (!ok) break;
-        umma_commit(&acc_full[acc]);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
       }
-      if (!ok) {
-        umma_commit(drain_bar);
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 1000000ull) {
-        }
+      if (!ok) break;
+      umma_commit_warp(&acc_full[acc], lead);
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
+    }
+    if (!ok) {
+      umma_commit_warp(drain_bar, lead);
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 1000000ull) {
       }
     }
+    __syncwarp();
   } else {
     // The MX rows of X are cut into H x R blocks of kSub rows; in pass h rank r finishes block h * R + r: it keeps
     // that block of its own sums and sends each peer q the block h * R + q (slot "sender" of q's `partial`, four rows
@@ -974,6 +970,8 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // loop costs the same at every width and only the epilogue shrinks with it. Per CTA the run is
 //   waves x max(main loop, epilogue) + one last epilogue,   waves = ceil(tiles / SMs),
 // so narrow tiles pay only when they save a whole wave (or the problem is all epilogue).
+// A result of this many bytes is streamed to DRAM while the kernel runs, and its stores set the pace.
+constexpr long long kStreamedBytes = 96ll << 20;
 int choose_tile_n(long long m, long long n, long long k, long long batch) {
   const long long sms = sm_count();
   const long long tm = (m + kBM - 1) / kBM;
@@ -987,7 +985,9 @@ int choose_tile_n(long long m, long long n, long long k, long long batch) {
   // K = 128 with N = 1024 / 2048: 128 against 118 / 107; K = 40 (rows of 80 bytes, padded to one k-block) with N = 2048 /
   // 4096: 141 against 125 (the wide tile fetches a quarter fewer operand rows, and TMA pays per row). So the narrow
   // tile is taken for one full k-block, and for two only on a narrow result.
-  if (n >= 128 && batch * m * n * 2 > (96ll << 20) && ((k == kBK) || (k > kBK && k <= 2 * kBK && n <= 512))) return 128;
+  // K = 32 (whole 64-byte rows): 102 us at 1024 x [512 x 512] against 125.
+  if (n >= 128 && batch * m * n * 2 > kStreamedBytes && (k <= 32 || k == kBK || (k > kBK && k <= 2 * kBK && n <= 512)))
+    return 128;
   int best = 256;
   long long best_cost = -1;
   for (int bn : {256, 128, 64}) {
@@ -998,6 +998,15 @@ int choose_tile_n(long long m, long long n, long long k, long long batch) {
     if (best_cost < 0 || cost < best_cost) best = bn, best_cost = cost;
   }
   return best;
+}
+
+// How many stages of its operand ring a launch uses, where that is fewer than the kernel has. One k-block per tile: the ring
+// runs ahead of the stores by as many tiles as it has stages, and operands fetched far ahead of use compete with the result
+// for DRAM. 1024 x [512 x 512 x 64], us with 2 / 3 / 4 / 6 stages of 128-wide tiles: 127 / 121 / 135 / 134; 768 x [384 x 384
+// x 64]: 56 / 52 / 59 / 61; 300 x [512 x 512 x 64]: 43 / 37 / 39 / 39. Smaller results are level, K = 32 is (103 / 102), two
+// k-blocks per tile want all six (512 x [512 x 512 x 128]: 93 / 75 / 73 / 70), other widths show nothing clear.
+int operand_ring_limit(long long out_bytes, long long k, int tile_n) {
+  return out_bytes > kStreamedBytes && k <= kBK && tile_n == 128 ? 3 : 64;
 }
 
 // Split-K plan: how many K-splits a problem gets and the fp32 workspace they need.
@@ -1281,6 +1290,10 @@ void gemm_run(const GemmArgs& g_in) {
   p.tiles_n = (p.N + bn - 1) / bn;
   p.num_tiles = p.tiles_m * p.tiles_n * p.batch;
   p.num_units = p.num_tiles * p.splits;
+  const FastDiv by_batch(p.tiles_m * p.tiles_n), by_group(kGroupM * p.tiles_n), by_rest(std::max(1, p.tiles_m % kGroupM));
+  p.batch_mul = by_batch.mul, p.batch_shr = by_batch.shr, p.group_mul = by_group.mul, p.group_shr = by_group.shr;
+  p.rest_mul = by_rest.mul, p.rest_shr = by_rest.shr;
+  p.ring_limit = operand_ring_limit(g.batch * g.m * g.n * 2, g.k, pair ? 0 : bn);
   const int grid = pair ? 2 * std::min(p.num_units, sm_count() / 2) : std::min(p.num_units, sm_count());
   CUtensorMap td0 = ta;
   p.tma_d0 = 0;

@@ -16,6 +16,7 @@ namespace b200ait {
 struct GemmParams {
   int M, N, K, batch;
   int tiles_m, tiles_n, num_tiles;
+  unsigned batch_mul, batch_shr, group_mul, group_shr, rest_mul, rest_shr;  // FastDiv constants of decode_tile
   int splits, kb_per_split, num_units;  // split-K: unit = tile * splits + split
   float* partial;                       // [splits, batch, M, N] fp32 partial sums when splits > 1
   int a_batch_mul, b_batch_mul;  // 0 when that operand is broadcast over the batch
@@ -37,6 +38,7 @@ struct GemmParams {
   int vec_ok;  // 16-byte epilogue accesses are legal
   int tma_store;  // output goes through shared memory + TMA store (tensor maps `outs`)
   int num_out;    // destinations of the staged store (1 unless the caller passed several output buffers)
+  int ring_limit;  // stages of the operand ring in use, where the kernel has more
   int tma_d0;     // the residual d0 arrives by TMA in the output staging boxes (tensor map `tma_d0`)
   int* status;
   // batched "0213" store (bmm_*_permute): batch b = hi * c_bdiv + lo lands at hi * c_bs_hi + lo * c_bs, rows ldc
@@ -79,7 +81,7 @@ static __device__ long long g_gemm_probe[32];  // one copy per translation unit 
 #endif
 
 constexpr int kBK = 64;
-constexpr int kGroupM = 8;
+constexpr int kGroupM = 8;  // row blocks whose tiles run side by side
 constexpr int kEpiWarps = 8;                      // two per TMEM lane quarter, each takes half of the columns
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;  // producer warp + MMA warp + epilogue warps
 
@@ -118,17 +120,18 @@ __host__ __device__ constexpr bool d0_box_of() {
   return PAIR && EPI >= 0 && epi_b1(EPI) != kBinaryNone && epi_b2(EPI) == kBinaryNone;
 }
 
+// tile -> (batch, row block, column block), in groups of kGroupM row blocks. Every role decodes each of its tiles, the
+// epilogue warps between two tiles: by multiply-high with constants of the host (three divisions took about 400 cycles).
 __device__ __forceinline__ void decode_tile(const GemmParams& p, int tile, int& b, int& m_blk, int& n_blk) {
   const int per_batch = p.tiles_m * p.tiles_n;
-  b = tile / per_batch;
+  b = fast_div(tile, per_batch, p.batch_mul, p.batch_shr);
   const int t = tile - b * per_batch;
   const int group_size = kGroupM * p.tiles_n;
-  const int g = t / group_size;
-  const int first_m = g * kGroupM;
-  const int gm = min(kGroupM, p.tiles_m - first_m);
+  const int g = fast_div(t, group_size, p.group_mul, p.group_shr);
+  const int first_m = g * kGroupM, gm = p.tiles_m - first_m;
   const int r = t - g * group_size;
-  m_blk = first_m + r % gm;
-  n_blk = r / gm;
+  n_blk = gm >= kGroupM ? r / kGroupM : fast_div(r, gm, p.rest_mul, p.rest_shr);  // the last group is smaller
+  m_blk = first_m + r - n_blk * min(gm, kGroupM);
 }
 
 // offset (in elements) of batch b of the output
@@ -422,6 +425,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   constexpr bool D0BOX = d0_box_of<EPI, PAIR>();
   using Cfg = TileCfg<BN, PAIR, D0BOX, EPI == kRowsEpilogue>;
   constexpr int kStages = Cfg::kStages;
+  const int ring = min(kStages, p.ring_limit);
   constexpr uint32_t kABytes = kBM * kBK * 2;
   constexpr uint32_t kStageBytes = Cfg::kStageBytes;
 
@@ -452,7 +456,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   static_assert((2 * kStages + 5 + 2 * kEpiWarps) * 8 + 8 <= Cfg::kBarrierBytes, "barrier area too small");
   float* sbias = reinterpret_cast<float*>(staging + Cfg::kStagingBytes + Cfg::kBarrierBytes);  // [2][BN]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be uniform
   const int lane = threadIdx.x & 31;
   const int num_kb = (p.K + kBK - 1) / kBK;
 #ifdef B200AIT_GEMM_PROBE
@@ -501,84 +505,88 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int unit = walker; ok && unit < num_units; unit += num_walkers) {
-        int b, m_blk, n_blk;
-        const int tile = unit / splits, split = unit - tile * splits;
-        decode_tile(p, tile, b, m_blk, n_blk);
-        if (PAIR) m_blk = 2 * m_blk + pair_rank;
-        const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
-          if (!ok) break;
-          uint8_t* sa = smem + stage * kStageBytes;
-          if (PAIR) {
-            // Both CTAs' copies are credited to the leader's barrier, which expects the bytes of both.
-            const uint32_t leader_bar = mapa_shared(smem_u32(&full_bar[stage]), 0);
-            if (pair_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * kStageBytes);
-            tma_load_3d_pair(sa, &tma_a, leader_bar, kb * kBK, m_blk * kBM, b * p.a_batch_mul);
-            const int n0 = n_blk * BN + pair_rank * (BN / 2);
-            if (BMN) {  // [K, N] storage: one box of 64 k-rows x 64 columns per 64-column chunk
+    // Loads, MMAs and stores are issued by a whole converged warp (elect_one in ptx.cuh): by one lane of a divergent branch, a
+    // k-block cost the producer or the MMA issuer about 420 cycles however narrow the tile. 1055 x 768 x 3072 + add 19.5 ->
+    // 12.2 us, 2048 x 320 x 1280 10.7 -> 7.3, 24576 x 3072 x 768 + fast_gelu 99 -> 90.
+    const uint32_t lead = elect_one();
+    const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar);
+    // Both CTAs' copies of a pair are credited to the leader's barrier, which expects the bytes of both.
+    const uint32_t full0_of_leader = PAIR ? __shfl_sync(0xffffffffu, mapa_shared(full0, 0), 0) : full0;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int unit = walker; ok && unit < num_units; unit += num_walkers) {
+      int b, m_blk, n_blk;
+      const int tile = unit / splits, split = unit - tile * splits;
+      decode_tile(p, tile, b, m_blk, n_blk);
+      if (PAIR) m_blk = 2 * m_blk + pair_rank;
+      const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
+      const int m0 = m_blk * kBM, n0 = n_blk * BN + (PAIR ? pair_rank * (BN / 2) : 0);
+      const int a_b = b * p.a_batch_mul, b_b = b * p.b_batch_mul;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+        if (!ok) break;
+        const uint32_t sa = smem0 + static_cast<uint32_t>(stage) * kStageBytes, sb = sa + kABytes;
+        const uint32_t bar = full0_of_leader + static_cast<uint32_t>(stage) * 8u;
+        if (PAIR) {
+          if (pair_rank == 0) mbar_arrive_expect_tx_warp(&full_bar[stage], 2 * kStageBytes, lead);
+          tma_load_3d_pair_warp(sa, &tma_a, bar, kb * kBK, m0, a_b, lead);
+          if (BMN) {  // [K, N] storage: one box of 64 k-rows x 64 columns per 64-column chunk
 #pragma unroll
-              for (int ch = 0; ch < Cfg::kBRows / 64; ++ch)
-                tma_load_3d_pair(sa + kABytes + ch * 8192, &tma_b, leader_bar, n0 + ch * 64, kb * kBK,
-                                 b * p.b_batch_mul);
-            } else {
-              tma_load_3d_pair(sa + kABytes, &tma_b, leader_bar, kb * kBK, n0, b * p.b_batch_mul);
-            }
+            for (int ch = 0; ch < Cfg::kBRows / 64; ++ch)
+              tma_load_3d_pair_warp(sb + ch * 8192, &tma_b, bar, n0 + ch * 64, kb * kBK, b_b, lead);
           } else {
-            mbar_arrive_expect_tx(&full_bar[stage], kStageBytes);
-            tma_load_3d(sa, &tma_a, &full_bar[stage], kb * kBK, m_blk * kBM, b * p.a_batch_mul);
-            if (BMN) {
+            tma_load_3d_pair_warp(sb, &tma_b, bar, kb * kBK, n0, b_b, lead);
+          }
+        } else {
+          mbar_arrive_expect_tx_warp(&full_bar[stage], kStageBytes, lead);
+          tma_load_3d_warp(sa, &tma_a, bar, kb * kBK, m0, a_b, lead);
+          if (BMN) {
 #pragma unroll
-              for (int ch = 0; ch < Cfg::kBRows / 64; ++ch)
-                tma_load_3d(sa + kABytes + ch * 8192, &tma_b, &full_bar[stage], n_blk * BN + ch * 64, kb * kBK,
-                            b * p.b_batch_mul);
-            } else {
-              tma_load_3d(sa + kABytes, &tma_b, &full_bar[stage], kb * kBK, n_blk * BN, b * p.b_batch_mul);
-            }
+            for (int ch = 0; ch < Cfg::kBRows / 64; ++ch)
+              tma_load_3d_warp(sb + ch * 8192, &tma_b, bar, n0 + ch * 64, kb * kBK, b_b, lead);
+          } else {
+            tma_load_3d_warp(sb, &tma_b, bar, kb * kBK, n0, b_b, lead);
           }
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        if (++stage == ring) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      if (PAIR) {
-        // The leader's MMA commits release stages in BOTH CTAs: wait until every release addressed to this
-        // CTA has landed, so that none arrives after the CTA has gone.
-        for (int s = 0; ok && s < kStages; ++s) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+    }
+    if (PAIR) {
+      // The leader's MMA commits release stages in BOTH CTAs: wait until every release addressed to this
+      // CTA has landed, so that none arrives after the CTA has gone.
+      for (int s = 0; ok && s < ring; ++s) {
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+        if (++stage == ring) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      if (!ok) {
-        // give copies that are still in flight a bounded time to land before the CTA exits
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) {
-        }
+    }
+    if (!ok) {
+      // give copies that are still in flight a bounded time to land before the CTA exits
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) {
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0 && pair_rank == 0) {
+    if (pair_rank == 0) {
       constexpr uint32_t idesc = umma_idesc_f16(PAIR ? 2 * kBM : kBM, BN, BF16, false, BMN);
+      const uint32_t lead = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      GEMM_PROBE_DECL(blockIdx.x == 0)
+      GEMM_PROBE_DECL(blockIdx.x == 0 && lane == 0)
       for (int unit = walker; ok && unit < num_units; unit += num_walkers) {
         GEMM_PROBE(3)  // other
-        ok = mbar_wait(&acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
+        ok = mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, kDevWaitAccEmptyTimeout);
         if (!ok) break;
         tc_fence_after();
         GEMM_PROBE(0)  // waiting for a free accumulator
@@ -587,40 +595,40 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
           GEMM_PROBE(2)  // issuing MMAs and commits
-          ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.status, kDevWaitFullTimeout);
+          ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, kDevWaitFullTimeout);
           if (!ok) break;
           tc_fence_after();
           GEMM_PROBE(1)  // waiting for operands
           const uint32_t a_addr = smem_u32(smem + stage * kStageBytes);
-          const uint32_t b_addr = a_addr + kABytes;
+          const uint32_t a_lo = umma_smem_desc_sw128_lo(a_addr, 16);
+          // [N, K] storage: K-major tile, 32 bytes per k-step. [K, N] storage: MN-major tile, rows are k (128 B
+          // each): 16 k-rows = 2048 B per k-step, 64-column chunks 8192 B apart, 8-row groups 1024 B apart.
+          const uint32_t b_lo = umma_smem_desc_sw128_lo(a_addr + kABytes, BMN ? 8192 : 16);
+          constexpr uint32_t kBStep = (BMN ? 2048 : 32) >> 4;
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t adesc = umma_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-            // [N, K] storage: K-major tile, 32 bytes per k-step. [K, N] storage: MN-major tile, rows are k (128 B
-            // each): 16 k-rows = 2048 B per k-step, 64-column chunks 8192 B apart, 8-row groups 1024 B apart.
-            const uint64_t bdesc = BMN ? umma_smem_desc_sw128(b_addr + k * 2048, 8192, 1024)
-                                       : umma_smem_desc_sw128(b_addr + k * 32, 16, 1024);
+            const uint32_t accumulate = (kb > kb0 || k != 0) ? 1u : 0u;
             if (PAIR) {
-              umma_f16_ss_pair(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k != 0) ? 1u : 0u);
+              umma_f16_ss_pair_warp(d_tmem, a_lo + k * (32 >> 4), b_lo + k * kBStep, idesc, accumulate, lead);
             } else {
-              umma_f16_ss(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k != 0) ? 1u : 0u);
+              umma_f16_ss_warp(d_tmem, a_lo + k * (32 >> 4), b_lo + k * kBStep, idesc, accumulate, lead);
             }
           }
           if (PAIR) {
-            umma_commit_pair(&empty_bar[stage], 3);  // frees this stage in both CTAs
+            umma_commit_pair_warp(&empty_bar[stage], 3, lead);  // frees this stage in both CTAs
           } else {
-            umma_commit(&empty_bar[stage]);
+            umma_commit_warp(&empty_bar[stage], lead);
           }
-          if (++stage == kStages) {
+          if (++stage == ring) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (!ok) break;
         if (PAIR) {
-          umma_commit_pair(&acc_full[acc], 3);  // both CTAs' epilogues read their half
+          umma_commit_pair_warp(&acc_full[acc], 3, lead);  // both CTAs' epilogues read their half
         } else {
-          umma_commit(&acc_full[acc]);
+          umma_commit_warp(&acc_full[acc], lead);
         }
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
@@ -628,14 +636,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       }
       GEMM_PROBE_FLUSH(0)
 #ifdef B200AIT_GEMM_PROBE
-      if (blockIdx.x == 0) g_gemm_probe[16] = clock64();  // end of the MMA thread's work
+      if (blockIdx.x == 0 && lane == 0) g_gemm_probe[16] = clock64();  // end of the MMA thread's work
 #endif
       if (!ok) {
         // let MMAs that were already issued finish before TMEM is released
         if (PAIR) {
-          umma_commit_pair(drain_bar, 1);
+          umma_commit_pair_warp(drain_bar, 1, lead);
         } else {
-          umma_commit(drain_bar);
+          umma_commit_warp(drain_bar, lead);
         }
         const uint64_t t0 = globaltimer_ns();
         while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < 1000000ull) {
@@ -663,6 +671,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     // residual through staging boxes: needs the TMA store path and a tensor map over d0
     const bool box_d0 = D0BOX && (kLean || (use_tma && p.tma_d0 != 0));
     uint8_t* my_staging = staging + ew * (Cfg::kBoxesPerWarp * 4096);
+    const uint32_t my_staging_u32 = smem_u32(my_staging);
+    const uint32_t lead = elect_one();
     uint64_t* my_d0_bar = d0_bar + 2 * ew;
     uint32_t d0_phase_bits = 0;  // bit i: parity to wait for on my_d0_bar[i]
     int acc = 0;
@@ -682,18 +692,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       if (box_d0) {
         // Fetch this warp's two 32 x 64 residual boxes into its staging buffers while the tile's MMAs run.
         // The previous tile's stores must have finished reading the buffers first.
-        if (lane == 0) {
-          bulk_wait_group_read0();
+        if (lead) bulk_wait_group_read0();
+        __syncwarp();
 #pragma unroll
-          for (int bx = 0; bx < 2; ++bx) {
-            const int gcol = colh + bx * 64;
-            if (row0 < p.M && gcol < p.N) {
-              mbar_arrive_expect_tx(&my_d0_bar[bx], 4096);
-              tma_load_3d(my_staging + bx * 4096, &tma_d0, &my_d0_bar[bx], gcol, row0, b);
-            }
+        for (int bx = 0; bx < 2; ++bx) {
+          const int gcol = colh + bx * 64;
+          if (row0 < p.M && gcol < p.N) {
+            mbar_arrive_expect_tx_warp(&my_d0_bar[bx], 4096, lead);
+            tma_load_3d_warp(my_staging_u32 + bx * 4096, &tma_d0, smem_u32(&my_d0_bar[bx]), gcol, row0, b, lead);
           }
         }
-        __syncwarp();
       }
       float* bias_s = sbias + acc * BN;
       if (has_bias) {  // CTA-uniform
@@ -784,7 +792,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         if (use_tma) {
           // Stage this warp's 32 rows x 64 columns (two chunks) in 128-byte-swizzled shared memory and
           // let TMA write the box: full 128-byte lines reach L2, rows / columns past M / N are clipped.
-          uint8_t* box = my_staging + (box_d0 ? (c >> 1) * 4096 : 0);
+          const int box_at = box_d0 ? (c >> 1) * 4096 : 0;
+          uint8_t* box = my_staging + box_at;
           uint8_t* row_base = box + lane * 128;
           if (box_d0) {
             // the residual box sits where the output box will be written: combine in place
@@ -800,7 +809,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           }
           epilogue_math32<BF16, EPI>(p, v, d0c, b, row, col0, full || box_d0, row_ok);
           if (!box_d0 && (c & 1) == 0) {  // the box buffer is about to be rewritten: its last store must have read it
-            if (lane == 0) bulk_wait_group_read0();
+            if (lead) bulk_wait_group_read0();
             __syncwarp();
           }
 #pragma unroll
@@ -811,22 +820,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           if ((c & 1) != 0 || col0 + 32 >= p.N) {
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0 && row0 < p.M) {  // a box that starts past the last row has nothing to write
+            if (row0 < p.M) {  // a box that starts past the last row has nothing to write
               const int gcol = colh + (c & ~1) * 32;
+              const uint32_t src = my_staging_u32 + box_at;
               if (p.store_mode == 0) {
                 int b_lo = b, b_hi = 0;
                 if (EPI < 0 && p.c_bdiv != 0) b_hi = b / p.c_bdiv, b_lo = b - b_hi * p.c_bdiv;
-                tma_store_5d(&tma_out, box, gcol, row0, b_lo, b_hi, 0);
+                tma_store_5d_warp(&tma_out, src, gcol, row0, b_lo, b_hi, 0, lead);
                 if (MULTI)
-                  for (int i = 1; i < p.num_out; ++i) tma_store_5d(&outs.m[i], box, gcol, row0, b, 0, 0);
+                  for (int i = 1; i < p.num_out; ++i) tma_store_5d_warp(&outs.m[i], src, gcol, row0, b, 0, 0, lead);
               } else {
-                const int cc = gcol / p.d, r_b = row0 / p.t1;
-                tma_store_5d(&tma_out, box, gcol - cc * p.d, row0 - r_b * p.t1, cc % p.t3, r_b, cc / p.t3);
+                const int cc = gcol / p.d, r_b = row0 / p.t1, c2 = cc / p.t3;
+                tma_store_5d_warp(&tma_out, src, gcol - cc * p.d, row0 - r_b * p.t1, cc - c2 * p.t3, r_b, c2, lead);
                 if (MULTI)
                   for (int i = 1; i < p.num_out; ++i)
-                    tma_store_5d(&outs.m[i], box, gcol - cc * p.d, row0 - r_b * p.t1, cc % p.t3, r_b, cc / p.t3);
+                    tma_store_5d_warp(&outs.m[i], src, gcol - cc * p.d, row0 - r_b * p.t1, cc - c2 * p.t3, r_b, c2, lead);
               }
-              bulk_commit_group();
+              if (lead) bulk_commit_group();
             }
           }
         } else if constexpr (EPI == kRowsEpilogue) {
@@ -874,7 +884,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 #ifdef B200AIT_GEMM_PROBE
     if (blockIdx.x == 0 && threadIdx.x == 64) g_gemm_probe[17] = clock64();
 #endif
-    if (use_tma && lane == 0) bulk_wait_group0();  // shared memory must outlive the stores that read it
+    if (use_tma && lead) bulk_wait_group0();  // shared memory must outlive the stores that read it
   }
 
   tc_fence_before();

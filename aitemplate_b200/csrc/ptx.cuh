@@ -135,13 +135,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     }
   }
 }
-// One 32-bit word into the shared memory of a CTA of this cluster, asynchronously: the 4 bytes are credited to the
-// mbarrier at `cluster_bar` (same CTA as the destination) when they have landed, so the sender orders nothing.
-__device__ __forceinline__ void st_async_cluster_b32(uint32_t cluster_addr, uint32_t v, uint32_t cluster_bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr),
-               "r"(v), "r"(cluster_bar)
-               : "memory");
-}
 // Four consecutive 32-bit words (16-byte aligned), same contract: 16 bytes credited.
 __device__ __forceinline__ void st_async_cluster_v4(uint32_t cluster_addr, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3,
                                                     uint32_t cluster_bar) {
@@ -157,29 +150,9 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_add
 // the cluster-wide barrier in two halves (every thread of every CTA of the cluster executes each exactly once)
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-// one fp32 word into the shared memory of a CTA of this cluster (address from mapa_shared)
-__device__ __forceinline__ void st_shared_cluster_f32(uint32_t cluster_addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
-}
-
 // --------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
-                                            int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
-          "r"(smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1,
                                             int c2, int c3) {
@@ -190,23 +163,10 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
-// TMA store of one box from shared memory (bulk-group completion)
-__device__ __forceinline__ void tma_store_5d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2,
-                                             int c3, int c4) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(
-          reinterpret_cast<uint64_t>(m)),
-      "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
-      : "memory");
-}
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // waits until the bulk groups of this thread have finished READING their shared-memory source
 __device__ __forceinline__ void bulk_wait_group_read0() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-// ... all but the latest one
-__device__ __forceinline__ void bulk_wait_group_read1() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
@@ -225,32 +185,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]; accumulate==0 overwrites D.
-__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// the mbarrier receives one arrival when every tcgen05 op issued so far by this thread is done
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
 // ------------------------------------------------ issue by a whole, converged warp
 // The operands of a tcgen05.mma sit in uniform registers. Code under `if (lane == 0)` cannot compute there: every descriptor
 // is worked out in ordinary registers and moved over, about 60 cycles per MMA whatever its size (four 128 x 64 x 16 MMAs
@@ -268,12 +202,17 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
 }
-// Descriptors of 128-byte-swizzled tiles as their low words; the high word is the same for every tile whose 8-row groups are
-// 1024 bytes apart. `lead`: elect_one()'s answer.
+// Shared-memory matrix descriptor of a 128-byte-swizzled tile whose rows are 128 bytes (64 half elements) apart:
+//   bits  0-13 start address >> 4      bits 16-29 leading byte offset >> 4
+//   bits 32-45 stride byte offset >> 4 bits 46-47 descriptor version (1 on sm_100)
+//   bits 61-63 swizzle mode (2 = 128 B)
+// Passed as its low word; the high word is the same for every tile here (8-row groups 1024 bytes apart).
 __device__ __forceinline__ uint32_t umma_smem_desc_sw128_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
 constexpr uint32_t kUmmaDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+// `lead`: elect_one()'s answer.
+// D[tmem] (+)= A[smem] * B[smem]; accumulate == 0 overwrites D
 __device__ __forceinline__ void umma_f16_ss_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                                  uint32_t accumulate, uint32_t lead) {
   asm volatile(
@@ -284,6 +223,7 @@ __device__ __forceinline__ void umma_f16_ss_warp(uint32_t d_tmem, uint32_t a_lo,
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHiSw128), "r"(lead)
       : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem]
 __device__ __forceinline__ void umma_f16_ts_warp(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc,
                                                  uint32_t accumulate, uint32_t lead) {
   asm volatile(
@@ -294,6 +234,7 @@ __device__ __forceinline__ void umma_f16_ts_warp(uint32_t d_tmem, uint32_t a_tme
       "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHiSw128), "r"(lead)
       : "memory");
 }
+// the mbarrier receives one arrival when every tcgen05 op issued so far by the elected lane is done
 __device__ __forceinline__ void umma_commit_warp(uint64_t* bar, uint32_t lead) {
   asm volatile(
       "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
@@ -329,22 +270,15 @@ __device__ __forceinline__ void tma_load_4d_warp(uint32_t smem_dst, const CUtens
       : "memory");
 }
 
-// `policy`: l2_policy_store()
+// TMA store of one box from shared memory (bulk-group completion)
 __device__ __forceinline__ void tma_store_5d_warp(const CUtensorMap* m, uint32_t smem_src, int c0, int c1, int c2, int c3,
-                                                  int c4, uint64_t policy, uint32_t lead) {
+                                                  int c4, uint32_t lead) {
   asm volatile(
-      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %8, 0;\n\t"
-      "@e cp.async.bulk.tensor.5d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3, %4, %5, %6}], [%1], %7;\n\t}" ::
-          "l"(reinterpret_cast<uint64_t>(m)),
-      "r"(smem_src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "l"(policy), "r"(lead)
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %7, 0;\n\t"
+      "@e cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];\n\t}" ::"l"(
+          reinterpret_cast<uint64_t>(m)),
+      "r"(smem_src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(lead)
       : "memory");
-}
-// how long stored lines stay in L2: as usual, or gone first
-__device__ __forceinline__ uint64_t l2_policy_store(bool streamed) {
-  uint64_t normal, first;
-  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
-  return streamed ? first : normal;
 }
 
 // ------------------------------------------------ CTA pairs (cluster of two)
@@ -365,19 +299,6 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// TMA load issued by either CTA of a pair; the byte count is credited to the mbarrier at
-// `bar_cluster_addr`, which may live in the peer CTA. No multicast: the data lands in the issuing CTA.
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
-                                                 int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
                "r"(ncols)
@@ -389,26 +310,8 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// D (256 rows: 128 in each CTA's TMEM) (+)= A (128 rows per CTA) * B (N/2 rows per CTA)
-__device__ __forceinline__ void umma_f16_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// one arrival on the mbarrier at this shared-memory offset in every CTA of `cta_mask`
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(cta_mask)
-      : "memory");
-}
-
-// the same three by a converged warp (see elect_one)
+// TMA load by either CTA of a pair; the byte count is credited to the mbarrier at `bar_cluster_addr`, which may live in the
+// peer CTA. No multicast: the data lands in the issuing CTA.
 __device__ __forceinline__ void tma_load_3d_pair_warp(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
                                                       int c0, int c1, int c2, uint32_t lead) {
   asm volatile(
@@ -418,6 +321,7 @@ __device__ __forceinline__ void tma_load_3d_pair_warp(uint32_t smem_dst, const C
       "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(lead)
       : "memory");
 }
+// D (256 rows: 128 in each CTA's TMEM) (+)= A (128 rows per CTA) * B (N/2 rows per CTA)
 __device__ __forceinline__ void umma_f16_ss_pair_warp(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                                       uint32_t accumulate, uint32_t lead) {
   asm volatile(
@@ -428,6 +332,7 @@ __device__ __forceinline__ void umma_f16_ss_pair_warp(uint32_t d_tmem, uint32_t 
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(kUmmaDescHiSw128), "r"(lead)
       : "memory");
 }
+// one arrival on the mbarrier at this shared-memory offset in every CTA of `cta_mask`
 __device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar, uint16_t cta_mask, uint32_t lead) {
   asm volatile(
       "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
@@ -435,21 +340,6 @@ __device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar, uint16_t ct
           smem_u32(bar)),
       "h"(cta_mask), "r"(lead)
       : "memory");
-}
-
-// Shared-memory matrix descriptor for a 128-byte-swizzled tile whose rows are
-// 128 bytes (64 half elements) apart and whose 8-row groups are `sbo` bytes apart.
-//   bits  0-13 start address >> 4      bits 16-29 leading byte offset >> 4
-//   bits 32-45 stride byte offset >> 4 bits 46-47 descriptor version (1 on sm_100)
-//   bits 61-63 swizzle mode (2 = 128 B)
-__device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
 }
 
 // Instruction descriptor for kind::f16 with fp32 accumulation.
