@@ -352,7 +352,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   static_assert((2 * Cfg::kStages + 9) * 8 + 8 <= 256, "barrier area too small");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());
   const int walker = blockIdx.x / R, num_walkers = gridDim.x / R;
   // a unit of work: one slab of 128 weight rows against one group of MX rows of X (consecutive units share the slab,
@@ -365,16 +365,11 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 
   // Set-up, kept short because a small problem's whole run is a few microseconds: the lanes of warp 0 initialise one
   // barrier each while warp 1 allocates tensor memory, and the opening cluster barrier is arrived at without a release
-  // (the initialisations are published by fence.mbarrier_init; a releasing arrive alone was measured at 0.5 us):
-  // 0.68 us from the CTA's start to its first instruction after the set-up, 1.26 us with everything done in turn.
-  // (Letting the producer thread start streaming before the set-up barriers changed nothing: the first bytes land
-  // 1.7 us after the CTA's start either way, a tensor-map fetch plus a trip to HBM after the first TMA instruction.)
+  // (the initialisations are published by fence.mbarrier_init; a releasing arrive alone was measured at 0.5 us). Only the
+  // epilogue warps touch the peers, so only they wait for the cluster here: the producer goes on to its loads as soon as its
+  // barriers stand, the MMA issuer once tensor memory is there too, and both wait for the cluster after their work.
+  constexpr int kSetupBar = 1;
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tma_w);
-      tma_prefetch_desc(&tma_x);
-      *abort_flag = 0;
-    }
     // barriers in the order they lie in shared memory: full[kStages], empty[kStages], acc_full[2], acc_empty[2],
     // partial_ready, partial_taken[2], drain_bar, tile_summed
     constexpr int kBars = 2 * Cfg::kStages + 9;
@@ -384,17 +379,23 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       const uint32_t count = (j == 2 || j == 3 || j == 8) ? 128u : (j == 5 || j == 6) ? 128u * (R > 1 ? R - 1 : 1) : 1u;
       mbar_init(&full_bar[i], count);
     }
+    if (lane == 0) *abort_flag = 0;
     fence_mbar_init();
+    fence_proxy_async_smem();  // the loads below credit barriers that other lanes have initialised
+    __syncwarp();
   } else if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);  // two accumulators
     tmem_relinquish();
   }
   tc_fence_before();
   cluster_arrive_relaxed();
-  __syncthreads();
-  cluster_wait();  // the peers' barriers are initialised before anything signals them
+  if (warp == 0) {
+    named_bar_arrive(kSetupBar, kSwapThreads);
+  } else {
+    named_bar_sync(kSetupBar, kSwapThreads);
+    if (warp != 1) cluster_wait();  // the peers' barriers are initialised before anything signals them
+  }
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
   bool epi_arrived = false;  // this thread has arrived at the closing cluster barrier
 
   if (warp == 0) {
@@ -405,6 +406,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     const int nkb = kb1 - kb0;
     int stage = 0;
     uint32_t phase = 0;
+    bool first = true;  // the first pass over the ring: every stage is free
     bool ok = true;
     for (int unit = walker; ok && unit < my_units; unit += num_walkers) {
       const int slab = unit / num_groups, grp = unit - slab * num_groups;
@@ -413,7 +415,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       const int rot = nkb > 0 ? static_cast<int>((static_cast<unsigned>(slab) * 11u) % static_cast<unsigned>(nkb)) : 0;
       for (int i = 0; i < nkb; ++i) {
         const int kb = kb0 + (i + rot >= nkb ? i + rot - nkb : i + rot);
-        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+        if (!first) ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
         if (!ok) break;
         const uint32_t sw = smem0 + static_cast<uint32_t>(stage) * Cfg::kStageBytes, bar = full0 + static_cast<uint32_t>(stage) * 8u;
         mbar_arrive_expect_tx_warp(&full_bar[stage], Cfg::kStageBytes, lead);
@@ -422,6 +424,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         if (++stage == Cfg::kStages) {
           stage = 0;
           phase ^= 1u;
+          first = false;
         }
       }
     }
@@ -431,8 +434,10 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       }
     }
     __syncwarp();
+    cluster_wait();
   } else if (warp == 1) {
     constexpr uint32_t idesc = umma_idesc_f16(128, MX, BF16, false, false);
+    const uint32_t tmem_base = *tmem_slot;
     const uint32_t lead = elect_one();
     int stage = 0;
     uint32_t phase = 0;
@@ -471,7 +476,9 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       }
     }
     __syncwarp();
+    cluster_wait();
   } else {
+    const uint32_t tmem_base = *tmem_slot;
     // The MX rows of X are cut into H x R blocks of kSub rows; in pass h rank r finishes block h * R + r: it keeps
     // that block of its own sums and sends each peer q the block h * R + q (slot "sender" of q's `partial`, four rows
     // of X per 16-byte store: a warp's store covers 512 consecutive bytes). The stores are asynchronous and credit their bytes to the receiver's
@@ -742,7 +749,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    tmem_dealloc(*tmem_slot, Cfg::kTmemCols);
   }
   cluster_wait();  // no CTA leaves while a peer can still write to it or signal it
 }

@@ -436,6 +436,10 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   return d;
 }
 
+// arrives at a named barrier (and publishes what was written before) without waiting for the others
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 // named barrier among a subset of the CTA's warps
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
