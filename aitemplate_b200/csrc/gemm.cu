@@ -836,62 +836,50 @@ static const std::vector<SwapKernel>& swap_kernels() {
 
 // Which weight-streaming kernel takes an unbatched problem (nullptr: the tile kernels do).
 //
-// Weights of more than 16 MB are bandwidth problems: W is read once at the HBM rate whatever the X tile, so the X
-// tile is as wide as M needs (one group up to M = 256), K goes two ways, or four / eight ways while the slabs are too
-// few to put most SMs to work. Bounds from sweeps against the tile kernels: M <= 128 from K = 512 on (M <= 32 from
-// K = 256), M <= 256 from K = 2048 on (4096 x 4096 at M = 256: 19.9 against 24.9 us), larger M in groups of 256 while
-// K >= 2048 and there are at most 32 units (beyond, the tile kernels are ahead again).
+// Up to 63 rows of X: weights of more than 16 MB are bandwidth problems, W is read once at the HBM rate whatever the X tile,
+// so one group holds all of X, and K goes two ways, or four / eight ways while the slabs are too few to put most SMs to work
+// (from K = 512 on; up to 32 rows from K = 256). Smaller weights are latency problems: a trip to memory takes about 0.7 us, a
+// launch about 3 us before the first byte arrives, so the time is the number of ring-fulls a rank streams, plus the exchange
+// (each CTA sends (R - 1) / R of its 128 x MX sums through the cluster's shared-memory window, about 40 GB/s per CTA),
+// plus a second wave's worth if the units outnumber the resident clusters; up to 64 output tiles of 128 x 128, 48 with an
+// added residual, 32 with another epilogue.
 //
-// Smaller problems are latency problems: a CTA's ring holds 150 - 190 KB, a trip to memory takes about 0.7 us, and a
-// launch costs about 3 us before the first byte arrives, so the time is the number of ring-fulls a rank streams, plus
-// the exchange (each CTA sends (R - 1) / R of its 128 x MX sums through the cluster's shared-memory window, measured
-// at about 40 GB/s per CTA), plus a second wave's worth if the units outnumber the resident clusters. X is therefore
-// cut into groups that are as small as it takes to fill one wave: 768 x 768 at M = 128 runs as 24 units of 32 rows,
-// K four ways (5.7 us) rather than 6 units of 128 rows (7.5 us). The estimate below was fitted to a sweep of 84 shapes
-// x 12 kernels (M = 32 .. 2048, N and K = 320 .. 4096) and picks within 2 % of the best kernel on average. Where the
-// tile kernels win instead was read off the same sweep: more than 64 output tiles of 128 x 128 (128 with K >= 4096; 48
-// with an added residual, 32 with any other epilogue beyond bias + relu), M > 1024 (2048 with K >= 4096), or K < 512
-// with M > 256.
-static const SwapKernel* plan_swapab(long long m, long long n, long long k, bool bf16, int epilogue_cost) {
-  if (n < 128 || m < 5) return nullptr;
-  const long long slabs = (n + 127) / 128, kb_total = (k + kBK - 1) / kBK;
+// From 64 to 2048 rows: by the estimates of rules.h, X in groups that are as small as it takes to fill one wave. The tile
+// kernels' are the firmer ones where both are close.
+static const SwapKernel* plan_swapab(const GemmProblem& g, int tile_width, bool bf16) {
+  if (g.n < 128 || g.m < 5 || g.k < 256 || g.m > 2048) return nullptr;
+  const long long slabs = (g.n + 127) / 128, kb_total = (g.k + kBK - 1) / kBK;
   const auto& table = swap_kernels();
-  auto find = [&](int mx, int r) -> const SwapKernel* {
+  const SwapKernel* best = nullptr;
+  double best_us = 0.0;
+  if (g.m < 64 && g.n * g.k * 2 > (16ll << 20)) {
+    if (g.k < 512 && g.m > 32) return nullptr;
+    const int r = (slabs <= sm_count() / 16 && kb_total >= 32) ? 8 : slabs <= sm_count() / 4 ? 4 : 2;
+    const int mx = std::max(8 * r, g.m <= 16 ? 16 : g.m <= 32 ? 32 : 64);
     for (const SwapKernel& sk : table)
       if (sk.mx == mx && sk.r == r) return &sk;
     return nullptr;
-  };
-  if (n * k * 2 > (16ll << 20)) {
-    const long long units = ((m + kSwapMaxM - 1) / kSwapMaxM) * slabs;
-    const bool take = m <= 128   ? (k >= 512 || (k >= 256 && m <= 32))
-                      : m <= 256 ? k >= 2048
-                                 : (k >= 2048 && units <= 32);
-    if (!take) return nullptr;
-    const int r = (units <= sm_count() / 16 && kb_total >= 32) ? 8 : units <= sm_count() / 4 ? 4 : 2;
-    const int mx = std::max(8 * r, m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : m <= 128 ? 128 : 256);
-    return find(mx, r);
   }
-  const long long tiles = ((m + 127) / 128) * slabs;
-  const bool deep = kb_total >= 64;
-  // (an activation other than relu costs this kernel a pre-pass over its tile, a second residual, a multiplied one or
-  // a permuted store its long store loop, all of which the tile kernels compile away: 3072 x 768 + fast_gelu at
-  // M = 256, 48 tiles, is 9.0 us here against 8.4)
-  // (with an added residual, 1024 x 1024 at M = 1024, 64 tiles: 10.3 us here against 9.6; 768 x 768, 48 tiles: level)
-  const long long max_tiles = epilogue_cost >= 2 ? 32 : epilogue_cost == 1 ? 48 : deep ? 128 : 64;
-  if (k < 256 || (k < 512 && m > 256) || tiles > max_tiles || m > (deep ? 2048 : 1024)) return nullptr;
-  const SwapKernel* best = nullptr;
-  double best_us = 0.0;
+  if (g.m < 64) {
+    if (slabs > (g.swap_epilogue >= 2 ? 32 : g.swap_epilogue == 1 ? 48 : kb_total >= 64 ? 128 : 64)) return nullptr;
+    for (const SwapKernel& sk : table) {
+      if (kb_total < sk.r) continue;                       // every rank needs a k-block
+      const long long units = ((g.m + sk.mx - 1) / sk.mx) * slabs;
+      const long long waves = (units + sk.resident(bf16) - 1) / sk.resident(bf16);
+      const double kb_rank = static_cast<double>((kb_total + sk.r - 1) / sk.r);
+      const double stream = std::max(0.7, kb_rank / sk.stages * 0.7) + kb_rank * 0.06;
+      const double tail = 128.0 * sk.mx * 4.0 * (sk.r - 1) / sk.r / 40e3 + 0.005 * sk.mx / sk.r;
+      const double us = 3.0 + stream + tail + (waves - 1) * (std::max(stream, tail) + 0.3);
+      if (best == nullptr || us < best_us) best = &sk, best_us = us;
+    }
+    return best;
+  }
   for (const SwapKernel& sk : table) {
-    if (kb_total < sk.r) continue;                       // every rank needs a k-block
-    const long long units = ((m + sk.mx - 1) / sk.mx) * slabs;
-    const long long waves = (units + sk.resident(bf16) - 1) / sk.resident(bf16);
-    const double kb_rank = static_cast<double>((kb_total + sk.r - 1) / sk.r);
-    const double stream = std::max(0.7, kb_rank / sk.stages * 0.7) + kb_rank * 0.06;
-    const double tail = 128.0 * sk.mx * 4.0 * (sk.r - 1) / sk.r / 40e3 + 0.005 * sk.mx / sk.r;
-    const double us = 3.0 + stream + tail + (waves - 1) * (std::max(stream, tail) + 0.3);
+    if (kb_total < sk.r) continue;
+    const double us = gemm_swap_us(g, sk.mx, sk.r, sk.resident(bf16));
     if (best == nullptr || us < best_us) best = &sk, best_us = us;
   }
-  return best;
+  return best_us < 0.97 * gemm_tile_us(g, tile_width, sm_count()) ? best : nullptr;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -968,21 +956,14 @@ struct GemmArgs {
   int* status = nullptr;  // device status word to use instead of the library's allocated one
 };
 
-constexpr int kTilePair = 512;  // tile_n value that asks for 256 x 256 tiles on CTA pairs
+constexpr int kTilePair = kGemmPairWidth;  // tile_n value that asks for 256 x 256 tiles on CTA pairs
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Tile width by a cost model of the persistent kernel. A tcgen05 MMA of 128 rows takes ~128 cycles per 16
-// of K whatever its N (the array is as wide as N = 256; narrower tiles leave columns idle), so a tile's main
-// loop costs the same at every width and only the epilogue shrinks with it. Per CTA the run is
-//   waves x max(main loop, epilogue) + one last epilogue,   waves = ceil(tiles / SMs),
-// so narrow tiles pay only when they save a whole wave (or the problem is all epilogue).
 // A result of this many bytes is streamed to DRAM while the kernel runs, and its stores set the pace.
 constexpr long long kStreamedBytes = 96ll << 20;
-int choose_tile_n(long long m, long long n, long long k, long long batch) {
-  const long long sms = sm_count();
-  const long long tm = (m + kBM - 1) / kBM;
-  const long long mainloop = ((k + kBK - 1) / kBK) * 512;  // cycles
+// Tile width: 64, 128, 256, or kTilePair.
+int choose_tile_n(const GemmProblem& g) {
   // Result streamed to DRAM behind one or two k-blocks per tile (the attention-score shape of bmm_rcr): the run
   // is the drain of the staged stores. A 256-wide tile gives each epilogue warp two 64-column boxes to store
   // through its one staging buffer, the second waiting for the first to drain; 128-wide tiles store one box per
@@ -993,18 +974,36 @@ int choose_tile_n(long long m, long long n, long long k, long long batch) {
   // 4096: 141 against 125 (the wide tile fetches a quarter fewer operand rows, and TMA pays per row). So the narrow
   // tile is taken for one full k-block, and for two only on a narrow result.
   // K = 32 (whole 64-byte rows): 102 us at 1024 x [512 x 512] against 125.
-  if (n >= 128 && batch * m * n * 2 > kStreamedBytes && (k <= 32 || k == kBK || (k > kBK && k <= 2 * kBK && n <= 512)))
+  if (g.n >= 128 && g.batch * g.m * g.n * 2 > kStreamedBytes && (g.k <= 32 || g.k == kBK || (g.k > kBK && g.k <= 2 * kBK && g.n <= 512)))
     return 128;
-  int best = 256;
-  long long best_cost = -1;
-  for (int bn : {256, 128, 64}) {
-    const long long tiles = tm * ((n + bn - 1) / bn) * batch;
-    const long long waves = (tiles + sms - 1) / sms;
-    const long long epilogue = 1500 + 8 * bn;  // measured: ~3.5 k cycles for a 128 x 256 tile, ~1.5 k of it fixed
-    const long long cost = waves * std::max(mainloop, epilogue) + epilogue;
-    if (best_cost < 0 || cost < best_cost) best = bn, best_cost = cost;
-  }
-  return best;
+  return gemm_best_width(g, sm_count());
+}
+
+struct GemmPlan {
+  int tile_n;              // choose_tile_n
+  const SwapKernel* swap;  // the weight-streaming kernel to take instead, or null
+};
+// The estimates of one problem take about half a microsecond of host time, which a call of a few microseconds would pay every
+// time: each thread keeps the plans of the problem sizes it saw last (by their sizes alone; 64 of them).
+static GemmPlan plan_gemm(const GemmProblem& g, bool bf16, bool streams) {
+  struct Slot {
+    GemmProblem g;
+    int sms, flags;
+    GemmPlan plan;
+  };
+  thread_local Slot slots[64] = {};
+  const int sms = sm_count(), flags = 1 | (bf16 ? 2 : 0) | (streams ? 4 : 0);
+  uint64_t h = static_cast<uint64_t>(g.batch);
+  for (const long long v : {g.m, g.n, g.k, g.pitch, static_cast<long long>(g.epilogue * 16 + g.swap_epilogue * 4 + g.generic * 64 + flags)})
+    h = (h ^ static_cast<uint64_t>(v)) * 0x9e3779b97f4a7c15ull;
+  Slot& s = slots[h >> 58];
+  if (s.flags == flags && s.sms == sms && s.g.batch == g.batch && s.g.m == g.m && s.g.n == g.n && s.g.k == g.k &&
+      s.g.epilogue == g.epilogue && s.g.swap_epilogue == g.swap_epilogue && s.g.pitch == g.pitch && s.g.generic == g.generic)
+    return s.plan;
+  GemmPlan plan{choose_tile_n(g), nullptr};
+  if (streams) plan.swap = plan_swapab(g, plan.tile_n, bf16);
+  s = Slot{g, sms, flags, plan};
+  return plan;
 }
 
 // How many stages of its operand ring a launch uses, where that is fewer than the kernel has. One k-block per tile: the ring
@@ -1022,13 +1021,16 @@ struct SplitPlan {
   int tile_n, splits, kb_per_split;
   long long bytes;
 };
-SplitPlan plan_split_k(long long batch, long long m, long long n, long long k, int tile_n, int max_splits,
-                       long long workspace_bytes) {
-  SplitPlan sp{tile_n ? tile_n : choose_tile_n(m, n, k, batch), 1, 0, 0};
+// `tile_n`: the caller's choice or 0, `planned_tile_n` what is taken for it. `streams`: the weight-streaming kernels could have taken the problem; where their planner preferred unsplit tiles, they stay so.
+SplitPlan plan_split_k(const GemmProblem& g, int tile_n, int planned_tile_n, int max_splits, long long workspace_bytes,
+                       bool streams) {
+  const long long batch = g.batch, m = g.m, n = g.n, k = g.k;
+  SplitPlan sp{planned_tile_n, 1, 0, 0};
   const long long num_kb = (k + kBK - 1) / kBK;
   sp.kb_per_split = static_cast<int>(num_kb);
   const long long sms = sm_count();
-  if (max_splits == 1 || num_kb < 4) return sp;
+  if (max_splits == 1 || num_kb < 4 || (max_splits == 0 && streams && m >= 5 && n >= 128)) return sp;
+  const int width = std::min(sp.tile_n, 256);  // (CTA pairs never split K)
   // One tile row (M <= 128): the run time is the time to stream the weights once. A tcgen05 MMA takes as long
   // as its M x K says, whatever N is, so a CTA consumes weight rows fastest through wide tiles: 128- and
   // 64-wide tiles cap a CTA at half and a quarter of the 256-wide rate, below its share of HBM bandwidth.
@@ -1046,7 +1048,7 @@ SplitPlan plan_split_k(long long batch, long long m, long long n, long long k, i
                        ((num_kb + per - 1) / per) * m * n * 4};
     }
   }
-  const long long tiles = ((m + kBM - 1) / kBM) * ((n + sp.tile_n - 1) / sp.tile_n) * batch;
+  const long long tiles = ((m + kBM - 1) / kBM) * ((n + width - 1) / width) * batch;
   long long s;
   if (max_splits > 1) {
     s = std::min<long long>(max_splits, num_kb / 2);  // the caller's choice
@@ -1060,11 +1062,12 @@ SplitPlan plan_split_k(long long batch, long long m, long long n, long long k, i
   }
   while (s > 1 && s * batch * m * n * 4 > workspace_bytes) --s;
   if (s <= 1) return sp;
+  sp.tile_n = width;
   const long long per = (num_kb + s - 1) / s;
   sp.splits = static_cast<int>((num_kb + per - 1) / per);  // no empty split
   sp.kb_per_split = static_cast<int>(per);
   sp.bytes = static_cast<long long>(sp.splits) * batch * m * n * 4;
-  if (sp.splits <= 1) sp = SplitPlan{sp.tile_n, 1, static_cast<int>(num_kb), 0};
+  if (sp.splits <= 1) sp = SplitPlan{width, 1, static_cast<int>(num_kb), 0};
   return sp;
 }
 
@@ -1199,7 +1202,12 @@ void gemm_run(const GemmArgs& g_in) {
     return;
   }
   // few rows of X, or few output tiles: the weight-streaming kernel where its planner takes the problem
-  if (tma_ok && g.batch == 1 && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0) {
+  const bool streams = tma_ok && g.batch == 1 && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0;
+  // (row-major B: its boxes are not rows of K, and the figures of rules.h do not hold)
+  const long long pitch = g.b_mn ? kBK : gemm_copy_row_us(g.lda) > gemm_copy_row_us(g.ldb) ? g.lda : g.ldb;
+  GemmProblem problem{g.batch, g.m, g.n, g.k, 0, 0, pitch, g.b_mn || g.num_out > 1};
+  GemmPlan planned{g.tile_n, nullptr};
+  {
     const int code = p.epilogue;
     // what the weight-streaming kernel's short store loop does without an activation pre-pass: bias [+ relu]
     // [+ one added residual [+ relu]] into a row-major output
@@ -1207,7 +1215,10 @@ void gemm_run(const GemmArgs& g_in) {
     const bool plain = (epi_b1(code) == kBinaryNone || added) && epi_b2(code) == kBinaryNone &&
                        (epi_u2(code) == kUnaryIdentity || (added && epi_u2(code) == kUnaryRelu)) &&
                        (epi_u1(code) == kUnaryIdentity || epi_u1(code) == kUnaryRelu) && p.store_mode == 0;
-    if (const SwapKernel* sk = plan_swapab(g.m, g.n, g.k, bf16, !plain ? 2 : added ? 1 : 0)) {
+    problem.swap_epilogue = !plain ? 2 : added ? 1 : 0;
+    problem.epilogue = b1 != kBinaryNone ? 1 : epi_u1(code) != kUnaryIdentity && epi_u1(code) != kUnaryRelu ? 2 : 0;
+    if (g.tile_n == 0) planned = plan_gemm(problem, bf16, streams);
+    if (const SwapKernel* sk = planned.swap) {
       const int num_groups = static_cast<int>((g.m + sk->mx - 1) / sk->mx);
       const int num_slabs = static_cast<int>((g.n + 127) / 128);
       CUtensorMap tw = make_tile_map(g.b, bf16, g.k, g.n, 1, g.ldb, 0, 128);
@@ -1232,26 +1243,15 @@ void gemm_run(const GemmArgs& g_in) {
                   "gemm: tile_n must be 64, 128, 256 or 512 (256 x 256 tiles on CTA pairs)");
   const bool ws_ok = g.workspace != nullptr && aligned16(g.workspace);
   const bool force_pair = g.tile_n == kTilePair;
-  SplitPlan sp = force_pair ? SplitPlan{256, 1, static_cast<int>((g.k + kBK - 1) / kBK), 0}
-                            : plan_split_k(g.batch, g.m, g.n, g.k, g.tile_n, g.num_out > 1 ? 1 : g.split_k,
-                                           ws_ok ? g.workspace_bytes : 0);
+  SplitPlan sp = force_pair ? SplitPlan{kTilePair, 1, static_cast<int>((g.k + kBK - 1) / kBK), 0}
+                            : plan_split_k(problem, g.tile_n, planned.tile_n, g.num_out > 1 ? 1 : g.split_k, ws_ok ? g.workspace_bytes : 0,
+                                           streams);
   if (g.num_out > 1 && sp.tile_n == 64 && g.tile_n == 0) sp.tile_n = 128;  // several destinations need the staged store
-  const int bn = sp.tile_n;
-  // CTA pairs (256 x 256 tiles, cta_group::2): a third less operand traffic per flop into each SM. Chosen
-  // when the 256-wide tile was picked automatically, the 256-row tiles still fill every pair once, and K is
-  // deep enough for the main loop (not the per-tile epilogue and pair hand-shake) to set the pace.
-  const long long pair_tiles = ((g.m + 2 * kBM - 1) / (2 * kBM)) * ((g.n + 255) / 256) * g.batch;
+  const int bn = std::min(sp.tile_n, 256);
+  // CTA pairs (256 x 256 tiles, cta_group::2): a third less operand traffic per flop into each SM, and a residual comes by
+  // TMA into the staging boxes where the single-CTA kernels load it per thread.
   B200AIT_REQUIRE(!(force_pair && p.c_bdiv != 0), "bmm permute: the CTA-pair tiles do not take the permuted store");
-  // With one residual operand the pair kernel pays from K = 256 on: it fetches the residual by TMA into its
-  // staging boxes where the single-CTA kernels load it per thread (8192 x 1280 x 320 "mul": 18.7 against 21.6 us).
-  const bool staged_residual = b1 != kBinaryNone && b2 == kBinaryNone;
-  // From K = 2048 on the pairs win even when only 3 in 5 of them get a tile: the operand traffic they save counts for
-  // more than the idle SMs (768 x 4096 x 4096: 28.2 against 32.0 us with 48 tiles for 74 pairs).
-  // (and with a residual, which only the pairs fetch by TMA: 3072 x 1280 x 320 + add: 11.3 against 12.3 us)
-  const long long pair_tiles_min = (g.k >= 2048 || staged_residual) ? sm_count() * 3 / 10 : sm_count() / 2;
-  const bool pair = force_pair || (g.tile_n == 0 && bn == 256 && sp.splits == 1 &&
-                                   g.k >= (staged_residual ? 256 : 512) && pair_tiles >= pair_tiles_min &&
-                                   p.c_bdiv == 0);
+  const bool pair = force_pair || (sp.tile_n == kTilePair && p.c_bdiv == 0);
   p.splits = sp.splits;
   p.kb_per_split = sp.kb_per_split;
   p.partial = static_cast<float*>(g.workspace);
@@ -1421,7 +1421,9 @@ B200AIT_EXPORT int b200ait_gemm_rcr_workspace_bytes(int64_t batch, int64_t m, in
     B200AIT_REQUIRE(bytes_out, "bytes_out is null");
     *bytes_out = 0;
     if (batch <= 0 || m <= 0 || n <= 0 || k <= 0) return;
-    *bytes_out = tile_n == kTilePair ? 0 : plan_split_k(batch, m, n, k, tile_n, split_k, (1ll << 62)).bytes;
+    if (tile_n == kTilePair) return;
+    const GemmProblem g{batch, m, n, k, 0, 0, k, false};
+    *bytes_out = plan_split_k(g, tile_n, tile_n ? tile_n : choose_tile_n(g), split_k, 1ll << 62, false).bytes;
   });
 }
 

@@ -951,8 +951,8 @@ void launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps&
   B200AIT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tout.m[0], td0, p, tout));
 }
 
-// Epilogues that get their own straight-line instantiation (fp16): bias, relu, gelu, fast_gelu, add,
-// add_relu, mul. Everything else, and bf16, runs the generic instantiation.
+// Epilogues that get their own straight-line instantiation: bias, relu, gelu, fast_gelu, add, add_relu, mul. Everything
+// else runs the generic instantiation.
 #define B200AIT_FOR_EACH_FAST_EPILOGUE(X)                                                  \
   X(make_epilogue(kUnaryIdentity, kBinaryNone, kBinaryNone, kUnaryIdentity))              \
   X(make_epilogue(kUnaryRelu, kBinaryNone, kBinaryNone, kUnaryIdentity))                  \
@@ -976,6 +976,17 @@ void launch_tc_width<128>(bool, const CUtensorMap&, const CUtensorMap&, const Ou
 template <>
 void launch_tc_width<256>(bool, const CUtensorMap&, const CUtensorMap&, const OutMaps&, const GemmParams&, int,
                           cudaStream_t);
+
+// The straight-line instantiations in bfloat16, defined in gemm_bn<BN>_bf16.cu.
+template <int BN>
+void launch_tc_width_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout, const GemmParams& p, int grid,
+                          cudaStream_t stream);
+template <>
+void launch_tc_width_bf16<64>(const CUtensorMap&, const CUtensorMap&, const OutMaps&, const GemmParams&, int, cudaStream_t);
+template <>
+void launch_tc_width_bf16<128>(const CUtensorMap&, const CUtensorMap&, const OutMaps&, const GemmParams&, int, cudaStream_t);
+template <>
+void launch_tc_width_bf16<256>(const CUtensorMap&, const CUtensorMap&, const OutMaps&, const GemmParams&, int, cudaStream_t);
 
 // CTA-pair kernel, 256 x 256 tiles; defined in gemm_pair256.cu.
 void launch_tc_pair256(bool bf16, const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout,
@@ -1018,17 +1029,20 @@ void launch_tc_pair256_bf16_lean(const CUtensorMap& ta, const CUtensorMap& tb, c
         launch_tc<BN_, false, kRowsEpilogue>(ta, tb, tout, p, grid, stream);                                   \
       return;                                                                                                  \
     }                                                                                                          \
-    if (bf16) {                                                                                                \
-      launch_tc<BN_, true, -1>(ta, tb, tout, p, grid, stream);                                                 \
-      return;                                                                                                  \
-    }                                                                                                          \
     /* the compile-time-epilogue kernels of the wide tiles are lean (see the kernel): anything else is generic */ \
     const bool lean_ok = BN_ < 128 || epi_b1(p.epilogue) != kBinaryNone ||                                     \
                          (p.alpha == 1.f && p.tma_store != 0 && p.splits == 1);                                \
-    if (!lean_ok) {                                                                                            \
-      launch_tc<BN_, false, -1>(ta, tb, tout, p, grid, stream);                                                \
-      return;                                                                                                  \
-    }                                                                                                          \
+    if (!lean_ok) {                                                                                           \
+      if (bf16)                                                                                               \
+        launch_tc<BN_, true, -1>(ta, tb, tout, p, grid, stream);                                              \
+      else                                                                                                    \
+        launch_tc<BN_, false, -1>(ta, tb, tout, p, grid, stream);                                             \
+      return;                                                                                                 \
+    }                                                                                                         \
+    if (bf16) { /* in a translation unit of their own */                                                      \
+      launch_tc_width_bf16<BN_>(ta, tb, tout, p, grid, stream);                                               \
+      return;                                                                                                 \
+    }                                                                                                         \
     switch (p.epilogue) {                                                                                      \
       B200AIT_FOR_EACH_FAST_EPILOGUE(B200AIT_CASE_##BN_)                                                       \
       default:                                                                                                 \
@@ -1037,3 +1051,14 @@ void launch_tc_pair256_bf16_lean(const CUtensorMap& ta, const CUtensorMap& tb, c
   }
 
 }  // namespace b200ait
+
+#define B200AIT_DEFINE_LAUNCH_TC_WIDTH_BF16(BN_)                                                                 \
+  template <>                                                                                                    \
+  void launch_tc_width_bf16<BN_>(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout,              \
+                                 const GemmParams& p, int grid, cudaStream_t stream) {                           \
+    switch (p.epilogue) {                                                                                        \
+      B200AIT_FOR_EACH_FAST_EPILOGUE(B200AIT_CASE_BF16_##BN_)                                                    \
+      default:                                                                                                   \
+        launch_tc<BN_, true, -1>(ta, tb, tout, p, grid, stream);                                                 \
+    }                                                                                                            \
+  }

@@ -105,4 +105,77 @@ inline bool gemm_rows_output(int n, int tile_n, bool one_residual) {
   return n > (tile_n > 64 ? 32 : one_residual ? 47 : 42);
 }
 
+// GEMM: the time of a launch of the tile kernels (128 x 64, 128 x 128, 128 x 256 tiles, and 256 x 256 on CTA pairs: width 512)
+// and of the weight-streaming kernel, in us. Both were fitted to a sweep of 650 problems (M = 64 .. 3000, N and K = 256 .. 8192,
+// N whole and not whole 16-byte rows, three epilogues, every tile and every weight-streaming kernel forced, fp16, one launch
+// behind the other) and are within 5 % of it; the launch they pick takes 1.007 times the best one's time on average (1.003
+// where N is not a multiple of 8). The rules before (a width by whole waves at 512 cycles per k-block, K split over CTAs, the
+// weight-streaming kernel up to a number of tiles) took 1.055 and 1.14 times.
+struct GemmProblem {
+  long long batch, m, n, k;
+  int epilogue;      // 0: bias [+ relu], 1: a residual operand, 2: another activation
+  int swap_epilogue; // as the weight-streaming kernel sees it: 0: bias [+ relu], 1: an added residual, 2: anything else
+  long long pitch;   // of the operands' rows, in elements (the worse aligned one's)
+  bool generic;      // an epilogue read from the parameters (row-major B, several destinations)
+};
+constexpr int kGemmPairWidth = 512;
+// What TMA takes for a 128-byte row of an operand box that does not start on a 128-byte boundary, in us: 2.85 cycles if it starts
+// on a 16-byte one only, 1.97 on 32, 1.7 on 64 (1.3 if aligned, which the costs below contain). 2048 x 2048 x 2040 takes 44,
+// 31, 24 and 19 us with 64-, 128-, 256-wide tiles and pairs, x 2048 23, 18, 16 and 16.
+inline double gemm_copy_row_us(long long pitch) {
+  return pitch % 64 == 0 ? 0.0 : pitch % 32 == 0 ? 0.00086 : pitch % 16 == 0 ? 0.00100 : 0.00146;
+}
+inline double gemm_tile_us(const GemmProblem& g, int width, int sms) {
+  // launch, k-block, and a tile's epilogue by GemmProblem::epilogue; then what an epilogue costs beyond that where the tiles
+  // of a CTA follow on each other's heels
+  struct Cost {
+    double launch, k_block, epilogue[3], next;
+  };
+  // A k-block of 64-wide tiles is bound by the issue of its copies, of 128-wide ones by shared memory (operands come in and are
+  // read by the MMA at 128 bytes a cycle), above that by the MMA. All CTAs together draw at most 22 TB/s of operands from L2.
+  static constexpr Cost whole[4] = {{2.28, 0.130, {1.63, 2.05, 1.89}, 0.14},
+                                    {2.56, 0.176, {1.27, 2.42, 1.91}, 0.19},
+                                    {2.67, 0.327, {2.02, 4.10, 2.89}, 0.98},
+                                    {2.18, 0.305, {3.31, 3.95, 4.01}, -0.68}};
+  static constexpr Cost ragged[4] = {{3.01, 0.128, {3.22, 4.96, 3.50}, 0.62},
+                                     {3.73, 0.175, {4.52, 7.20, 5.09}, 1.40},
+                                     {4.82, 0.315, {8.24, 13.43, 9.46}, 2.73},
+                                     {5.47, 0.301, {8.21, 13.43, 9.30}, 2.40}};
+  const int at = width == 64 ? 0 : width == 128 ? 1 : width == 256 ? 2 : 3;
+  const Cost& c = (g.n % 8 == 0 ? whole : ragged)[at];
+  const bool pair = width == kGemmPairWidth;
+  const long long bm = pair ? 256 : 128, bn = pair ? 256 : width, walkers = pair ? sms / 2 : sms;
+  const long long tiles = ((g.m + bm - 1) / bm) * ((g.n + bn - 1) / bn) * g.batch;
+  const long long waves = (tiles + walkers - 1) / walkers;
+  const double ctas = static_cast<double>(std::min(tiles, walkers) * (pair ? 2 : 1));
+  const int rows = pair ? 256 : 128 + width;  // that a CTA fetches per k-block
+  const double k_block = std::max({c.k_block, 128.0 * rows * ctas / 22.1e6, rows * gemm_copy_row_us(g.pitch)});
+  const double loop = static_cast<double>((g.k + 63) / 64) * k_block;
+  // 64-wide tiles are stored by the threads, 64 bytes each, which are not whole sectors where the rows are not
+  constexpr double kGeneric[4] = {0.0, 1.2, 1.5, 1.0};
+  const double epilogue = c.epilogue[g.epilogue] + (g.generic ? kGeneric[at] : 0.0) + (width == 64 && g.n % 16 != 0 ? (g.n % 8 == 0 ? 1.3 : 2.1) : 0.0);
+  return c.launch + loop + epilogue + static_cast<double>(waves - 1) * std::max(loop, epilogue + c.next);
+}
+// mx rows of X per group, K split r ways over a cluster, `resident` clusters on the GPU at once
+inline double gemm_swap_us(const GemmProblem& g, int mx, int r, int resident) {
+  const long long units = ((g.m + mx - 1) / mx) * ((g.n + 127) / 128);
+  const long long waves = (units + resident - 1) / resident;
+  const double ctas = static_cast<double>(std::min<long long>(units, resident) * r);
+  const long long k_blocks = ((g.k + 63) / 64 + r - 1) / r;
+  const double stream = static_cast<double>(k_blocks) * std::max({0.0754 + 0.0012 * mx, (16384.0 + mx * 128.0) * ctas / 26.6e6,
+                                                                  (128 + mx) * gemm_copy_row_us(g.pitch)});
+  // the exchange of partial sums, then the rows a rank finishes; output rows that are not whole 16-byte units go out by element
+  const double row = 0.0105 + (g.swap_epilogue == 1 ? 0.0121 : g.swap_epilogue == 2 ? 0.0229 : 0.0) + (g.n % 8 == 0 ? 0.0 : 0.26);
+  const double tail = 0.0268 * mx * (r - 1) / r + row * mx / r;
+  return 3.79 + stream + tail + static_cast<double>(waves - 1) * (std::max(stream, tail) + 0.8);
+}
+inline int gemm_best_width(const GemmProblem& g, int sms) {
+  int best = 64;
+  for (int width : {128, 256, kGemmPairWidth}) {
+    if (width == kGemmPairWidth && (g.n < 256 || (g.generic && g.k < 512))) break;  // (659 x [344 x 512 x 40], row-major B: 88 us, pairs 111)
+    if (gemm_tile_us(g, width, sms) < gemm_tile_us(g, best, sms)) best = width;
+  }
+  return best;
+}
+
 }  // namespace b200ait

@@ -1,0 +1,74 @@
+"""The estimates by which a GEMM goes to a tile width or to a weight-streaming kernel (csrc/rules.h), compiled for the host and
+checked against times measured on a B200 (us, fp16, one launch behind the other). 148 SMs."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+_WRAPPERS = """
+#include "rules.h"
+using namespace b200ait;
+extern "C" double tile_us(long long m, long long n, long long k, int e, int width) {
+  return gemm_tile_us(GemmProblem{1, m, n, k, e, e, k, false}, width, 148);
+}
+extern "C" double swap_us(long long m, long long n, long long k, int e, int mx, int r) {
+  return gemm_swap_us(GemmProblem{1, m, n, k, e, e, k, false}, mx, r, r == 2 ? 74 : r == 4 ? 33 : 15);
+}
+extern "C" int best_width(long long b, long long m, long long n, long long k, int e) {
+  return gemm_best_width(GemmProblem{b, m, n, k, e, e, k, false}, 148);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    work = tmp_path_factory.mktemp("plan")
+    src, lib = work / "plan.cpp", work / "plan.so"
+    src.write_text(_WRAPPERS)
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I",
+                    os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
+    lib = ctypes.CDLL(str(lib))
+    lib.tile_us.restype = lib.swap_us.restype = ctypes.c_double
+    return lib
+
+
+def _ll(*v):
+    return [ctypes.c_longlong(x) for x in v]
+
+
+# the fit is within 5 % (root mean square); one problem may lie a few times that off
+@pytest.mark.parametrize(
+    "m,n,k,e,width,us",
+    [
+        (256, 2304, 768, 0, 128, 5.97), (1055, 768, 3072, 0, 64, 11.3), (2048, 1024, 4096, 0, 128, 17.1),
+        (1055, 4096, 4096, 0, 256, 29.2), (1055, 4096, 4096, 0, 512, 43.9),
+        (384, 2305, 768, 0, 64, 10.0), (1055, 2305, 768, 1, 128, 21.5), (384, 3000, 640, 0, 128, 5.75),
+        (2048, 2048, 2040, 0, 512, 19.2), (2048, 2048, 2040, 0, 64, 43.6),
+    ])
+def test_tile_estimates(plan, m, n, k, e, width, us):
+    got = plan.tile_us(*_ll(m, n, k), e, width)
+    assert abs(got / us - 1) < 0.16, got
+
+
+@pytest.mark.parametrize("m,n,k,e,mx,r,us", [(1055, 256, 2048, 0, 32, 2, 7.1), (1055, 512, 8192, 0, 64, 2, 14.95),
+                                            (130, 769, 768, 0, 16, 2, 6.97), (384, 2305, 768, 0, 32, 2, 22.5)])
+def test_weight_streaming_estimates(plan, m, n, k, e, mx, r, us):
+    got = plan.swap_us(*_ll(m, n, k), e, mx, r)
+    assert abs(got / us - 1) < 0.2, got
+
+
+@pytest.mark.parametrize(
+    "batch,m,n,k,e,width",
+    [
+        (1, 24576, 3072, 768, 2, 512), (1, 8192, 8192, 8192, 0, 512),  # many tiles, deep K: pairs
+        (1, 1055, 4096, 4096, 0, 256),                                # one wave of single tiles, two of pairs
+        (1, 512, 3072, 768, 2, 128), (1, 1055, 768, 3072, 0, 64),      # few tiles
+        (1, 384, 3000, 640, 0, 128),                                  # rows that are not whole sectors
+        (1, 300, 200, 512, 0, 128),                                   # (no pair tile is wider than the result)
+        (1, 2048, 2048, 2040, 0, 512),                                # rows off every 32-byte boundary: as few copies as can be
+    ])
+def test_widths(plan, batch, m, n, k, e, width):
+    assert plan.best_width(*_ll(batch, m, n, k), e) == width
