@@ -135,6 +135,39 @@ def load() -> ctypes.CDLL:
         return lib
 
 
+# entry points that torch_calls.so calls, in the order of its Library structure
+_CALLED = ["b200ait_gemm_rcr", "b200ait_gemm_rrr", "b200ait_gemm_rcr_workspace_bytes", "b200ait_mem_eff_attention",
+           "b200ait_flash_attention", "b200ait_layernorm", "b200ait_softmax", "b200ait_concatenate", "b200ait_split",
+           "b200ait_permute", "b200ait_last_error", "AITemplateModelContainerRun"]
+_calls = None
+
+
+def load_calls():
+    """Loads torch_calls.so, the native host path of the eager calls, bound to the loaded library; raises if it has not been
+    built."""
+    global _calls
+    if _calls is not None:
+        return _calls
+    lib = load()
+    with _lock:
+        if _calls is not None:
+            return _calls
+        import importlib.machinery
+        import importlib.util
+
+        import torch
+
+        path = LIB_PATH.with_name("torch_calls.so")
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it with `python -m aitemplate_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("torch_calls", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("torch_calls", loader))
+        loader.exec_module(module)
+        module.bind(tuple(ctypes.cast(getattr(lib, n), c_void_p).value for n in _CALLED), torch.nn.Parameter)
+        _calls = module
+        return module
+
+
 def kernel_launch_count() -> int:
     """Kernels launched by the library in this process so far."""
     n = c_int64(0)

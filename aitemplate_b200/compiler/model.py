@@ -232,6 +232,12 @@ class Model:
                          graph_mode: bool = False):
         """Runs the model with torch tensors (lists ordered by the index maps, or name -> tensor dicts);
         returns name -> output tensor viewed with the shape the run produced."""
+        if type(self) is Model and self.DLL.is_open:
+            # plain dicts of tensors go through native code (csrc/torch_calls.cpp); None: not plain, or to be refused below
+            done = _lib.load_calls().run_model(self.handle.value, inputs, outputs, self._input_name_to_index,
+                                               self._output_name_to_index, self._output_ndims, stream_ptr, sync, graph_mode)
+            if done is not None:
+                return done
         _check_tensors_contiguous_and_on_gpu(inputs, name="inputs")
         _check_tensors_contiguous_and_on_gpu(outputs, name="outputs")
         if stream_ptr is None:

@@ -60,8 +60,18 @@ def epilogue_code(name: str) -> int:
     return _EPILOGUE_CODES[name]
 
 
-# The wrappers below are paid by every eager call, and most calls take the GPU less time than the wrapper took the host
-# (256 x 3072 x 768: 8.8 us of kernel behind 24.6 us of host).
+# The wrappers below are paid by every eager call, and most calls take the GPU less time than the wrapper took the host. So a
+# plain call goes to native code (csrc/torch_calls.cpp; 256 x 3072 x 768: 6 us of kernel, 12 us of host by the code below, 6 there),
+# which answers None to whatever is not plain; those calls, and the ones to refuse, take the code below.
+_calls = None
+
+
+def _native():
+    global _calls
+    _calls = _lib.load_calls()
+    return _calls
+
+
 def _stream() -> int:
     """The current device's current stream, without the Stream object torch.cuda.current_stream() builds (3.2 us).
     Both calls are private to PyTorch (2.11 has them)."""
@@ -109,6 +119,10 @@ def gemm_rcr(
 ) -> torch.Tensor:
     """y = epilogue(x @ w.T + bias, d0, d1); x [..., K] (leading dims fold into M), w [N, K].
     split_k: 0 lets the library decide, 1 disables split-K, n allows at most n splits."""
+    if permute_shape is None and out is None:
+        y = (_calls or _native()).gemm_rcr(x, w, bias, d0, d1, _EPILOGUE_CODES.get(epilogue), alpha, tile_n, split_k)
+        if y is not None:
+            return y
     _check_cuda(x, w, bias, d0, d1)
     if out is not None and not out.is_cuda:
         raise ValueError("tensors must be CUDA tensors")
@@ -203,6 +217,9 @@ def gemm_rrr(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = No
 
 def bmm_rrr(a: torch.Tensor, b: torch.Tensor, alpha: float = 1.0, tile_n: int = 0) -> torch.Tensor:
     """c[i] = a[i] @ b[i] with a [B, M, K] (or [M, K]) and b [B, K, N] (or [K, N]); batch 1 broadcasts."""
+    c = (_calls or _native()).bmm(a, b, alpha, tile_n, True)
+    if c is not None:
+        return c
     _check_cuda(a, b)
     a3 = a if a.dim() == 3 else a.unsqueeze(0)
     b3 = b if b.dim() == 3 else b.unsqueeze(0)
@@ -260,6 +277,9 @@ def _workspace_bytes(device: int, m: int, n: int, k: int, tile_n: int, split_k: 
 
 def bmm_rcr(a: torch.Tensor, b: torch.Tensor, alpha: float = 1.0, tile_n: int = 0) -> torch.Tensor:
     """c[i] = a[i] @ b[i].T with a [B, M, K] (or [M, K]) and b [B, N, K] (or [N, K]); batch 1 broadcasts."""
+    c = (_calls or _native()).bmm(a, b, alpha, tile_n, False)
+    if c is not None:
+        return c
     _check_cuda(a, b)
     a3 = a if a.dim() == 3 else a.unsqueeze(0)
     b3 = b if b.dim() == 3 else b.unsqueeze(0)
@@ -285,6 +305,10 @@ def mem_eff_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal:
     """q [B,H,Sq,D], k [B,H,Skv,D], v [B,H,Skv,Dv] -> [B,Sq,H,Dv]; scale defaults to 1/sqrt(D).
     lengths_kv / lengths_q: int32 device tensors of B values (batch b sees its first lengths_kv[b] keys; only its
     first lengths_q[b] rows are written - pass `out` to choose what the other rows hold)."""
+    if out is None:
+        o = (_calls or _native()).mem_eff_attention(q, k, v, causal, scale, lengths_kv, lengths_q)
+        if o is not None:
+            return o
     _check_cuda(q, k, v)
     bsz, h, sq, d = q.shape
     skv, dv = k.shape[2], v.shape[3]
@@ -338,6 +362,9 @@ def mem_eff_attention_strided(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
 def flash_attention(qkv: torch.Tensor, cu_seqlens: torch.Tensor, max_seq_len: int, causal: bool = False,
                     scale: Optional[float] = None) -> torch.Tensor:
     """qkv [total, 3, H, D] packed, cu_seqlens int32 [batch + 1] -> [total, H, D]."""
+    o = (_calls or _native()).flash_attention(qkv, cu_seqlens, max_seq_len, causal, scale)
+    if o is not None:
+        return o
     _check_cuda(qkv, cu_seqlens)
     if cu_seqlens.dtype != torch.int32:
         raise ValueError("cu_seqlens must be int32")
@@ -357,6 +384,9 @@ def flash_attention(qkv: torch.Tensor, cu_seqlens: torch.Tensor, max_seq_len: in
 
 def layernorm(x: torch.Tensor, gamma: Optional[torch.Tensor], beta: Optional[torch.Tensor], eps: float = 1e-5,
               normalized_ndim: int = 1) -> torch.Tensor:
+    y = (_calls or _native()).layernorm(x, gamma, beta, eps, normalized_ndim)
+    if y is not None:
+        return y
     _check_cuda(x, gamma, beta)
     n = math.prod(x.shape[x.dim() - normalized_ndim:])
     m = x.numel() // n if n else 0
@@ -369,6 +399,9 @@ def layernorm(x: torch.Tensor, gamma: Optional[torch.Tensor], beta: Optional[tor
 
 
 def softmax(x: torch.Tensor, dim: int = -1) -> torch.Tensor:
+    y = (_calls or _native()).softmax(x, dim)
+    if y is not None:
+        return y
     _check_cuda(x)
     dim = dim % x.dim()
     outer = math.prod(x.shape[:dim])
@@ -386,6 +419,10 @@ def _i64(vals) -> ctypes.Array:
 
 def concatenate(tensors: List[torch.Tensor], dim: int = 0, input_masks: Optional[Sequence[bool]] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    if input_masks is None and out is None:
+        y = (_calls or _native()).concatenate(tensors, dim)
+        if y is not None:
+            return y
     _check_cuda(*tensors)
     rank = tensors[0].dim()
     dim = dim % rank
@@ -408,6 +445,9 @@ def concatenate(tensors: List[torch.Tensor], dim: int = 0, input_masks: Optional
 
 
 def split(x: torch.Tensor, split_size_or_sections, dim: int = 0) -> List[torch.Tensor]:
+    parts = (_calls or _native()).split(x, split_size_or_sections, dim)
+    if parts is not None:
+        return parts
     _check_cuda(x)
     rank = x.dim()
     dim = dim % rank
@@ -432,6 +472,9 @@ def split(x: torch.Tensor, split_size_or_sections, dim: int = 0) -> List[torch.T
 
 
 def permute(x: torch.Tensor, dims: Sequence[int]) -> torch.Tensor:
+    y = (_calls or _native()).permute(x, dims)
+    if y is not None:
+        return y
     _check_cuda(x)
     dims = [d % x.dim() for d in dims]
     out = x.new_empty([x.shape[d] for d in dims])
