@@ -18,9 +18,9 @@
 //               S and P are double-buffered: the MMAs of key block j+1 overlap the softmax of block j; heads of up
 //               to 64 channels double-buffer O across items
 //   warps 2-5   one thread per query row: TMEM -> registers, mask (skipped for full, unmasked blocks),
-//               reference max / row sum, exp2, P (16-bit pairs) -> TMEM; O is touched only when a row's
-//               maximum outgrows the reference by more than 2^8 (then O and the row sum are rescaled in
-//               TMEM) and once at the end of the item (O / row sum -> global memory)
+//               exp2 against the row's reference maximum, row sum, P (16-bit pairs) -> TMEM; O is touched only when a
+//               row outgrows its reference (then O and the row sum are rescaled in TMEM) and once at the end of the item
+//               (O / row sum -> global memory)
 // Two CTAs share an SM so one CTA's softmax also overlaps the other's MMAs (unless there are no items for a second one).
 // Shared-memory bandwidth is what the MMAs of this kernel run into (a 128 x 64 x 16 MMA with both operands in
 // shared memory reads 6 KB and issues every 48 cycles = 128 B / clk, the whole bandwidth of an SM), which is why P
@@ -39,34 +39,6 @@
 #include "rules.h"
 
 namespace b200ait {
-
-// Cycle probes for tuning (compiled only with -DB200AIT_ATTN_PROBE; never part of the shipped library): CTA 0 adds
-// the clock64() time its softmax warp 2 / its MMA thread spend in each phase to g_attn_probe[slot].
-#ifdef B200AIT_ATTN_PROBE
-__device__ long long g_attn_probe[32];
-#define ATTN_PROBE_DECL(cond)                \
-  const bool probe_on = (cond);              \
-  long long probe_acc[4] = {0, 0, 0, 0};     \
-  long long probe_t = clock64();
-// phase times are kept in registers (slot & 3) and flushed once by ATTN_PROBE_FLUSH(base)
-#define ATTN_PROBE(slot)                                   \
-  if (probe_on) {                                          \
-    const long long probe_now = clock64();                 \
-    probe_acc[(slot) & 3] += probe_now - probe_t;          \
-    probe_t = probe_now;                                   \
-  }
-#define ATTN_PROBE_SKIP() \
-  if (probe_on) probe_t = clock64();
-#define ATTN_PROBE_FLUSH(base)                                                  \
-  if (probe_on) {                                                               \
-    for (int pi = 0; pi < 4; ++pi) g_attn_probe[(base) + pi] += probe_acc[pi];  \
-  }
-#else
-#define ATTN_PROBE_DECL(cond)
-#define ATTN_PROBE(slot)
-#define ATTN_PROBE_SKIP()
-#define ATTN_PROBE_FLUSH(base)
-#endif
 
 // defined in gemm.cu
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -109,14 +81,13 @@ struct AttnOperand {
 constexpr int kAttnThreads = 224;  // producer, P V issuer, 4 softmax warps, S issuer
 constexpr int kBlockM = 128;
 constexpr int kBlockN = 64;     // keys per block
-constexpr float kRescaleLog2 = 8.f;  // a row's reference maximum may lag its true maximum by this much (log2 units)
+// The reference maximum of a row may lag its true maximum while the row's sum over a block stays below this: P is then at most
+// half of what float16 holds, and as exact as with the true maximum.
+constexpr float kMaxRowSum = 32768.f;
 // Of every eight pairs of scores, this many get their exp2 from the FMA pipe (exp2_poly2 below) instead of the
 // special-function unit, which is the busiest unit of the kernel (64 exp2 per row and key block at 4 lanes per
 // clock and scheduler).
-#ifndef B200AIT_ATTN_POLY_OF8
-#define B200AIT_ATTN_POLY_OF8 2
-#endif
-constexpr int kPolyOf8 = B200AIT_ATTN_POLY_OF8;
+constexpr int kPolyOf8 = 2;
 
 // exp2 of two values on the FMA pipe: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f by a cubic whose relative
 // error stays below 7.5e-5 (P is rounded to 11 significant bits right after, 4.9e-4); n goes into the exponent
@@ -177,9 +148,15 @@ struct AttnCfg {
 //   MMA warp:      S(0), S(1); then for each j: wait P(j) -> O += P(j) V(j) -> S(j+2)
 //   softmax warps: wait S(j) -> max / exp2 / row sum -> P(j) -> signal; at the item's end O / row sum -> global
 // so the tensor core computes S(j+1), S(j+2) and P(j-1) V(j-1) while the softmax threads work on block j.
+// What a softmax warp does with a block is bound by its instructions: 128 rows of 128 keys take two warps per scheduler 2011
+// cycles without any wait (exponentials alone 1536, everything else 1024), three warps per scheduler no less per row. So what is
+// left out counts: with the row maximum taken only where it has to be, 4 x 12 heads x 4096 rows of 64 take 245 us instead of
+// 261, 64 x 12 x 384 50.5 instead of 53.5, 8 packed causal sequences of 512 .. 4096 rows and 16 heads of 128 249 instead of 270.
+// Blocks of 128 keys (fewer waits, 200 registers for a row of scores) came to 244, 51 and 290; three chains of softmax warps
+// on an SM to 275 and 57.
 // The softmax is "lazy" about the running maximum: a row keeps a reference maximum m_ref and evaluates
-// p = exp2(s * scale - m_ref); m_ref is raised (and O and the row sum rescaled by exp2(m_ref_old - m_ref_new))
-// only when the block's maximum exceeds it by more than kRescaleLog2, so p never exceeds 2^kRescaleLog2 and the
+// p = exp2(s * scale - m_ref); m_ref is the maximum of an item's first block and raised (O and the row sum rescaled by
+// exp2(m_ref_old - m_ref_new)) only when a block's row sum shows that some p may have left the range of P (kMaxRowSum). The
 // final O / l is the same quotient the reference forms with the exact running maximum
 // (attention_scaling_coefs_updater.h:85-165), up to the rounding of P at a different power-of-two-ish scale.
 // NOMASK: no causal mask and a key length that is a multiple of the block: every key block is "plain", and the
@@ -258,12 +235,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     w.n_blocks = (w.q0 < w.q_len) ? (w.kv_len + kBlockN - 1) / kBlockN : 0;
     return w;
   };
-  auto load_rows = [&](void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int row, const Item& w, int order) {
-    if (order == 0)
-      tma_load_4d(dst, map, bar, c0, row, w.h, w.b4);
-    else
-      tma_load_4d(dst, map, bar, c0, w.h, row, w.b4);
-  };
   if constexpr (SKIP) {
     // The condition always holds, but the compiler does not know: it would keep this decoding of the first item in registers
     // for the roles to share (8 packed causal sequences of 512 .. 4096 rows, 16 heads of 128: 250 us; 256 .. 260 so, no skip 254).
@@ -271,101 +242,97 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   }
   const int dsteps = (p.D + 15) / 16;  // k-steps of Q K^T
 
-  if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(q_full + 1, 1);
-    for (int s = 0; s < Cfg::kKvStages; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
-      if (Cfg::kSplitKv) mbar_init(&v_full[s], 1);
+  // Set-up in parallel: the lanes of warp 0 initialise a barrier each while warp 1 allocates tensor memory. The producer
+  // (warp 0) needs nothing else and goes on to its loads. Barriers in the order they lie in shared memory: q_full[2],
+  // kv_full, kv_empty, s_full[2], p_full[2], o_empty[2], drain[2], q_empty[2], v_full.
+  constexpr int kSetupBar = 1;
+  if (warp == 0) {
+    constexpr int kBars = 12 + (Cfg::kSplitKv ? 3 : 2) * Cfg::kKvStages;
+    for (int i = lane; i < kBars; i += 32) {
+      const int j = i - (2 + 2 * Cfg::kKvStages);  // from s_full on
+      mbar_init(&q_full[i], (j >= 2 && j < 6) ? 128u : 1u);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&o_empty[i], 128);
-    }
-    mbar_init(drain_bar, 1);
-    mbar_init(drain_bar + 1, 1);
-    mbar_init(q_empty, 1);
-    mbar_init(q_empty + 1, 1);
-    *abort_flag = 0;
+    if (lane == 0) *abort_flag = 0;
     fence_mbar_init();
-    tma_prefetch_desc(&tma_q);
-    tma_prefetch_desc(&tma_k);
-    tma_prefetch_desc(&tma_v);
-  }
-  __syncthreads();
-  if (warp == 1) {
+    fence_proxy_async_smem();  // the loads below credit barriers that other lanes have initialised
+    __syncwarp();
+  } else if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  if (warp == 0)
+    named_bar_arrive(kSetupBar, kAttnThreads);
+  else
+    named_bar_sync(kSetupBar, kAttnThreads);
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = *tmem_slot;    // (nothing yet in warp 0, which has no use for it)
   const uint32_t tmem_s = tmem_base;        // S(j) at + (j & 1) * 64; P(j) as 16-bit pairs over its first 32 columns
   const uint32_t tmem_o = tmem_base + 128;  // O of item it at + o_buf(it) * kTWidth
   auto o_buf = [](int it) { return Cfg::kOBufs == 2 ? (it & 1) : 0; };
   auto o_phase = [](int it) { return static_cast<uint32_t>(Cfg::kOBufs == 2 ? (it >> 1) & 1 : it & 1); };
 
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true;
-      int g = 0;  // global key-block counter (K/V ring position)
-      int it = 0;
-      for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-        const Item w = decode_item(item);
-        if (w.n_blocks == 0) continue;
-        // Q buffer qb is free once the last S = Q K^T of the item that used it before has completed
-        const int qb = it % Cfg::kQBufs;
-        const uint32_t qph = static_cast<uint32_t>(it / Cfg::kQBufs) & 1u;
-        ok = mbar_wait(&q_empty[qb], qph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
-        if (!ok) break;
-        mbar_arrive_expect_tx(&q_full[qb], Cfg::kQBytes);
+    const uint32_t lead = elect_one();
+    auto load_rows = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int c0, int row, const Item& w, int order) {
+      if (order == 0)
+        tma_load_4d_warp(smem_u32(dst), map, smem_u32(bar), c0, row, w.h, w.b4, lead);
+      else
+        tma_load_4d_warp(smem_u32(dst), map, smem_u32(bar), c0, w.h, row, w.b4, lead);
+    };
+    bool ok = true;
+    int g = 0;  // global key-block counter (K/V ring position)
+    int it = 0;
+    for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
+      const Item w = decode_item(item);
+      if (w.n_blocks == 0) continue;
+      // Q buffer qb is free once the last S = Q K^T of the item that used it before has completed
+      const int qb = it % Cfg::kQBufs;
+      const uint32_t qph = static_cast<uint32_t>(it / Cfg::kQBufs) & 1u;
+      ok = mbar_wait_warp(&q_empty[qb], qph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+      if (!ok) break;
+      mbar_arrive_expect_tx_warp(&q_full[qb], Cfg::kQBytes, lead);
 #pragma unroll
-        for (int c = 0; c < DCH; ++c)
-          load_rows(sQ + qb * Cfg::kQBytes + c * kBlockM * 128, &tma_q, &q_full[qb], c * 64, w.row0 + w.q0, w, p.q_order);
-        for (int j = 0; j < w.n_blocks; ++j, ++g) {
-          const int st = g % Cfg::kKvStages;
-          const uint32_t ph = (g / Cfg::kKvStages) & 1;
-          uint8_t* sK = sKV + st * 2 * Cfg::kKBytes;
-          uint8_t* sV = sK + Cfg::kKBytes;
-          if constexpr (Cfg::kSplitKv) {
-            // the block that had this stage before is g - 2: K is free when its S is complete, V when its P V is
-            ok = mbar_wait(&s_full[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
-            if (!ok) break;
-            mbar_arrive_expect_tx(&kv_full[st], Cfg::kKBytes);
-#pragma unroll
-            for (int c = 0; c < DCH; ++c)
-              load_rows(sK + c * kBlockN * 128, &tma_k, &kv_full[st], c * 64, w.row0 + j * kBlockN, w, p.k_order);
-            ok = mbar_wait(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
-            if (!ok) break;
-            mbar_arrive_expect_tx(&v_full[st], Cfg::kKBytes);
-#pragma unroll
-            for (int c = 0; c < DCH; ++c)
-              load_rows(sV + c * kBlockN * 128, &tma_v, &v_full[st], c * 64, w.row0 + j * kBlockN, w, p.v_order);
-            continue;
-          }
-          ok = mbar_wait(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+      for (int c = 0; c < DCH; ++c)
+        load_rows(sQ + qb * Cfg::kQBytes + c * kBlockM * 128, &tma_q, &q_full[qb], c * 64, w.row0 + w.q0, w, p.q_order);
+      for (int j = 0; j < w.n_blocks; ++j, ++g) {
+        const int st = g % Cfg::kKvStages;
+        const uint32_t ph = static_cast<uint32_t>(g / Cfg::kKvStages) & 1u;
+        uint8_t* sK = sKV + st * 2 * Cfg::kKBytes;
+        uint8_t* sV = sK + Cfg::kKBytes;
+        if constexpr (Cfg::kSplitKv) {
+          // the block that had this stage before is g - 2: K is free when its S is complete, V when its P V is
+          ok = mbar_wait_warp(&s_full[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
           if (!ok) break;
-          mbar_arrive_expect_tx(&kv_full[st], 2 * Cfg::kKBytes);
+          mbar_arrive_expect_tx_warp(&kv_full[st], Cfg::kKBytes, lead);
 #pragma unroll
-          for (int c = 0; c < DCH; ++c) {
+          for (int c = 0; c < DCH; ++c)
             load_rows(sK + c * kBlockN * 128, &tma_k, &kv_full[st], c * 64, w.row0 + j * kBlockN, w, p.k_order);
-            load_rows(sV + c * kBlockN * 128, &tma_v, &kv_full[st], c * 64, w.row0 + j * kBlockN, w, p.v_order);
-          }
+          ok = mbar_wait_warp(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+          if (!ok) break;
+          mbar_arrive_expect_tx_warp(&v_full[st], Cfg::kKBytes, lead);
+#pragma unroll
+          for (int c = 0; c < DCH; ++c)
+            load_rows(sV + c * kBlockN * 128, &tma_v, &v_full[st], c * 64, w.row0 + j * kBlockN, w, p.v_order);
+          continue;
         }
-        ++it;
+        ok = mbar_wait_warp(&kv_empty[st], ph ^ 1u, abort_flag, p.status, kDevWaitEmptyTimeout);
+        if (!ok) break;
+        mbar_arrive_expect_tx_warp(&kv_full[st], 2 * Cfg::kKBytes, lead);
+#pragma unroll
+        for (int c = 0; c < DCH; ++c) {
+          load_rows(sK + c * kBlockN * 128, &tma_k, &kv_full[st], c * 64, w.row0 + j * kBlockN, w, p.k_order);
+          load_rows(sV + c * kBlockN * 128, &tma_v, &kv_full[st], c * 64, w.row0 + j * kBlockN, w, p.v_order);
+        }
       }
-      if (!ok) {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) {
-        }
+      ++it;
+    }
+    if (!ok) {
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) {
       }
     }
-#ifndef B200AIT_ATTN_NO_SYNCWARP
     __syncwarp();
-#endif
   } else if (warp == 1) {
     // P V issuer: O(item) += P(g) V(g) as soon as the softmax threads have put P(g) into TMEM
     constexpr uint32_t idesc_t = umma_idesc_f16(kBlockM, Cfg::kTWidth, BF16, false, true);  // V is MN-major
@@ -459,7 +426,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     bool ok = true;
     int gb = 0;  // global index of the item's first key block
     int it = 0;
-    ATTN_PROBE_DECL(blockIdx.x == 0 && threadIdx.x == 64)
     // The read-out of an item's O (wait for its last P V, O / row sum -> global memory) is deferred until this thread
     // has handed the NEXT item's first P block to the tensor core: by then the last P V has long completed, so the
     // thread never waits for it, and its TMEM loads and stores overlap the other warps' exponentials. What makes
@@ -525,7 +491,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         ok = mbar_wait(&s_full[g & 1], (g >> 1) & 1, abort_flag, p.status, kDevWaitAccFullTimeout);
         if (!ok) break;
         tc_fence_after();
-        ATTN_PROBE(0)  // wait for S (and whatever the loop does before it)
         const uint32_t s_addr = tmem_s + lane_addr + static_cast<uint32_t>((g & 1) * kBlockN);
         const int key0 = j * kBlockN;
         int limit = kv_len - key0;  // keys [0, limit) of this block are visible to this row
@@ -538,103 +503,106 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         tmem_ld_32x32b_x32(s_addr, s0);
         tmem_ld_32x32b_x32(s_addr + 32, s1);
         tmem_ld_wait();
-        ATTN_PROBE(1)  // S from TMEM
-        float l0 = 0.f, l1 = 0.f;
         // One body, compiled twice: kPlain drops every per-element mask.
         auto softmax_block = [&](auto plain_tag) {
           constexpr bool kPlain = decltype(plain_tag)::value;
-          float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+          auto row_max = [&] {
+            float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const float a0 = __uint_as_float(s0[i]), a1 = __uint_as_float(s0[i + 1]);
-            const float a2 = __uint_as_float(s0[i + 2]), a3 = __uint_as_float(s0[i + 3]);
-            const float b0 = __uint_as_float(s1[i]), b1 = __uint_as_float(s1[i + 1]);
-            const float b2 = __uint_as_float(s1[i + 2]), b3 = __uint_as_float(s1[i + 3]);
-            if constexpr (kPlain) {
-              m0 = max3(m0, a0, a1);
-              m1 = max3(m1, a2, a3);
-              m2 = max3(m2, b0, b1);
-              m3 = max3(m3, b2, b3);
-            } else {
-              m0 = max3(m0, (i < limit) ? a0 : -INFINITY, (i + 1 < limit) ? a1 : -INFINITY);
-              m1 = max3(m1, (i + 2 < limit) ? a2 : -INFINITY, (i + 3 < limit) ? a3 : -INFINITY);
-              m2 = max3(m2, (32 + i < limit) ? b0 : -INFINITY, (33 + i < limit) ? b1 : -INFINITY);
-              m3 = max3(m3, (34 + i < limit) ? b2 : -INFINITY, (35 + i < limit) ? b3 : -INFINITY);
-            }
-          }
-          const float m_blk = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * p.scale_log2;
-          // Raise the reference maximum only when some row of this warp outgrew it by more than the slack
-          // (always on an item's first block, where nothing has been accumulated yet). The TMEM accesses of
-          // the rescale are warp-wide, so the decision is too; rows that did not move get alpha = 1.
-          if (__any_sync(0xffffffffu, m_blk > m_ref + kRescaleLog2)) {
-            const float m_new = fmaxf(m_ref, m_blk);
-            if (j > 0) {
-              // O holds blocks 0 .. j-1 once P(j-1) V(j-1) is done; P(j) V(j) cannot start before this
-              // thread's arrival on p_full below
-              if (!mbar_wait(&kv_empty[(g - 1) % Cfg::kKvStages], ((g - 1) / Cfg::kKvStages) & 1, abort_flag, p.status,
-                             kDevWaitAccFullTimeout)) {
-                ok = false;
-              } else {
-                tc_fence_after();
-                const float alpha = (m_new == -INFINITY) ? 1.f : exp2f(m_ref - m_new);  // m_ref = -inf: O is 0 anyway
-                const uint64_t alpha2 = pack2(alpha, alpha);
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t(&sv)[32] = h == 0 ? s0 : s1;
 #pragma unroll
-                for (int c = 0; c < DCH * 4; ++c) {
-                  if (c * 16 < p.Dv) {  // warp-uniform
-                    uint32_t v[16];
-                    tmem_ld_32x32b_x16(o_addr + c * 16, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                      float x0, x1;
-                      unpack2(mul2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), alpha2), x0, x1);
-                      v[i] = __float_as_uint(x0);
-                      v[i + 1] = __float_as_uint(x1);
-                    }
-                    tmem_st_32x32b_x16(o_addr + c * 16, v);
-                  }
-                }
-                tmem_st_wait();
-                l_run *= alpha;
+              for (int i = 0; i < 32; i += 2) {
+                const float a0 = __uint_as_float(sv[i]), a1 = __uint_as_float(sv[i + 1]);
+                float& mi = m[h * 2 + ((i >> 1) & 1)];
+                if constexpr (kPlain)
+                  mi = max3(mi, a0, a1);
+                else
+                  mi = max3(mi, (h * 32 + i < limit) ? a0 : -INFINITY, (h * 32 + i + 1 < limit) ? a1 : -INFINITY);
               }
+            }
+            return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])) * p.scale_log2;
+          };
+          uint32_t packed[32];
+          float l_blk, poly_max;
+          // p = exp2(s * scale - m_ref), row sum, P rounded to 16 bits (kernel_forward.h:785-824)
+          auto exponentials = [&] {
+            const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+            const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), negm2 = pack2(-m_use, -m_use);
+            uint64_t lsum2 = pack2(0.f, 0.f);
+            poly_max = -INFINITY;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t(&sv)[32] = h == 0 ? s0 : s1;
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {
+                float x0, x1, p0, p1;
+                unpack2(fma2(pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, negm2), x0, x1);
+                if (((i >> 1) & 7) < kPolyOf8) {  // compile-time: the loop is unrolled
+                  poly_max = max3(poly_max, x0, x1);
+                  exp2_poly2(x0, x1, p0, p1);
+                } else {
+                  p0 = exp2f(x0);
+                  p1 = exp2f(x1);
+                }
+                if (!kPlain) {
+                  p0 = (h * 32 + i < limit) ? p0 : 0.f;
+                  p1 = (h * 32 + i + 1 < limit) ? p1 : 0.f;
+                }
+                lsum2 = add2(lsum2, pack2(p0, p1));
+                packed[h * 16 + (i >> 1)] = E::from_float2(p0, p1);
+              }
+            }
+            float l0, l1;
+            unpack2(lsum2, l0, l1);
+            l_blk = l0 + l1;
+          };
+          if (j == 0) m_ref = row_max();  // nothing has been accumulated yet
+          exponentials();
+          // A row's reference maximum is raised only when its block has outgrown it: no p exceeds the row's sum, so a sum of
+          // at most kMaxRowSum shows that every P was in range (a sum that is no number, or a score too far up for the
+          // polynomial, counts as out of range). The maximum itself is looked for only then, with the scores read again:
+          // taking it in every block cost 200 of a block's 1250 cycles. The TMEM accesses are warp-wide, so the decision is
+          // too; rows that did not move get alpha = 1.
+          if (j > 0 && __any_sync(0xffffffffu, !(l_blk <= kMaxRowSum) || poly_max > 120.f || m_ref == -INFINITY)) {
+            tmem_ld_32x32b_x32(s_addr, s0);
+            tmem_ld_32x32b_x32(s_addr + 32, s1);
+            tmem_ld_wait();
+            const float m_new = fmaxf(m_ref, row_max());
+            // O holds blocks 0 .. j-1 once P(j-1) V(j-1) is done; P(j) V(j) cannot start before this thread's arrival on
+            // p_full below
+            if (!mbar_wait(&kv_empty[(g - 1) % Cfg::kKvStages], ((g - 1) / Cfg::kKvStages) & 1, abort_flag, p.status,
+                           kDevWaitAccFullTimeout)) {
+              ok = false;
+            } else {
+              tc_fence_after();
+              const float alpha = (m_new == -INFINITY) ? 1.f : exp2f(m_ref - m_new);  // m_ref = -inf: O is 0 anyway
+              const uint64_t alpha2 = pack2(alpha, alpha);
+#pragma unroll 1
+              for (int c = 0; c < DCH * 4; ++c) {
+                if (c * 16 < p.Dv) {  // warp-uniform
+                  uint32_t v[16];
+                  tmem_ld_32x32b_x16(o_addr + c * 16, v);
+                  tmem_ld_wait();
+#pragma unroll
+                  for (int i = 0; i < 16; i += 2) {
+                    float x0, x1;
+                    unpack2(mul2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), alpha2), x0, x1);
+                    v[i] = __float_as_uint(x0);
+                    v[i + 1] = __float_as_uint(x1);
+                  }
+                  tmem_st_32x32b_x16(o_addr + c * 16, v);
+                }
+              }
+              tmem_st_wait();
+              l_run *= alpha;
             }
             m_ref = m_new;
+            exponentials();
           }
-          ATTN_PROBE(2)  // row max (+ rescale when it happens)
-          const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-          // p = exp2(s * scale - m_ref), row sum, P rounded to 16 bits (kernel_forward.h:785-824) and written as
-          // pairs over the first 32 columns of this S buffer: every S value of the row is in registers by now
-          const uint64_t scale2 = pack2(p.scale_log2, p.scale_log2), negm2 = pack2(-m_use, -m_use);
-          uint64_t lsum2 = pack2(0.f, 0.f);
-          uint32_t packed[32];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint32_t(&sv)[32] = h == 0 ? s0 : s1;
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              float x0, x1;
-              unpack2(fma2(pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale2, negm2), x0, x1);
-#ifdef B200AIT_ATTN_EXP_SKIP  // tuning experiment: no exponentials, to expose the MMA side's own pace
-              float p0 = x0, p1 = x1;
-#else
-              float p0, p1;
-              if (((i >> 1) & 7) < kPolyOf8) {  // compile-time: the loop is unrolled
-                exp2_poly2(x0, x1, p0, p1);
-              } else {
-                p0 = exp2f(x0);
-                p1 = exp2f(x1);
-              }
-#endif
-              if (!kPlain) {
-                p0 = (h * 32 + i < limit) ? p0 : 0.f;
-                p1 = (h * 32 + i + 1 < limit) ? p1 : 0.f;
-              }
-              lsum2 = add2(lsum2, pack2(p0, p1));
-              packed[h * 16 + (i >> 1)] = E::from_float2(p0, p1);
-            }
-          }
+          // as pairs over the first 32 columns of this S buffer: every score of the row has been used by now
           tmem_st_32x32b_x32(s_addr, packed);
-          unpack2(lsum2, l0, l1);
+          l_run += l_blk;
         };
         if constexpr (NOMASK) {
           softmax_block(std::true_type{});
@@ -644,11 +612,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
           else
             softmax_block(std::false_type{});
         }
-        l_run += l0 + l1;
         tmem_st_wait();  // P is in TMEM
         tc_fence_before();
         mbar_arrive(&p_full[g & 1]);
-        ATTN_PROBE(3)  // exp2 pass, P to TMEM, fence, arrive
         if (j == 0 && ok) ok = flush_pending();  // the previous item's O, now that this item's first P is on its way
       }
       gb += n_blocks;
@@ -659,11 +625,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
         pend.inv_l = (l_run > 0.f) ? 1.f / l_run : 0.f;
         pend.out = (q_idx < w.q_len) ? static_cast<T*>(p.out) + ((w.out_row0 + q_idx) * p.H + w.h) * p.Dv : nullptr;
       }
-      ATTN_PROBE(0)  // item bookkeeping (booked with the wait for S)
       ++it;
     }
     if (ok) ok = flush_pending();  // the last item of this CTA
-    ATTN_PROBE_FLUSH(0)
   }
 
   tc_fence_before();
@@ -985,15 +949,3 @@ B200AIT_EXPORT int b200ait_flash_attention(void* output, const void* qkv, const 
     attention_run(output, q, k, v, p, total_rows, total_rows, false, dtype == kDTypeBFloat16, stream);
   });
 }
-
-#ifdef B200AIT_ATTN_PROBE
-// tuning builds only: copies the probe counters to the host and clears them
-B200AIT_EXPORT int b200ait_attn_probe_read(long long* out32) {
-  return guarded("b200ait_attn_probe_read", [&] {
-    B200AIT_CUDA_CHECK(cudaDeviceSynchronize());
-    B200AIT_CUDA_CHECK(cudaMemcpyFromSymbol(out32, g_attn_probe, sizeof(long long) * 32));
-    long long zero[32] = {};
-    B200AIT_CUDA_CHECK(cudaMemcpyToSymbol(g_attn_probe, zero, sizeof(zero)));
-  });
-}
-#endif
