@@ -149,3 +149,20 @@ def test_random_shapes_bit_exact():
         rng.shuffle(dims)
         x = torch.randn(shape, generator=gen).to(dtype)
         assert torch.equal(kernels.permute(x.cuda(), dims).cpu(), x.permute(dims).contiguous()), f"permute {shape} {dims} {dtype}"
+
+
+@pytest.mark.parametrize("batch,rows,cols", [(33, 72, 104), (64, 384, 64), (1, 64, 64), (7, 136, 1000), (16, 200, 520), (3, 66, 72), (2, 72, 70), (1, 8, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.int16])
+@pytest.mark.parametrize("offset", [0, 8, 4, 1])
+def test_transpose_vectors(batch, rows, cols, dtype, offset):
+    """The transpose in 16-byte pieces (rows, columns and addresses all multiples of 16 bytes) and its neighbours that take
+    narrower ones: full and partial 64 x 64 tiles, operands that begin `offset` elements into their allocation."""
+    from aitemplate_b200 import kernels
+
+    n = batch * rows * cols
+    flat = torch.randint(-32768, 32767, (n + offset,), dtype=torch.int16, generator=torch.Generator().manual_seed(n))
+    x = flat.view(dtype)[offset:].view(batch, rows, cols)
+    xg = flat.cuda().view(dtype)[offset:].view(batch, rows, cols)
+    assert xg.data_ptr() % 16 == 2 * offset % 16
+    y = kernels.permute(xg, (0, 2, 1))
+    assert torch.equal(y.cpu().view(torch.int16), x.permute(0, 2, 1).contiguous().view(torch.int16))
