@@ -171,6 +171,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   using Cfg = AttnCfg<DCH, LONE>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {  // swizzled tiles need 1024-byte alignment
+    grid_wait();
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kDevBadSmemAlignment);
     return;
   }
@@ -236,6 +237,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     return w;
   };
   if constexpr (SKIP) {
+    grid_wait();  // (this early: the sequence lengths are read)
     // The condition always holds, but the compiler does not know: it would keep this decoding of the first item in registers
     // for the roles to share (8 packed causal sequences of 512 .. 4096 rows, 16 heads of 128: 250 us; 256 .. 260 so, no skip 254).
     if (gridDim.x == p.num_items && decode_item(blockIdx.x).n_blocks == 0) return;
@@ -258,6 +260,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
+    grid_release();
     tmem_relinquish();
   }
   tc_fence_before();
@@ -266,6 +269,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   else
     named_bar_sync(kSetupBar, kAttnThreads);
   tc_fence_after();
+  if constexpr (!SKIP) grid_wait();
   const uint32_t tmem_base = *tmem_slot;    // (nothing yet in warp 0, which has no use for it)
   const uint32_t tmem_s = tmem_base;        // S(j) at + (j & 1) * 64; P(j) as 16-bit pairs over its first 32 columns
   const uint32_t tmem_o = tmem_base + 128;  // O of item it at + o_buf(it) * kTWidth
@@ -744,8 +748,10 @@ void launch_attn_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   constexpr int kSmemBytes = AttnCfg<DCH, LONE>::kSmemBytes;
   static std::atomic<uint64_t> configured{0};
   opt_in_smem_once(configured, reinterpret_cast<const void*>(kernel), kSmemBytes);
-  ::b200ait::count_launch(), kernel<<<grid, kAttnThreads, kSmemBytes, stream>>>(tq, tk, tv, p);
-  B200AIT_CUDA_CHECK(cudaGetLastError());
+  // early where a CTA walks few items, for the reason given at gemm_starts_early (rules.h): 2 x 8 heads x 4096 rows x 40, 1.7 items
+  // a CTA, is worth 2 us behind its projection; in a layer of 4 x 4096 rows with 12 heads, 5.2 a CTA, it cost 11 of 534 us
+  const bool early = 2ll * p.num_items <= 5ll * grid;
+  launch_early(kernel, dim3(grid), kAttnThreads, kSmemBytes, stream, early, 1, tq, tk, tv, p);
 }
 
 template <int DCH, bool BF16, bool NOMASK, bool LONE = false>

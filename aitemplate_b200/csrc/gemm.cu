@@ -385,6 +385,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     __syncwarp();
   } else if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);  // two accumulators
+    grid_release();
     tmem_relinquish();
   }
   tc_fence_before();
@@ -396,6 +397,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     if (warp != 1) cluster_wait();  // the peers' barriers are initialised before anything signals them
   }
   tc_fence_after();
+  grid_wait();
   bool epi_arrived = false;  // this thread has arrived at the closing cluster barrier
 
   if (warp == 0) {
@@ -788,20 +790,8 @@ static void launch_swapab(const CUtensorMap& tw, const CUtensorMap& tx, const Ge
                           int num_groups, cudaStream_t stream) {
   using Cfg = SwapCfg<MX, R, H>;
   const int walkers = swapab_resident_clusters<BF16, MX, R, H>();  // also opts the kernel in to its shared memory
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(R * std::min(num_slabs * num_groups, walkers)));
-  cfg.blockDim = dim3(kSwapThreads);
-  cfg.dynamicSmemBytes = Cfg::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = R;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  ::b200ait::count_launch();
-  B200AIT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, &gemm_swapab_kernel<BF16, MX, R, H>, tw, tx, p, num_slabs, num_groups));
+  launch_early(&gemm_swapab_kernel<BF16, MX, R, H>, dim3(static_cast<unsigned>(R * std::min(num_slabs * num_groups, walkers))),
+               kSwapThreads, Cfg::kSmemBytes, stream, true, R, tw, tx, p, num_slabs, num_groups);
 }
 
 // The instantiations the planner chooses from: MX rows of X per group, K split R ways, exchange in H passes.

@@ -489,9 +489,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   } else if (warp == 1) {
     if (PAIR) {  // the same warp of both CTAs, same result slot
       tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
+      grid_release();
       tmem_relinquish_pair();
     } else {
       tmem_alloc(tmem_slot, Cfg::kTmemCols);
+      grid_release();
       tmem_relinquish();
     }
   } else if (threadIdx.x == 64) {
@@ -512,6 +514,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     named_bar_sync(kSetupBar, kGemmThreads);
   if (PAIR) cluster_wait();
   tc_fence_after();
+  grid_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -922,9 +925,8 @@ void launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout
   static std::atomic<uint64_t> configured{0};
   opt_in_smem_once(configured, reinterpret_cast<const void*>(&gemm_tc_kernel<BN, BF16, EPI, false, BMN, MULTI>),
                    Cfg::kSmemBytes);
-  ::b200ait::count_launch(), gemm_tc_kernel<BN, BF16, EPI, false, BMN, MULTI><<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(
-      ta, tb, tout.m[0], ta, p, tout);
-  B200AIT_CUDA_CHECK(cudaGetLastError());
+  launch_early(&gemm_tc_kernel<BN, BF16, EPI, false, BMN, MULTI>, dim3(static_cast<unsigned>(grid)), kGemmThreads, Cfg::kSmemBytes,
+               stream, gemm_starts_early(p.num_units, grid, p.tma_store), 1, ta, tb, tout.m[0], ta, p, tout);
 }
 
 // CTA-pair variant: `grid` counts CTAs (twice the number of pairs); launched as clusters of two.
@@ -935,20 +937,8 @@ void launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps&
   static std::atomic<uint64_t> configured{0};
   auto* kernel = &gemm_tc_kernel<BN, BF16, EPI, true, BMN, MULTI>;
   opt_in_smem_once(configured, reinterpret_cast<const void*>(kernel), Cfg::kSmemBytes);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(kGemmThreads);
-  cfg.dynamicSmemBytes = Cfg::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  ::b200ait::count_launch();
-  B200AIT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tout.m[0], td0, p, tout));
+  launch_early(kernel, dim3(static_cast<unsigned>(grid)), kGemmThreads, Cfg::kSmemBytes, stream,
+               gemm_starts_early(p.num_units, grid / 2, p.tma_store), 2, ta, tb, tout.m[0], td0, p, tout);
 }
 
 // Epilogues that get their own straight-line instantiation: bias, relu, gelu, fast_gelu, add, add_relu, mul. Everything

@@ -31,6 +31,8 @@ struct CopyBatch {
 
 template <typename V>
 __global__ void __launch_bounds__(256) copy2d_kernel(const CopyBatch batch) {
+  grid_release();
+  grid_wait();
   const CopyJob j = batch.job[blockIdx.y];
   const long long total = batch.rows * j.row_vecs;
   const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -93,11 +95,11 @@ void run_copies(const std::vector<HostCopy>& copies, long long rows, cudaStream_
     const unsigned gx = static_cast<unsigned>(std::min<long long>((max_vecs + per_block - 1) / per_block, 148 * 16));
     dim3 grid(std::max(gx, 1u), n);
     switch (vec) {
-      case 16: ::b200ait::count_launch(), copy2d_kernel<uint4><<<grid, 256, 0, stream>>>(b); break;
-      case 8: ::b200ait::count_launch(), copy2d_kernel<uint2><<<grid, 256, 0, stream>>>(b); break;
-      case 4: ::b200ait::count_launch(), copy2d_kernel<uint32_t><<<grid, 256, 0, stream>>>(b); break;
-      case 2: ::b200ait::count_launch(), copy2d_kernel<uint16_t><<<grid, 256, 0, stream>>>(b); break;
-      default: ::b200ait::count_launch(), copy2d_kernel<uint8_t><<<grid, 256, 0, stream>>>(b); break;
+      case 16: launch_early(&copy2d_kernel<uint4>, grid, 256, 0, stream, true, 1, b); break;
+      case 8: launch_early(&copy2d_kernel<uint2>, grid, 256, 0, stream, true, 1, b); break;
+      case 4: launch_early(&copy2d_kernel<uint32_t>, grid, 256, 0, stream, true, 1, b); break;
+      case 2: launch_early(&copy2d_kernel<uint16_t>, grid, 256, 0, stream, true, 1, b); break;
+      default: launch_early(&copy2d_kernel<uint8_t>, grid, 256, 0, stream, true, 1, b); break;
     }
     B200AIT_CUDA_CHECK(cudaGetLastError());
   }
@@ -118,6 +120,8 @@ struct PermuteParams {
 // one, and a thread does one per dimension for each 16-byte vector it moves).
 template <typename V, typename I>
 __global__ void __launch_bounds__(256) permute_gather_kernel(const PermuteParams p) {
+  grid_release();
+  grid_wait();
   const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.total; i += step) {
     I rem = static_cast<I>(i), off = 0;
@@ -138,6 +142,8 @@ __global__ void __launch_bounds__(256) permute_gather_kernel(const PermuteParams
 template <typename V>
 __global__ void __launch_bounds__(256) transpose_kernel(const V* __restrict__ src, V* __restrict__ dst, long long R,
                                                         long long C) {
+  grid_release();
+  grid_wait();
   __shared__ V tile[32][33];
   const long long b = blockIdx.z;
   const V* s = src + b * R * C;
@@ -161,6 +167,8 @@ __global__ void __launch_bounds__(256) transpose_kernel(const V* __restrict__ sr
 // warp reads and writes full 128-byte lines (the 32 x 32 kernel above moves 64-byte half lines of 16-bit data).
 __global__ void __launch_bounds__(256) transpose16_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst,
                                                           long long R, long long C) {
+  grid_release();
+  grid_wait();
   __shared__ __align__(4) uint16_t tile[64][66];
   const long long b = blockIdx.z;
   const uint16_t* s = src + b * R * C;
@@ -194,6 +202,8 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const uint16_t* __rest
 // 24 x [512 x 512] 8.2 -> 6.3, 12 x [384 x 64] 2.2 -> 1.8. No shape measured was slower (13, smallest 1 x [64 x 64]: 1.8 -> 1.4).
 __global__ void __launch_bounds__(256) transpose16_vec_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst,
                                                               long long R, long long C) {
+  grid_release();
+  grid_wait();
   __shared__ __align__(16) uint32_t tile[64 * 32];
   const long long b = blockIdx.z;
   const uint16_t* s = src + b * R * C;
@@ -281,12 +291,12 @@ void permute_run(const void* src, void* dst, const int64_t* in_shape, const int6
           (reinterpret_cast<uintptr_t>(src) & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
         dim3 grid64(static_cast<unsigned>((C + 63) / 64), static_cast<unsigned>((R + 63) / 64), static_cast<unsigned>(B));
         const bool vec = R % 8 == 0 && C % 8 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
-        ::b200ait::count_launch(), (vec ? transpose16_vec_kernel : transpose16_kernel)<<<grid64, 256, 0, stream>>>(
-            static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
+        launch_early(vec ? &transpose16_vec_kernel : &transpose16_kernel, grid64, 256, 0, stream, true, 1,
+                     static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
       } else if (elem_size == 2)
-        ::b200ait::count_launch(), transpose_kernel<uint16_t><<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
+        launch_early(&transpose_kernel<uint16_t>, grid, 256, 0, stream, true, 1, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
       else
-        ::b200ait::count_launch(), transpose_kernel<uint32_t><<<grid, 256, 0, stream>>>(static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), R, C);
+        launch_early(&transpose_kernel<uint32_t>, grid, 256, 0, stream, true, 1, static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), R, C);
       B200AIT_CUDA_CHECK(cudaGetLastError());
       return;
     }
@@ -317,9 +327,9 @@ void permute_run(const void* src, void* dst, const int64_t* in_shape, const int6
 #define B200AIT_GATHER(V)                                                   \
   do {                                                                      \
     if (small)                                                              \
-      ::b200ait::count_launch(), permute_gather_kernel<V, uint32_t><<<grid, 256, 0, stream>>>(p);      \
+      launch_early(&permute_gather_kernel<V, uint32_t>, dim3(grid), 256, 0, stream, true, 1, p); \
     else                                                                    \
-      ::b200ait::count_launch(), permute_gather_kernel<V, long long><<<grid, 256, 0, stream>>>(p);     \
+      launch_early(&permute_gather_kernel<V, long long>, dim3(grid), 256, 0, stream, true, 1, p); \
   } while (0)
   switch (vec) {
     case 16: B200AIT_GATHER(uint4); break;
@@ -404,6 +414,8 @@ __device__ __forceinline__ long long ew_index(const EwParams& p, int i, long lon
 
 template <bool BF16>
 __global__ void __launch_bounds__(256) elementwise_kernel(const EwParams p) {
+  grid_release();
+  grid_wait();
   using E = Elem16<BF16>;
   using T = typename E::T;
   const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -618,9 +630,9 @@ B200AIT_EXPORT int b200ait_elementwise(void* output, const int64_t* out_shape, i
     const long long work = vec ? p.total / 8 : p.total;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((work + 255) / 256, 148 * 32));
     if (dtype == kDTypeBFloat16)
-      ::b200ait::count_launch(), elementwise_kernel<true><<<grid, 256, 0, stream>>>(p);
+      launch_early(&elementwise_kernel<true>, dim3(grid), 256, 0, stream, true, 1, p);
     else
-      ::b200ait::count_launch(), elementwise_kernel<false><<<grid, 256, 0, stream>>>(p);
+      launch_early(&elementwise_kernel<false>, dim3(grid), 256, 0, stream, true, 1, p);
     B200AIT_CUDA_CHECK(cudaGetLastError());
   });
 }

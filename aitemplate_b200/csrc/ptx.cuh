@@ -436,6 +436,13 @@ template <int REGS>
 __device__ __forceinline__ void reg_give() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
 }
+// Kernels launched by launch_early (common.h) may be resident before the kernel ahead of them on the stream has finished:
+// everything that reads or writes global memory comes after grid_wait, which every thread of every CTA calls (a CTA that left
+// without it could let the next kernel but one start too early).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel's CTAs may become resident once every CTA of this grid has called this or has left. A kernel that allocates
+// tensor memory calls it after its allocation: a waiting CTA of the next kernel must not hold the columns that this one needs.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // arrives at a named barrier (and publishes what was written before) without waiting for the others
 __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

@@ -66,6 +66,8 @@ struct LayerNormParams {
 template <int VPL, bool BF16>
 __global__ void __launch_bounds__(256, (VPL >= 12) ? 2 : (VPL >= 6) ? 4 : (VPL >= 3) ? 6 : 8)
     layernorm_warp_kernel(const LayerNormParams p) {
+  grid_release();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= p.m) return;
@@ -384,7 +386,7 @@ void layernorm_launch(const LayerNormParams& p, cudaStream_t stream) {
     const int wpb = (vpl <= 4) ? 8 : 4;  // warps per block
     const unsigned grid = static_cast<unsigned>((p.m + wpb - 1) / wpb);
     const int threads = wpb * 32;
-#define B200AIT_LN(V) ::b200ait::count_launch(), layernorm_warp_kernel<V, BF16><<<grid, threads, 0, stream>>>(p)
+#define B200AIT_LN(V) launch_early(&layernorm_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, true, 1, p)
     if (vpl <= 1)
       B200AIT_LN(1);
     else if (vpl <= 2)
@@ -445,6 +447,8 @@ struct SoftmaxParams {
 
 template <int VPL, bool BF16>
 __global__ void __launch_bounds__(256) softmax_warp_kernel(const SoftmaxParams p) {
+  grid_release();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= p.outer) return;
@@ -752,7 +756,7 @@ void softmax_launch(const SoftmaxParams& p, cudaStream_t stream) {
     const int wpb = (vpl <= 4) ? 8 : 4;
     const unsigned grid = static_cast<unsigned>((p.outer + wpb - 1) / wpb);
     const int threads = wpb * 32;
-#define B200AIT_SM(V) ::b200ait::count_launch(), softmax_warp_kernel<V, BF16><<<grid, threads, 0, stream>>>(p)
+#define B200AIT_SM(V) launch_early(&softmax_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, true, 1, p)
     if (vpl <= 1)
       B200AIT_SM(1);
     else if (vpl <= 2)
