@@ -9,10 +9,10 @@
 // by one persistent, warp-specialised kernel:
 //   warp 0      TMA producer: cp.async.bulk.tensor loads of 128x64 (A) and BNx64 (B) tiles into a
 //               128-byte-swizzled shared-memory ring guarded by full/empty mbarriers
-//   warp 1      MMA issuer: one thread issues tcgen05.mma (M=128, N=BN, K=16) into one of two TMEM
+//   warp 1      MMA issuer: tcgen05.mma (M=128, N=BN, K=16) into one of two TMEM
 //               accumulators, tcgen05.commit releases smem stages / publishes the accumulator
-//   warps 2-5   epilogue: tcgen05.ld of this warp's 32 TMEM lanes, bias / activation / residual in
-//               fp32, one rounding, 16-byte global stores (row-major with stride, or permuted)
+//   warps 2-9   epilogue: tcgen05.ld of this warp's 32 TMEM lanes, bias / activation / residual in fp32, one
+//               rounding, staged TMA or 16-byte global stores (row-major with stride, or permuted)
 // The epilogue of tile i overlaps the main loop of tile i+1 (two accumulators).
 // Shapes that TMA cannot address (K or a leading stride not a multiple of 8 elements, unaligned
 // pointers) run on a plain tiled CUDA-core kernel in this file; there is no host fallback.
