@@ -216,7 +216,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
     w.h = bh - b * p.H;
     w.q0 = q_blk * kBlockM;
     if (p.cu_seqlens) {
-      const int lo = __ldg(p.cu_seqlens + b), hi = __ldg(p.cu_seqlens + b + 1);
+      const int lo = p.cu_seqlens[b], hi = p.cu_seqlens[b + 1];
       w.b4 = 0;
       w.row0 = lo;
       w.q_len = w.kv_len = max(hi - lo, 0);
@@ -227,8 +227,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
       w.q_len = p.Sq;
       w.kv_len = p.Skv;
       if constexpr (!NOMASK) {  // (the host sends problems with lengths to the masking variant)
-        if (p.lengths_q) w.q_len = min(max(__ldg(p.lengths_q + b), 0), p.Sq);
-        if (p.lengths_kv) w.kv_len = min(max(__ldg(p.lengths_kv + b), 0), p.Skv);
+        if (p.lengths_q) w.q_len = min(max(p.lengths_q[b], 0), p.Sq);
+        if (p.lengths_kv) w.kv_len = min(max(p.lengths_kv[b], 0), p.Skv);
       }
       w.out_row0 = static_cast<long long>(b) * p.Sq;
     }

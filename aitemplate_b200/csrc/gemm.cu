@@ -514,8 +514,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       const bool vec = p.vec_ok && col0 + 8 <= p.N;
       float bias_v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (vec && p.bias != nullptr)
-        unpack8<BF16>(__ldg(reinterpret_cast<const uint4*>(static_cast<const typename Elem16<BF16>::T*>(p.bias) + col0)),
-                      bias_v);
+        unpack8<BF16>(*reinterpret_cast<const uint4*>(static_cast<const typename Elem16<BF16>::T*>(p.bias) + col0), bias_v);
       ok = mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, kDevWaitAccFullTimeout);
       if (!ok) break;
       tc_fence_after();
@@ -641,7 +640,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
               const int jj = j + 8 * t < my_rows ? j + 8 * t : j;
-              if (add_d0) r0[t] = __ldg(reinterpret_cast<const uint4*>(res0 + static_cast<long long>(out_row0 + jj) * p.ldd));
+              if (add_d0) r0[t] = *reinterpret_cast<const uint4*>(res0 + static_cast<long long>(out_row0 + jj) * p.ldd);
               const float* src = tile + jj * 128 + (et & 15) * 8;
               const float4 a0 = *reinterpret_cast<const float4*>(src), a1 = *reinterpret_cast<const float4*>(src + 4);
               o[t][0] = a0.x, o[t][1] = a0.y, o[t][2] = a0.z, o[t][3] = a0.w;
@@ -683,8 +682,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
               o[t * 8 + 0] = a0.x, o[t * 8 + 1] = a0.y, o[t * 8 + 2] = a0.z, o[t * 8 + 3] = a0.w;
               o[t * 8 + 4] = a1.x, o[t * 8 + 5] = a1.y, o[t * 8 + 6] = a1.z, o[t * 8 + 7] = a1.w;
               const long long d_at = static_cast<long long>(out_row0 + jj) * p.ldd + col0;
-              if (b1 != kBinaryNone) r0[t] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.d0) + d_at));
-              if (b2 != kBinaryNone) r1[t] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.d1) + d_at));
+              if (b1 != kBinaryNone) r0[t] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.d0) + d_at);
+              if (b2 != kBinaryNone) r1[t] = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.d1) + d_at);
             }
             if (!pre) {
 #pragma unroll

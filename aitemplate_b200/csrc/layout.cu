@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) copy2d_kernel(const CopyBatch batch) {
       const long long i = i0 + u * step;
       if (i < total) {
         const long long r = i / j.row_vecs, c = i - r * j.row_vecs;
-        v[u] = __ldcs(reinterpret_cast<const V*>(j.src + r * j.src_row_stride + c * sizeof(V)));
+        v[u] = ld_stream(reinterpret_cast<const V*>(j.src + r * j.src_row_stride + c * sizeof(V)));
         dst_off[u] = r * j.dst_row_stride + c * sizeof(V);
       }
     }
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) permute_gather_kernel(const PermuteParams
 
 // batched [R, C] -> [C, R] transpose of 16-bit or 32-bit elements through shared memory
 template <typename V>
-__global__ void __launch_bounds__(256) transpose_kernel(const V* __restrict__ src, V* __restrict__ dst, long long R,
+__global__ void __launch_bounds__(256) transpose_kernel(const V* src, V* dst, long long R,
                                                         long long C) {
   grid_release();
   grid_wait();
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const V* __restrict__ sr
 
 // The same transpose for 16-bit elements with even R and C: 64 x 64 tiles moved with 32-bit accesses, so that a
 // warp reads and writes full 128-byte lines (the 32 x 32 kernel above moves 64-byte half lines of 16-bit data).
-__global__ void __launch_bounds__(256) transpose16_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst,
+__global__ void __launch_bounds__(256) transpose16_kernel(const uint16_t* src, uint16_t* dst,
                                                           long long R, long long C) {
   grid_release();
   grid_wait();
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const uint16_t* __rest
     const int row = ty + i * 8;
     const long long r = r0 + row, c = c0 + 2 * tx;
     if (r < R && c < C)
-      *reinterpret_cast<uint32_t*>(&tile[row][2 * tx]) = __ldcs(reinterpret_cast<const uint32_t*>(s + r * C + c));
+      *reinterpret_cast<uint32_t*>(&tile[row][2 * tx]) = ld_stream(reinterpret_cast<const uint32_t*>(s + r * C + c));
   }
   __syncthreads();
 #pragma unroll
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const uint16_t* __rest
 // of eight rows and stores eight rows of each column; eight lanes fill 128 bytes of an output row. Bound by HBM.
 // 64 x [384 x 1024]: 24.6 us with 4-byte accesses, 17.0 here (floor at the copy rate 15.4, a plain copy 17.2); 8192 x 8192 64.9 -> 45.4,
 // 24 x [512 x 512] 8.2 -> 6.3, 12 x [384 x 64] 2.2 -> 1.8. No shape measured was slower (13, smallest 1 x [64 x 64]: 1.8 -> 1.4).
-__global__ void __launch_bounds__(256) transpose16_vec_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst,
+__global__ void __launch_bounds__(256) transpose16_vec_kernel(const uint16_t* src, uint16_t* dst,
                                                               long long R, long long C) {
   grid_release();
   grid_wait();
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256) transpose16_vec_kernel(const uint16_t* __
   for (int i = 0; i < 2; ++i) {
     const int row = (t >> 3) + i * 32;
     v[i] = make_uint4(0, 0, 0, 0);
-    if (r0 + row < R && c0 + group * 8 < C) v[i] = __ldcs(reinterpret_cast<const uint4*>(s + (r0 + row) * C + c0 + group * 8));
+    if (r0 + row < R && c0 + group * 8 < C) v[i] = ld_stream(reinterpret_cast<const uint4*>(s + (r0 + row) * C + c0 + group * 8));
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {

@@ -438,8 +438,37 @@ __device__ __forceinline__ void reg_give() {
 }
 // Kernels launched by launch_early (common.h) may be resident before the kernel ahead of them on the stream has finished:
 // everything that reads or writes global memory comes after grid_wait, which every thread of every CTA calls (a CTA that left
-// without it could let the next kernel but one start too early).
+// without it could let the next kernel but one start too early). What it reads there may still have been written while it was
+// resident, which rules out the read-only path (__ldg, `const T* __restrict__` parameters: their data must not change while the
+// kernel is resident, and the compiler may move such a load above the wait) and loads whose place the compiler does not
+// know to matter (__ldcs). So such kernels read through plain pointers or by ld_stream.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// a load with the streaming hint, which stays where it is written
+template <typename V>
+__device__ __forceinline__ V ld_stream(const V* p) {
+  static_assert(sizeof(V) == 16 || sizeof(V) == 8 || sizeof(V) == 4 || sizeof(V) == 2 || sizeof(V) == 1, "a vector or an element");
+  if constexpr (sizeof(V) == 16) {
+    uint4 v;
+    asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+  } else if constexpr (sizeof(V) == 8) {
+    uint2 v;
+    asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+  } else if constexpr (sizeof(V) == 4) {
+    uint32_t v;
+    asm volatile("ld.global.cs.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+  } else if constexpr (sizeof(V) == 2) {
+    uint16_t v;
+    asm volatile("ld.global.cs.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+  } else {
+    uint16_t v;
+    asm volatile("ld.global.cs.u8 %0, [%1];" : "=h"(v) : "l"(p));
+    return static_cast<V>(v);
+  }
+}
 // The next kernel's CTAs may become resident once every CTA of this grid has called this or has left. A kernel that allocates
 // tensor memory calls it after its allocation: a waiting CTA of the next kernel must not hold the columns that this one needs.
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

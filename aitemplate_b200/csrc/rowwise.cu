@@ -23,7 +23,6 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-__device__ __forceinline__ uint4 ld_stream(const uint4* p) { return __ldcs(p); }
 __device__ __forceinline__ void st_stream(uint4* p, const uint4& v) { __stcs(p, v); }
 
 // block-wide reductions (result broadcast to every thread); `red` holds >= 33 floats
@@ -116,13 +115,13 @@ __global__ void __launch_bounds__(256, (VPL >= 12) ? 2 : (VPL >= 6) ? 4 : (VPL >
       float f[8], g[8], b[8], o[8];
       unpack8<BF16>(raw[i], f);
       if (g4) {
-        unpack8<BF16>(__ldg(g4 + v), g);
+        unpack8<BF16>(g4[v], g);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) g[j] = 1.f;
       }
       if (b4) {
-        unpack8<BF16>(__ldg(b4 + v), b);
+        unpack8<BF16>(b4[v], b);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) b[j] = 0.f;
@@ -225,13 +224,13 @@ __global__ void __launch_bounds__(512) layernorm_wide_kernel(const LayerNormPara
       float f[8], g[8], b[8], o[8];
       unpack8<BF16>(raw[i], f);
       if (g4) {
-        unpack8<BF16>(__ldg(g4 + v), g);
+        unpack8<BF16>(g4[v], g);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) g[j] = 1.f;
       }
       if (b4) {
-        unpack8<BF16>(__ldg(b4 + v), b);
+        unpack8<BF16>(b4[v], b);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) b[j] = 0.f;
@@ -301,7 +300,7 @@ __global__ void __launch_bounds__(512) layernorm_block_staged_kernel(const Layer
     const uint32_t* x2 = reinterpret_cast<const uint32_t*>(x);
     uint32_t* xs2 = reinterpret_cast<uint32_t*>(xs);
     for (int i = tid; i < (p.n >> 1); i += nt) {
-      const uint32_t w = __ldcs(x2 + i);
+      const uint32_t w = ld_stream(x2 + i);
       xs2[i] = w;
       const float2 f = E::to_float2(w);
       s += f.x + f.y;
@@ -331,13 +330,13 @@ __global__ void __launch_bounds__(512) layernorm_block_staged_kernel(const Layer
       float f[8], gv[8], bv[8], o[8];
       unpack8<BF16>(reinterpret_cast<const uint4*>(xs)[i], f);
       if (g) {
-        unpack8<BF16>(__ldg(g8 + i), gv);
+        unpack8<BF16>(g8[i], gv);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) gv[j] = 1.f;
       }
       if (b) {
-        unpack8<BF16>(__ldg(b8 + i), bv);
+        unpack8<BF16>(b8[i], bv);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) bv[j] = 0.f;
@@ -638,7 +637,7 @@ __global__ void __launch_bounds__(512) softmax_block_staged_kernel(const Softmax
     const uint32_t* x2 = reinterpret_cast<const uint32_t*>(x);
     uint32_t* xs2 = reinterpret_cast<uint32_t*>(xs);
     for (int i = tid; i < (p.k >> 1); i += nt) {
-      const uint32_t w = __ldcs(x2 + i);
+      const uint32_t w = ld_stream(x2 + i);
       xs2[i] = w;
       const float2 f = E::to_float2(w);
       mx = fmaxf(mx, fmaxf(f.x, f.y));
