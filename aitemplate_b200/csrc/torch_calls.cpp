@@ -286,19 +286,19 @@ PyObject* concatenate(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     if (n == 0) return unhandled();
     std::vector<const void*> pointers;
     std::vector<const int64_t*> shapes;
-    std::vector<at::Tensor> held;  // (the list may change while the lock is released)
-    const at::Tensor* first = nullptr;
+    // The list may change while the lock is released, or under a dispatch mode while the output is allocated: from here on the
+    // tensors are read through `held` alone.
+    std::vector<at::Tensor> held;
     std::vector<int64_t> shape;
     int64_t dim = 0;
     for (Py_ssize_t i = 0; i < n; ++i) {
       const at::Tensor* t = plain(PySequence_Fast_GET_ITEM(args[0], i));
       if (!t || t->numel() == 0) return unhandled();
       if (i == 0) {
-        first = t;
         shape.assign(t->sizes().begin(), t->sizes().end());
         if (!as_dim(args[1], t->dim(), &dim)) return unhandled();
       } else {
-        if (t->dim() != first->dim() || t->scalar_type() != first->scalar_type()) return unhandled();
+        if (t->dim() != held[0].dim() || t->scalar_type() != held[0].scalar_type()) return unhandled();
         for (int64_t j = 0; j < t->dim(); ++j)
           if (j != dim && t->size(j) != shape[j]) return unhandled();
         shape[dim] += t->size(dim);
@@ -309,11 +309,11 @@ PyObject* concatenate(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     }
     const std::vector<uint8_t> masks(n, 1);
     std::vector<int64_t> out_shape(shape.size());
-    at::Tensor out = first->new_empty(shape);
+    at::Tensor out = held[0].new_empty(shape);
     const b200ait_stream_t stream = current_stream();
     if (unlocked([&] {
-          return lib.concatenate(out.data_ptr(), out_shape.data(), pointers.data(), shapes.data(), masks.data(), dim, first->dim(), n,
-                                 static_cast<int64_t>(first->element_size()), stream);
+          return lib.concatenate(out.data_ptr(), out_shape.data(), pointers.data(), shapes.data(), masks.data(), dim, held[0].dim(), n,
+                                 static_cast<int64_t>(held[0].element_size()), stream);
         }))
       return failed("b200ait_concatenate");
     return THPVariable_Wrap(std::move(out));

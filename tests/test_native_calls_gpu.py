@@ -108,6 +108,23 @@ def test_refused_calls(name, monkeypatch):
     assert isinstance(native, tuple) and native == python
 
 
+def test_concatenate_of_a_list_that_changes_during_the_call():
+    """Allocating the output may run Python code (a dispatch mode), and other threads run while the kernel is launched: the tensors
+    of the call are the ones it was given."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Clears(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            parts.clear()
+            return func(*args, **(kwargs or {}))
+
+    want = torch.cat([_t(5, 3, 16), _t(5, 4, 16, seed=1)], dim=1)
+    parts = [_t(5, 3, 16), _t(5, 4, 16, seed=1)]
+    with Clears():
+        y = K.concatenate(parts, dim=1)
+    assert not parts and torch.equal(y, want)
+
+
 def test_run_with_tensors(tmp_path):
     from aitemplate_b200.compiler import compile_model
     from aitemplate_b200.testing import detect_target, workloads
