@@ -171,7 +171,7 @@ __device__ __forceinline__ void epilogue_chunk32(const GemmParams& p, float (&v)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float f[8];
-        unpack8<BF16>(reinterpret_cast<const uint4*>(bias)[q], f);
+        unpack8<BF16>(__ldg(reinterpret_cast<const uint4*>(bias) + q), f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[q * 8 + j] += f[j];
       }
@@ -190,7 +190,7 @@ __device__ __forceinline__ void epilogue_chunk32(const GemmParams& p, float (&v)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float f[8];
-        unpack8<BF16>(reinterpret_cast<const uint4*>(d0)[q], f);
+        unpack8<BF16>(__ldg(reinterpret_cast<const uint4*>(d0) + q), f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[q * 8 + j] = (b1 == kBinaryAdd) ? v[q * 8 + j] + f[j] : v[q * 8 + j] * f[j];
       }
@@ -209,7 +209,7 @@ __device__ __forceinline__ void epilogue_chunk32(const GemmParams& p, float (&v)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float f[8];
-        unpack8<BF16>(reinterpret_cast<const uint4*>(d1)[q], f);
+        unpack8<BF16>(__ldg(reinterpret_cast<const uint4*>(d1) + q), f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[q * 8 + j] = (b2 == kBinaryAdd) ? v[q * 8 + j] + f[j] : v[q * 8 + j] * f[j];
       }
