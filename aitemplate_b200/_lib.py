@@ -44,6 +44,7 @@ def _signatures():
                                                c_void_p, c_int64, c_int, c_void_p],
         ),
         "b200ait_gemm_rcr_workspace_bytes": (c_int, [c_int64] * 4 + [c_int, c_int, I64P]),
+        "b200ait_gemm_rcr_scratch_bytes": (c_int, [c_int64] * 3 + [c_int, c_int, I64P]),
         "b200ait_gemm_rrr": (
             c_int,
             [c_void_p] * 6 + [c_int64] * 12 + [c_int, c_int, c_float, c_int, c_void_p, c_int64, c_int, c_void_p],
@@ -136,7 +137,7 @@ def load() -> ctypes.CDLL:
 
 
 # entry points that torch_calls.so calls, in the order of its Library structure
-_CALLED = ["b200ait_gemm_rcr", "b200ait_gemm_rrr", "b200ait_gemm_rcr_workspace_bytes", "b200ait_mem_eff_attention",
+_CALLED = ["b200ait_gemm_rcr", "b200ait_gemm_rrr", "b200ait_gemm_rcr_scratch_bytes", "b200ait_mem_eff_attention",
            "b200ait_flash_attention", "b200ait_layernorm", "b200ait_softmax", "b200ait_concatenate", "b200ait_split",
            "b200ait_permute", "b200ait_last_error", "AITemplateModelContainerRun"]
 _calls = None

@@ -833,10 +833,10 @@ static const std::vector<SwapKernel>& swap_kernels() {
 // plus a second wave's worth if the units outnumber the resident clusters; up to 64 output tiles of 128 x 128, 48 with an
 // added residual, 32 with another epilogue.
 //
-// From 64 to 2048 rows: by the estimates of rules.h, X in groups that are as small as it takes to fill one wave. The tile
+// From 64 rows on: by the estimates of rules.h, X in groups that are as small as it takes to fill one wave. The tile
 // kernels' are the firmer ones where both are close.
 static const SwapKernel* plan_swapab(const GemmProblem& g, int tile_width, bool bf16) {
-  if (g.n < 128 || g.m < 5 || g.k < 256 || g.m > 2048) return nullptr;
+  if (g.n < 128 || g.m < 5 || g.k < 256) return nullptr;
   const long long slabs = (g.n + 127) / 128, kb_total = (g.k + kBK - 1) / kBK;
   const auto& table = swap_kernels();
   const SwapKernel* best = nullptr;
@@ -864,11 +864,11 @@ static const SwapKernel* plan_swapab(const GemmProblem& g, int tile_width, bool 
     return best;
   }
   for (const SwapKernel& sk : table) {
-    if (kb_total < sk.r) continue;
+    if (kb_total < sk.r || !gemm_swap_in_range(g.m, ((g.m + sk.mx - 1) / sk.mx) * slabs, sk.resident(bf16))) continue;
     const double us = gemm_swap_us(g, sk.mx, sk.r, sk.resident(bf16));
     if (best == nullptr || us < best_us) best = &sk, best_us = us;
   }
-  return best_us < 0.97 * gemm_tile_us(g, tile_width, sm_count()) ? best : nullptr;
+  return best != nullptr && best_us < 0.97 * gemm_tile_us(g, tile_width, sm_count()) ? best : nullptr;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1010,7 +1010,8 @@ struct SplitPlan {
   int tile_n, splits, kb_per_split;
   long long bytes;
 };
-// `tile_n`: the caller's choice or 0, `planned_tile_n` what is taken for it. `streams`: the weight-streaming kernels could have taken the problem; where their planner preferred unsplit tiles, they stay so.
+// `tile_n`: the caller's choice or 0, `planned_tile_n` what is taken for it. `streams`: operands and hints are such that the
+// weight-streaming kernels could have taken the problem (gemm_may_split in rules.h).
 SplitPlan plan_split_k(const GemmProblem& g, int tile_n, int planned_tile_n, int max_splits, long long workspace_bytes,
                        bool streams) {
   const long long batch = g.batch, m = g.m, n = g.n, k = g.k;
@@ -1018,7 +1019,7 @@ SplitPlan plan_split_k(const GemmProblem& g, int tile_n, int planned_tile_n, int
   const long long num_kb = (k + kBK - 1) / kBK;
   sp.kb_per_split = static_cast<int>(num_kb);
   const long long sms = sm_count();
-  if (max_splits == 1 || num_kb < 4 || (max_splits == 0 && streams && m >= 5 && n >= 128)) return sp;
+  if (max_splits == 1 || num_kb < 4 || (max_splits == 0 && streams && !gemm_may_split(m, n, k))) return sp;
   const int width = std::min(sp.tile_n, 256);  // (CTA pairs never split K)
   // One tile row (M <= 128): the run time is the time to stream the weights once. A tcgen05 MMA takes as long
   // as its M x K says, whatever N is, so a CTA consumes weight rows fastest through wide tiles: 128- and
@@ -1146,8 +1147,8 @@ void gemm_run(const GemmArgs& g_in) {
   B200AIT_REQUIRE(tma_ok || g.num_out == 1, "gemm: several output buffers need TMA-addressable operands");
   // M <= 4, deep K, the caller left tile width and split-K to the library: stream W once on the CUDA cores
   const long long rowdot_smem = (g.m <= 1 ? 1 : g.m <= 2 ? 2 : 4) * g.k * 2;
-  if (tma_ok && g.batch == 1 && g.m <= kRowDotMaxM && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0 &&
-      g.k >= 1024 && g.n >= 64 && rowdot_smem <= 160 * 1024) {
+  if (tma_ok && g.batch == 1 && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0 &&
+      gemm_rowdot_long(g.m, g.n, g.k)) {
     const unsigned grid = static_cast<unsigned>(std::min<long long>(sm_count(), (g.n + 3) / 4));
     const int smem = static_cast<int>(rowdot_smem);
 #define B200AIT_ROWDOT(BF, MR)                                                                                 \
@@ -1403,7 +1404,7 @@ B200AIT_EXPORT int b200ait_gemm_rcr_multi_out(const void* a, const void* b, cons
   });
 }
 
-// Bytes of split-K workspace b200ait_gemm_rcr would use for this problem if given enough.
+// The most split-K workspace that b200ait_gemm_rcr or b200ait_gemm_rrr would use for a problem of these sizes if given enough.
 B200AIT_EXPORT int b200ait_gemm_rcr_workspace_bytes(int64_t batch, int64_t m, int64_t n, int64_t k, int tile_n,
                                                     int split_k, int64_t* bytes_out) {
   return guarded("b200ait_gemm_rcr_workspace_bytes", [&] {
@@ -1412,6 +1413,18 @@ B200AIT_EXPORT int b200ait_gemm_rcr_workspace_bytes(int64_t batch, int64_t m, in
     if (batch <= 0 || m <= 0 || n <= 0 || k <= 0) return;
     if (tile_n == kTilePair) return;
     const GemmProblem g{batch, m, n, k, 0, 0, k, false};
+    *bytes_out = plan_split_k(g, tile_n, tile_n ? tile_n : choose_tile_n(g), split_k, 1ll << 62, false).bytes;
+  });
+}
+
+// The same for one unbatched launch of b200ait_gemm_rcr: 0 for the kernels that take none.
+B200AIT_EXPORT int b200ait_gemm_rcr_scratch_bytes(int64_t m, int64_t n, int64_t k, int tile_n, int split_k, int64_t* bytes_out) {
+  return guarded("b200ait_gemm_rcr_scratch_bytes", [&] {
+    B200AIT_REQUIRE(bytes_out, "bytes_out is null");
+    *bytes_out = 0;
+    if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || tile_n == kTilePair || split_k == 1) return;
+    if (tile_n == 0 && split_k == 0 && !gemm_may_split(m, n, k)) return;
+    const GemmProblem g{1, m, n, k, 0, 0, k, false};
     *bytes_out = plan_split_k(g, tile_n, tile_n ? tile_n : choose_tile_n(g), split_k, 1ll << 62, false).bytes;
   });
 }

@@ -169,6 +169,10 @@ inline double gemm_swap_us(const GemmProblem& g, int mx, int r, int resident) {
   const double tail = 0.0268 * mx * (r - 1) / r + row * mx / r;
   return 3.79 + stream + tail + static_cast<double>(waves - 1) * (std::max(stream, tail) + 0.8);
 }
+// The weight-streaming kernel in more rows than 2048: only where its units are one wave. The estimate does not hold for several waves
+// of large groups (8192 x 640 x 8192: 111 us, 74 by the estimate, tiles 91), in one wave it does (4096 x 128 x 8192: 12.7 us, tiles
+// 19.3, tiles with K in two parts 18.8; 2049 x 128 x 8192: 8.7, 17.2 and 15.6, 4096 x 128 x 2048: 6.2, 6.8 and 11.7).
+inline bool gemm_swap_in_range(long long m, long long units, int resident) { return m <= 2048 || units <= resident; }
 inline int gemm_best_width(const GemmProblem& g, int sms) {
   int best = 64;
   for (int width : {128, 256, kGemmPairWidth}) {
@@ -176,6 +180,18 @@ inline int gemm_best_width(const GemmProblem& g, int sms) {
     if (gemm_tile_us(g, width, sms) < gemm_tile_us(g, best, sms)) best = width;
   }
   return best;
+}
+
+// GEMM, unbatched, aligned operands, neither a tile width nor a number of splits asked for: one to four rows of X against long rows of
+// W (which fit in shared memory, 160 KB) go to the CUDA cores,
+inline bool gemm_rowdot_long(long long m, long long n, long long k) {
+  return m <= 4 && n >= 64 && k >= 1024 && (m <= 2 ? m : 4) * k <= 80 * 1024;
+}
+// and K is shared out through scratch memory only where no weight-streaming kernel could have taken the problem. Where one could, it or
+// whole tiles are ahead of K in parts: over M = 5 .. 8192, N = 128 .. 640 and K = 2048 .. 8192 the best of three widths and five
+// numbers of parts took 1.08 to 2.7 times as long as the launch chosen here.
+inline bool gemm_may_split(long long m, long long n, long long k) {
+  return !(m >= 5 && n >= 128) && !gemm_rowdot_long(m, n, k);
 }
 
 // May a tile kernel's CTAs become resident before the kernel ahead of it has ended (launch_early)? It saves 0.4 .. 0.8 us (3 .. 25 %

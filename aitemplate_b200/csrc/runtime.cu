@@ -41,6 +41,7 @@ int b200ait_gemm_rcr(const void*, const void*, const void*, const void*, const v
                      int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, int, float,
                      int, int64_t, int64_t, int64_t, int, void*, int64_t, int, cudaStream_t);
 int b200ait_gemm_rcr_workspace_bytes(int64_t, int64_t, int64_t, int64_t, int, int, int64_t*);
+int b200ait_gemm_rcr_scratch_bytes(int64_t, int64_t, int64_t, int, int, int64_t*);
 int b200ait_bmm_permute0213(const void*, const void*, void*, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t,
                             int64_t, int, int, float, int, cudaStream_t);
 int b200ait_gemm_rrr(const void*, const void*, const void*, const void*, const void*, void*, int64_t, int64_t, int64_t,
@@ -273,7 +274,9 @@ class Executor {
     blob_ = alloc_.Allocate(static_cast<size_t>(plan.blob_bytes));
     // one split-K scratch area shared by every GEMM of the plan, sized for the hungriest of them at the
     // lower and upper bound of its dynamic dims (reference: global workspace = max over ops,
-    // python/aitemplate/compiler/transform/memory_planning.py:141-195)
+    // python/aitemplate/compiler/transform/memory_planning.py:141-195). gemm_rrr launches of a plan split as far as that
+    // area goes, at sizes at which gemm_rcr has kernels that need none: with one in the plan the area is sized for either.
+    const bool either = std::any_of(plan.ops.begin(), plan.ops.end(), [](const OpInfo& op) { return op.kernel == "gemm_rrr"; });
     for (const OpInfo& op : plan.ops) {
       if (op.kernel != "gemm_rcr") continue;
       const TensorInfo& a = plan.tensors[op.operands[0]];
@@ -297,7 +300,9 @@ class Executor {
       const int split_hint = op.ints.size() > 8 ? static_cast<int>(op.ints[8]) : 0;
       for (int64_t m : ms) {
         int64_t bytes = 0;
-        if (b200ait_gemm_rcr_workspace_bytes(1, m, b.dims[0].v, a.dims.back().v, tile_hint, split_hint, &bytes) == 0)
+        const int64_t n = b.dims[0].v, k = a.dims.back().v;
+        if ((either ? b200ait_gemm_rcr_workspace_bytes(1, m, n, k, tile_hint, split_hint, &bytes)
+                    : b200ait_gemm_rcr_scratch_bytes(m, n, k, tile_hint, split_hint, &bytes)) == 0)
           workspace_bytes_ = std::max(workspace_bytes_, bytes);
       }
     }

@@ -29,7 +29,7 @@ namespace {
 struct Library {
   decltype(&b200ait_gemm_rcr) gemm_rcr;
   decltype(&b200ait_gemm_rrr) gemm_rrr;
-  decltype(&b200ait_gemm_rcr_workspace_bytes) workspace_bytes;
+  decltype(&b200ait_gemm_rcr_scratch_bytes) scratch_bytes;
   decltype(&b200ait_mem_eff_attention) attention;
   decltype(&b200ait_flash_attention) flash_attention;
   decltype(&b200ait_layernorm) layernorm;
@@ -127,13 +127,8 @@ PyObject* gemm_rcr(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     const int64_t k = x->size(-1), n = w->size(0);
     if (k == 0 || w->size(1) != k || x->numel() == 0 || n == 0) return unhandled();
     const int64_t m = x->numel() / k;
-    // Scratch for split-K goes the long way. Asked for only where a launch could split: not where a kernel without partial sums
-    // takes the problem (five rows of X and more against 128 columns, or a few rows against many channels).
-    const bool whole = k % 8 == 0 && (reinterpret_cast<uintptr_t>(x->data_ptr()) | reinterpret_cast<uintptr_t>(w->data_ptr())) % 16 == 0;
-    const bool no_scratch = tile_n == 0 && split_k == 0 && whole &&
-                            ((m >= 5 && n >= 128) || (m <= 4 && n >= 64 && k >= 1024 && (m == 3 ? 4 : m) * k <= 80 * 1024));
-    if (split_k != 1 && !no_scratch &&
-        (lib.workspace_bytes(1, m, n, k, static_cast<int>(tile_n), static_cast<int>(split_k), &ws) != 0 || ws != 0))
+    // (a launch that takes scratch goes the long way)
+    if (split_k != 1 && (lib.scratch_bytes(m, n, k, static_cast<int>(tile_n), static_cast<int>(split_k), &ws) != 0 || ws != 0))
       return unhandled();
     std::vector<int64_t> shape(x->sizes().begin(), x->sizes().end());
     shape.back() = n;

@@ -156,7 +156,7 @@ def gemm_rcr(
         ldc = out.stride(0)          # a column block of a wider buffer is written in place
     ws = None
     if split_k != 1 and m and n and k:
-        ws_bytes = _workspace_bytes(torch._C._cuda_getDevice(), m, n, k, tile_n, split_k)
+        ws_bytes = _scratch_bytes(torch._C._cuda_getDevice(), m, n, k, tile_n, split_k)
         if ws_bytes:
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
     code = _lib.load().b200ait_gemm_rcr(
@@ -262,7 +262,7 @@ def bmm_permute(a: torch.Tensor, b: torch.Tensor, d1: int, b_row_major: bool = F
 
 
 def gemm_workspace_bytes(batch: int, m: int, n: int, k: int, tile_n: int = 0, split_k: int = 0) -> int:
-    """Bytes of fp32 split-K scratch the library would use for this problem (0 = it would not split)."""
+    """The most fp32 split-K scratch that a gemm_rcr or gemm_rrr of these sizes would use (0 = neither would split)."""
     out = c_int64(0)
     _lib.check(_lib.load().b200ait_gemm_rcr_workspace_bytes(batch, m, n, k, tile_n, split_k, ctypes.byref(out)),
                "b200ait_gemm_rcr_workspace_bytes")
@@ -270,9 +270,12 @@ def gemm_workspace_bytes(batch: int, m: int, n: int, k: int, tile_n: int = 0, sp
 
 
 @functools.lru_cache(maxsize=4096)
-def _workspace_bytes(device: int, m: int, n: int, k: int, tile_n: int, split_k: int) -> int:
-    """gemm_workspace_bytes() of an unbatched problem, which depends on its sizes and the current device only."""
-    return gemm_workspace_bytes(1, m, n, k, tile_n, split_k)
+def _scratch_bytes(device: int, m: int, n: int, k: int, tile_n: int, split_k: int) -> int:
+    """Bytes of fp32 split-K scratch an unbatched gemm_rcr takes, by its sizes and the current device."""
+    out = c_int64(0)
+    _lib.check(_lib.load().b200ait_gemm_rcr_scratch_bytes(m, n, k, tile_n, split_k, ctypes.byref(out)),
+               "b200ait_gemm_rcr_scratch_bytes")
+    return out.value
 
 
 def bmm_rcr(a: torch.Tensor, b: torch.Tensor, alpha: float = 1.0, tile_n: int = 0) -> torch.Tensor:

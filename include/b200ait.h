@@ -71,9 +71,12 @@ int b200ait_gemm_rcr(const void* a, const void* b, const void* bias, const void*
  * when the output tiles cannot fill the GPU and K is deep, K is divided among CTAs that write fp32 partial
  * sums into `workspace` ([splits, batch, m, n] floats) and a second kernel reduces them and applies the
  * epilogue. split_k: 0 = library chooses, 1 = off, n = at most n. A null workspace disables splitting.
- * b200ait_gemm_rcr_workspace_bytes reports what the library would use for a problem. */
+ * b200ait_gemm_rcr_workspace_bytes reports the most that b200ait_gemm_rcr or b200ait_gemm_rrr would use for a problem of these
+ * sizes. An unbatched b200ait_gemm_rcr with tile_n = 0 and split_k = 0 uses none where m >= 5 and n >= 128, nor for a few rows
+ * against long ones: b200ait_gemm_rcr_scratch_bytes reports what such a launch on contiguous operands uses. */
 int b200ait_gemm_rcr_workspace_bytes(int64_t batch, int64_t m, int64_t n, int64_t k, int tile_n, int split_k,
                                      int64_t* bytes_out);
+int b200ait_gemm_rcr_scratch_bytes(int64_t m, int64_t n, int64_t k, int tile_n, int split_k, int64_t* bytes_out);
 /* b200ait_gemm_rcr with B stored [batch, k, n] (n contiguous, row stride ldb): gemm_rrr / gemm_rrr_bias / bmm_rrr
  * (python/aitemplate/compiler/ops/gemm_universal/gemm_rrr.py:26-80, bmm_xxx.py:223-260). No permuted store. */
 int b200ait_gemm_rrr(const void* a, const void* b, const void* bias, const void* d0, const void* d1, void* c,

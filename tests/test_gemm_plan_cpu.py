@@ -17,6 +17,8 @@ extern "C" double tile_us(long long m, long long n, long long k, int e, int widt
 extern "C" double swap_us(long long m, long long n, long long k, int e, int mx, int r) {
   return gemm_swap_us(GemmProblem{1, m, n, k, e, e, k, false}, mx, r, r == 2 ? 74 : r == 4 ? 33 : 15);
 }
+extern "C" bool swap_in_range(long long m, long long units, int resident) { return gemm_swap_in_range(m, units, resident); }
+extern "C" bool may_split(long long m, long long n, long long k) { return gemm_may_split(m, n, k); }
 extern "C" int best_width(long long b, long long m, long long n, long long k, int e) {
   return gemm_best_width(GemmProblem{b, m, n, k, e, e, k, false}, 148);
 }
@@ -32,6 +34,7 @@ def plan(tmp_path_factory):
                     os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     lib = ctypes.CDLL(str(lib))
     lib.tile_us.restype = lib.swap_us.restype = ctypes.c_double
+    lib.swap_in_range.restype = lib.may_split.restype = ctypes.c_bool
     return lib
 
 
@@ -72,3 +75,19 @@ def test_weight_streaming_estimates(plan, m, n, k, e, mx, r, us):
     ])
 def test_widths(plan, batch, m, n, k, e, width):
     assert plan.best_width(*_ll(batch, m, n, k), e) == width
+
+
+@pytest.mark.parametrize("m,n,taken", [(2048, 8192, True), (2049, 128, True), (4096, 128, True), (4800, 128, False), (8192, 640, False)])
+def test_weight_streaming_of_many_rows_is_one_wave(plan, m, n, taken):
+    """No K in parts from 128 columns on, so whatever splitting was for has to be in reach of the kernel that takes its place."""
+    assert not plan.may_split(*_ll(m, n, 8192))
+    units = -(-m // 64) * -(-n // 128)
+    assert plan.swap_in_range(*_ll(m, units), 74) == taken
+    if taken and m > 2048:
+        assert plan.swap_us(*_ll(m, n, 8192), 0, 64, 2) < 0.97 * min(plan.tile_us(*_ll(m, n, 8192), 0, w) for w in (64, 128, 256, 512))
+
+
+@pytest.mark.parametrize("m,n,k,split", [(4, 8192, 8192, False), (4, 8192, 20488, True), (2, 64, 40960, False), (2, 64, 40968, True),
+                                          (1, 63, 4096, True), (5, 127, 4096, True), (5, 128, 4096, False), (3, 64, 1016, True)])
+def test_where_k_may_be_split(plan, m, n, k, split):
+    assert plan.may_split(*_ll(m, n, k)) == split
