@@ -375,6 +375,7 @@ struct Side {
   std::vector<AITData> data;
   std::vector<const at::Tensor*> tensors;
   std::vector<PyObject*> names;
+  std::vector<size_t> given_order;  // the indexes in the order of the caller's dictionary
   bool read(PyObject* given, PyObject* index_of) {
     if (!PyDict_CheckExact(given) || !PyDict_CheckExact(index_of) || PyDict_GET_SIZE(given) != PyDict_GET_SIZE(index_of)) return false;
     const size_t n = static_cast<size_t>(PyDict_GET_SIZE(given));
@@ -399,7 +400,7 @@ struct Side {
         case at::kBool: dtype = AITemplateDtype::kBool; break;
         default: return false;
       }
-      names[i] = name, tensors[i] = t;
+      names[i] = name, tensors[i] = t, given_order.push_back(static_cast<size_t>(i));
       data[i] = AITData(t->data_ptr(), AITemplateParamShape(t->sizes().data(), static_cast<size_t>(t->dim())), dtype);
     }
     return true;
@@ -407,7 +408,7 @@ struct Side {
 };
 
 // run_model(handle, inputs, outputs, input name -> index, output name -> index, dimensions of each output, stream or None, sync,
-// graph mode) -> {name: the output as the run shaped it}
+// graph mode) -> {name: the output as the run shaped it}, in the order of `outputs`
 PyObject* run_model(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
     if (n_args != 9) return unhandled();
@@ -442,7 +443,7 @@ PyObject* run_model(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
                                       shape_pointers.data()));
     });
     PyObject* result = code ? failed("AITemplateModelContainerRun") : PyDict_New();
-    for (size_t i = 0; i < names.size(); ++i) {
+    for (const size_t i : out.given_order) {
       if (result && !code) {
         const at::Tensor& t = held[in.tensors.size() + i];
         int64_t numel = 1;

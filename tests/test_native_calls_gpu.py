@@ -152,3 +152,26 @@ def test_run_with_tensors(tmp_path):
     model.close()
     with pytest.raises(RuntimeError, match="closed"):
         model.run_with_tensors({"hidden_states": x}, {"output_0": outs[0]})
+
+
+def test_run_with_tensors_returns_the_outputs_in_the_order_they_were_given(tmp_path):
+    from aitemplate_b200.compiler import compile_model, ops
+    from aitemplate_b200.frontend import Tensor
+    from aitemplate_b200.testing import detect_target
+
+    x = Tensor([4, 64], name="x", is_input=True)
+    outputs = []
+    for name, dim in (("first", 0), ("second", 1), ("third", 1)):
+        y = ops.softmax()(x, 1) if name == "first" else ops.concatenate()([x, x], dim)
+        y._attrs["name"], y._attrs["is_output"] = name, True
+        outputs.append(y)
+    model = compile_model(outputs, detect_target(), str(tmp_path), "ordered")
+    given = _t(4, 64)
+    shapes = {"first": (4, 64), "second": (4, 128), "third": (4, 128)}
+    for order in (["third", "first", "second"], ["second", "third", "first"], ["first", "second", "third"]):
+        outs = {name: torch.empty(shapes[name], dtype=torch.float16, device="cuda") for name in order}
+        got = model.run_with_tensors({"x": given}, outs)
+        assert list(got) == order
+        assert all(got[name].data_ptr() == outs[name].data_ptr() for name in order)
+        assert torch.equal(got["first"], K.softmax(given)) and torch.equal(got["third"], torch.cat([given, given], 1))
+    model.close()
