@@ -136,35 +136,60 @@ def load() -> ctypes.CDLL:
         return lib
 
 
-# entry points that torch_calls.so calls, in the order of its Library structure
+# entry points that csrc/torch_calls.cpp calls, in the order of its Library structure
 _CALLED = ["b200ait_gemm_rcr", "b200ait_gemm_rrr", "b200ait_gemm_rcr_scratch_bytes", "b200ait_mem_eff_attention",
            "b200ait_flash_attention", "b200ait_layernorm", "b200ait_softmax", "b200ait_concatenate", "b200ait_split",
            "b200ait_permute", "b200ait_last_error", "AITemplateModelContainerRun"]
 _calls = None
 
 
+class _NoCalls:
+    """In place of the native host path where there is none: answers None to every call, as that does to calls it leaves to the
+    Python code."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def calls_path() -> Path:
+    """The native host path built for the running torch and Python. It reads torch's objects through torch's own headers, so a
+    file made for another build of either must not be loaded; the name keeps them apart."""
+    import sysconfig
+
+    import torch
+
+    build = f"{torch.__version__}-{(torch.version.git_version or '')[:10]}-{sysconfig.get_config_var('SOABI')}"
+    return LIB_PATH.with_name(f"torch_calls-{build}.so")
+
+
 def load_calls():
-    """Loads torch_calls.so, the native host path of the eager calls, bound to the loaded library; raises if it has not been
-    built."""
+    """The native host path of the eager calls, bound to the loaded library. Without it (torch was updated and the package not
+    built again) the Python code behind it serves every call, with the same kernels and more time on the host."""
     global _calls
     if _calls is not None:
         return _calls
+    if not LIB_PATH.exists():
+        return _NoCalls()  # the Python code refuses what it would refuse anyway, and says for the rest what is missing
     lib = load()
     with _lock:
         if _calls is not None:
             return _calls
         import importlib.machinery
         import importlib.util
+        import warnings
 
         import torch
 
-        path = LIB_PATH.with_name("torch_calls.so")
-        if not path.exists():
-            raise RuntimeError(f"{path} is missing: build it with `python -m aitemplate_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("torch_calls", str(path))
-        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("torch_calls", loader))
-        loader.exec_module(module)
-        module.bind(tuple(ctypes.cast(getattr(lib, n), c_void_p).value for n in _CALLED), torch.nn.Parameter)
+        path = calls_path()
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("torch_calls", str(path))
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("torch_calls", loader))
+            loader.exec_module(module)
+            module.bind(tuple(ctypes.cast(getattr(lib, n), c_void_p).value for n in _CALLED), torch.nn.Parameter)
+        except ImportError as e:
+            warnings.warn(f"calls take a slower path on the host: {path.name} cannot be loaded ({e}); build it with "
+                          "`python -m aitemplate_b200.build`", RuntimeWarning, stacklevel=3)
+            module = _NoCalls()
         _calls = module
         return module
 

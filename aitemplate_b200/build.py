@@ -18,7 +18,6 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "libb200ait.so"
-CALLS_PATH = LIB_DIR / "torch_calls.so"
 OBJ_DIR = PKG_DIR / "build"
 
 NVCC_FLAGS = [
@@ -64,33 +63,37 @@ def _compile_one(src: Path, verbose: bool) -> Path:
 
 
 def build_calls(force: bool = False, verbose: bool = False) -> Path:
-    """Compiles csrc/torch_calls.cpp, the host path of the eager calls, against the installed torch."""
+    """Compiles csrc/torch_calls.cpp, the host path of the eager calls, against the installed torch. The file's name says which
+    build of torch and of Python it is for."""
     import sysconfig
 
     import torch
 
+    from . import _lib
+
+    out = _lib.calls_path()
     src, root = CSRC / "torch_calls.cpp", Path(torch.__file__).resolve().parent
-    newest = max(src.stat().st_mtime, _headers_mtime(), (root / "version.py").stat().st_mtime)
-    if not force and CALLS_PATH.exists() and CALLS_PATH.stat().st_mtime >= newest:
-        return CALLS_PATH
+    newest = max(src.stat().st_mtime, _headers_mtime())
+    if not force and out.exists() and out.stat().st_mtime >= newest:
+        return out
     cuda = Path(_nvcc()).resolve().parent.parent
     includes = [PKG_DIR.parent / "include", root / "include", root / "include/torch/csrc/api/include", cuda / "include",
                 Path(sysconfig.get_paths()["include"])]
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     cmd += [a for i in includes for a in ("-I", str(i))]
-    cmd += [str(src), "-o", str(CALLS_PATH), "-L", str(root / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    cmd += [str(src), "-o", str(out), "-L", str(root / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     if verbose:
         print(" ".join(cmd), flush=True)
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for {src.name}:\n{res.stdout}\n{res.stderr}")
-    return CALLS_PATH
+    return out
 
 
 def build_library(force: bool = False, verbose: bool = False) -> Path:
-    """Compiles csrc/*.cu for sm_100a and links lib/libb200ait.so, and builds lib/torch_calls.so beside it. Returns the
-    library's path."""
+    """Compiles csrc/*.cu for sm_100a and links lib/libb200ait.so, and builds the host path of the eager calls beside
+    it. Returns the library's path."""
     LIB_DIR.mkdir(exist_ok=True)
     OBJ_DIR.mkdir(exist_ok=True)
     if force:
@@ -100,7 +103,6 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
         calls = ex.submit(build_calls, force, verbose)
         objs = list(ex.map(lambda s: _compile_one(s, verbose), srcs))
-        calls.result()
     newest_obj = max(o.stat().st_mtime for o in objs)
     if force or not LIB_PATH.exists() or LIB_PATH.stat().st_mtime < newest_obj:
         cmd = [_nvcc(), "-shared", "-o", str(LIB_PATH), *map(str, objs)]
@@ -109,6 +111,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    calls.result()  # (the library is complete without it)
     return LIB_PATH
 
 
