@@ -3,6 +3,7 @@
 import pytest
 import torch
 
+from aitemplate_b200 import _lib
 from aitemplate_b200 import kernels as K
 
 pytestmark = pytest.mark.gpu
@@ -15,7 +16,25 @@ class _Absent:
         return lambda *args: None
 
 
-def _both(monkeypatch, call):
+class _Recorder:
+    """The native module, noting of every call whether it was served."""
+
+    def __init__(self):
+        self.module, self.served = _lib.load_calls(), []
+
+    def __getattr__(self, name):
+        function = getattr(self.module, name)
+
+        def call(*args):
+            y = function(*args)
+            self.served.append(y is not None)
+            return y
+
+        return call
+
+
+def _both(monkeypatch, call, served=None):
+    """call() as it is and without the native module; `served`: whether the native module has to have served it."""
     def run():
         try:
             y = call()
@@ -23,7 +42,11 @@ def _both(monkeypatch, call):
             return type(e), str(e)
         return y
 
-    native = run()
+    with monkeypatch.context() as m:
+        recorder = _Recorder()
+        m.setattr(K, "_calls", recorder)
+        native = run()
+        assert recorder.served == ([served] if served is not None else recorder.served)
     with monkeypatch.context() as m:
         m.setattr(K, "_calls", _Absent())
         python = run()
@@ -72,6 +95,8 @@ PLAIN = {
     "permute": lambda: K.permute(_t(2, 3, 4), (0, -1, 1)),
     "on_a_side_stream": lambda: _on_side_stream(lambda: K.softmax(_t(64, 64))),
 }
+# plain, but left to the Python code: scratch for split K, sections, no rows
+LONG_WAY = {"gemm_split_k", "gemm_narrow_deep", "gemm_no_rows", "split_sections"}
 REFUSED = {
     "strided": lambda: K.gemm_rcr(_t(72, 33).t(), _t(40, 72)),
     "host": lambda: K.softmax(torch.zeros(3, 4)),
@@ -98,7 +123,7 @@ def _on_side_stream(call):
 
 @pytest.mark.parametrize("name", PLAIN)
 def test_plain_calls(name, monkeypatch):
-    native, python = _both(monkeypatch, PLAIN[name])
+    native, python = _both(monkeypatch, PLAIN[name], served=name not in LONG_WAY)
     assert _same(native, python), (native, python)
 
 
@@ -125,7 +150,7 @@ def test_concatenate_of_a_list_that_changes_during_the_call():
     assert not parts and torch.equal(y, want)
 
 
-def test_run_with_tensors(tmp_path):
+def test_run_with_tensors(tmp_path, monkeypatch):
     from aitemplate_b200.compiler import compile_model
     from aitemplate_b200.testing import detect_target, workloads
 
@@ -135,11 +160,14 @@ def test_run_with_tensors(tmp_path):
     model.set_many_constants_with_tensors({n: params[k].cuda() for n, k in workloads.BERT_PARAM_NAMES.items()})
     x = x.cuda()
     outs = [torch.empty((2, 40, 768), dtype=torch.float16, device="cuda") for _ in range(3)]
+    recorder = _Recorder()
+    monkeypatch.setattr(_lib, "_calls", recorder)
     a = model.run_with_tensors({"hidden_states": x}, {"output_0": outs[0]})
     b = model.run_with_tensors([x], [outs[1]], graph_mode=True)  # lists take the Python code
     wider = torch.empty((2, 41, 768), dtype=torch.float16, device="cuda")  # more room than the run needs
     c = model.run_with_tensors({"hidden_states": x}, {"output_0": wider}, sync=False, stream_ptr=torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
+    assert recorder.served == [True, False, True]
     assert list(a) == list(b) == list(c) == ["output_0"]
     assert a["output_0"].data_ptr() == outs[0].data_ptr() and c["output_0"].shape == (2, 40, 768)
     assert torch.equal(a["output_0"], b["output_0"]) and torch.equal(a["output_0"], c["output_0"])
