@@ -51,7 +51,9 @@ struct Error : public std::runtime_error {
 // Launches a kernel in clusters of `cluster` CTAs. With `early` its CTAs may become resident while the kernel ahead of it on the
 // stream still runs, and wait there (grid_wait in ptx.cuh, which such a kernel has to call) until that one has finished and
 // its writes can be seen: the launch and the kernel's own set-up are then over when the data is ready. Between two launches of
-// the tile GEMM that is worth 0.5 .. 0.8 us (154 x 320 x 768: 4.6 -> 3.8 us, 384 x 768 x 768 + add: 5.0 -> 4.2).
+// the tile GEMM that is worth 0.5 .. 0.8 us (154 x 320 x 768: 4.6 -> 3.8 us, 384 x 768 x 768 + add: 5.0 -> 4.2). The other kernels
+// (one to four rows of X, the sum of split K, unaligned GEMMs, rows that a warp cannot hold in 16-byte pieces, reductions over an
+// inner dimension, attention without tensor cores) are launched with <<<>>>: an early launch of them has not been measured.
 template <class... Params, class... Args>
 void launch_early(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool early,
                   unsigned cluster, Args&&... args) {

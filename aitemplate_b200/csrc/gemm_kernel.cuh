@@ -880,7 +880,7 @@ void launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tout
   opt_in_smem_once(configured, reinterpret_cast<const void*>(&gemm_tc_kernel<BN, BF16, EPI, false, BMN, MULTI>),
                    Cfg::kSmemBytes);
   launch_early(&gemm_tc_kernel<BN, BF16, EPI, false, BMN, MULTI>, dim3(static_cast<unsigned>(grid)), kGemmThreads, Cfg::kSmemBytes,
-               stream, gemm_starts_early(p.num_units, grid, p.tma_store), 1, ta, tb, tout.m[0], ta, p, tout);
+               stream, gemm_starts_early(p.num_units, grid, p.tma_store, sm_count()), 1, ta, tb, tout.m[0], ta, p, tout);
 }
 
 // CTA-pair variant: `grid` counts CTAs (twice the number of pairs); launched as clusters of two.
@@ -892,7 +892,7 @@ void launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps&
   auto* kernel = &gemm_tc_kernel<BN, BF16, EPI, true, BMN, MULTI>;
   opt_in_smem_once(configured, reinterpret_cast<const void*>(kernel), Cfg::kSmemBytes);
   launch_early(kernel, dim3(static_cast<unsigned>(grid)), kGemmThreads, Cfg::kSmemBytes, stream,
-               gemm_starts_early(p.num_units, grid / 2, p.tma_store), 2, ta, tb, tout.m[0], td0, p, tout);
+               gemm_starts_early(p.num_units, grid / 2, p.tma_store, sm_count()), 2, ta, tb, tout.m[0], td0, p, tout);
 }
 
 // Epilogues that get their own straight-line instantiation: bias, relu, gelu, fast_gelu, add, add_relu, mul. Everything

@@ -427,15 +427,6 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   return d;
 }
 
-// registers of the warps of this warpgroup (all four execute it); the block's shares add up to what it was launched with
-template <int REGS>
-__device__ __forceinline__ void reg_take() {
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
-}
-template <int REGS>
-__device__ __forceinline__ void reg_give() {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
-}
 // Kernels launched by launch_early (common.h) may be resident before the kernel ahead of them on the stream has finished:
 // everything that reads or writes global memory comes after grid_wait, which every thread of every CTA calls (a CTA that left
 // without it could let the next kernel but one start too early). What it reads there may still have been written while it was

@@ -108,9 +108,11 @@ inline bool gemm_rows_output(int n, int tile_n, bool one_residual) {
 // GEMM: the time of a launch of the tile kernels (128 x 64, 128 x 128, 128 x 256 tiles, and 256 x 256 on CTA pairs: width 512)
 // and of the weight-streaming kernel, in us. Both were fitted to a sweep of 650 problems (M = 64 .. 3000, N and K = 256 .. 8192,
 // N whole and not whole 16-byte rows, three epilogues, every tile and every weight-streaming kernel forced, fp16, one launch
-// behind the other) and are within 5 % of it; the launch they pick takes 1.007 times the best one's time on average (1.003
-// where N is not a multiple of 8). The rules before (a width by whole waves at 512 cycles per k-block, K split over CTAs, the
-// weight-streaming kernel up to a number of tiles) took 1.055 and 1.14 times.
+// behind the other), with 5 % root mean square. Launches have become shorter since (launch_early): over 160 other problems of these
+// ranges the estimates lie 15 % off (root mean square; -30 % and +35 % at worst), mostly too long, all widths alike. The launch
+// they pick takes 1.017 times the best one's time on average, 1.49 at worst (625 x 368 x 320), and 18 of the 160 more than
+// 1.05. (The rules before, a width by whole waves at 512 cycles per k-block, K split over CTAs and the weight-streaming
+// kernel up to a number of tiles, took 1.055 and, with N not a multiple of 8, 1.14 times in the first sweep.)
 struct GemmProblem {
   long long batch, m, n, k;
   int epilogue;      // 0: bias [+ relu], 1: a residual operand, 2: another activation
@@ -200,6 +202,8 @@ inline bool gemm_may_split(long long m, long long n, long long k) {
 // us, 8192^3 857 -> 876, bmm 855 x [430 x 88 x 96] 30.0 -> 31.2 and 204 x [221 x 168 x 120], 2.8 tiles a CTA, 13.6 -> 14.1;
 // 352 x [76 x 88 x 128], 2.4 a CTA, 7.9 -> 7.3 and 8192 x 1280 x 320, 2.2, 13.2 -> 12.7), and where tiles are stored straight to
 // rows that share sectors it already does with one (700 x 5003 x 1024 + add 23.2 -> 25.5; 384 x 769 x 768 11.3 -> 10.8).
-inline bool gemm_starts_early(int units, int walkers, bool staged) { return staged ? 2ll * units <= 5ll * walkers : 2 * units <= 148; }
+inline bool gemm_starts_early(int units, int walkers, bool staged, int sms) {
+  return staged ? 2ll * units <= 5ll * walkers : 2ll * units <= sms;  // (unstaged: at most half of the SMs get a tile)
+}
 
 }  // namespace b200ait

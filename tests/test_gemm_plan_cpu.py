@@ -42,7 +42,8 @@ def _ll(*v):
     return [ctypes.c_longlong(x) for x in v]
 
 
-# the fit is within 5 % (root mean square); one problem may lie a few times that off
+# times of the sweep that the estimates were fitted to, which they match to 5 % (root mean square); one problem may lie a few
+# times that off
 @pytest.mark.parametrize(
     "m,n,k,e,width,us",
     [
