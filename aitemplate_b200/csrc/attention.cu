@@ -238,9 +238,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   };
   if constexpr (SKIP) {
     grid_wait();  // (this early: the sequence lengths are read)
-    // The condition always holds, but the compiler does not know: it would keep this decoding of the first item in registers
-    // for the roles to share (8 packed causal sequences of 512 .. 4096 rows, 16 heads of 128: 250 us; 256 .. 260 so, no skip 254).
-    if (gridDim.x == p.num_items && decode_item(blockIdx.x).n_blocks == 0) return;
+    // a CTA per item (8 packed causal sequences of 512 .. 4096 rows, 16 heads of 128: 231.6 us, without this end 236.3)
+    if (decode_item(blockIdx.x).n_blocks == 0) return;
   }
   const int dsteps = (p.D + 15) / 16;  // k-steps of Q K^T
 
