@@ -983,11 +983,12 @@ static GemmPlan plan_gemm(const GemmProblem& g, bool bf16, bool streams) {
   thread_local Slot slots[64] = {};
   const int sms = sm_count(), flags = 1 | (bf16 ? 2 : 0) | (streams ? 4 : 0);
   uint64_t h = static_cast<uint64_t>(g.batch);
-  for (const long long v : {g.m, g.n, g.k, g.pitch, static_cast<long long>(g.epilogue * 16 + g.swap_epilogue * 4 + g.generic * 64 + flags)})
+  for (const long long v : {g.m, g.n, g.k, g.pitch, static_cast<long long>(g.epilogue * 16 + g.swap_epilogue * 4 + g.generic * 64 + g.pairs * 128 + flags * 256)})
     h = (h ^ static_cast<uint64_t>(v)) * 0x9e3779b97f4a7c15ull;
   Slot& s = slots[h >> 58];
   if (s.flags == flags && s.sms == sms && s.g.batch == g.batch && s.g.m == g.m && s.g.n == g.n && s.g.k == g.k &&
-      s.g.epilogue == g.epilogue && s.g.swap_epilogue == g.swap_epilogue && s.g.pitch == g.pitch && s.g.generic == g.generic)
+      s.g.epilogue == g.epilogue && s.g.swap_epilogue == g.swap_epilogue && s.g.pitch == g.pitch && s.g.generic == g.generic &&
+      s.g.pairs == g.pairs)
     return s.plan;
   GemmPlan plan{choose_tile_n(g), nullptr};
   if (streams) plan.swap = plan_swapab(g, plan.tile_n, bf16);
@@ -1195,7 +1196,7 @@ void gemm_run(const GemmArgs& g_in) {
   const bool streams = tma_ok && g.batch == 1 && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0;
   // (row-major B: its boxes are not rows of K, and the figures of rules.h do not hold)
   const long long pitch = g.b_mn ? kBK : gemm_copy_row_us(g.lda) > gemm_copy_row_us(g.ldb) ? g.lda : g.ldb;
-  GemmProblem problem{g.batch, g.m, g.n, g.k, 0, 0, pitch, g.b_mn || g.num_out > 1};
+  GemmProblem problem{g.batch, g.m, g.n, g.k, 0, 0, pitch, g.b_mn || g.num_out > 1, p.c_bdiv == 0};
   GemmPlan planned{g.tile_n, nullptr};
   {
     const int code = p.epilogue;
@@ -1241,7 +1242,7 @@ void gemm_run(const GemmArgs& g_in) {
   // CTA pairs (256 x 256 tiles, cta_group::2): a third less operand traffic per flop into each SM, and a residual comes by
   // TMA into the staging boxes where the single-CTA kernels load it per thread.
   B200AIT_REQUIRE(!(force_pair && p.c_bdiv != 0), "bmm permute: the CTA-pair tiles do not take the permuted store");
-  const bool pair = force_pair || (sp.tile_n == kTilePair && p.c_bdiv == 0);
+  const bool pair = sp.tile_n == kTilePair;
   p.splits = sp.splits;
   p.kb_per_split = sp.kb_per_split;
   p.partial = static_cast<float*>(g.workspace);

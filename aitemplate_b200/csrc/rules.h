@@ -119,6 +119,7 @@ struct GemmProblem {
   int swap_epilogue; // as the weight-streaming kernel sees it: 0: bias [+ relu], 1: an added residual, 2: anything else
   long long pitch;   // of the operands' rows, in elements (the worse aligned one's)
   bool generic;      // an epilogue read from the parameters (row-major B, several destinations)
+  bool pairs = true; // CTA pairs can take it (they do not write the permuted batches of bmm_*_permute)
 };
 constexpr int kGemmPairWidth = 512;
 // What TMA takes for a 128-byte row of an operand box that does not start on a 128-byte boundary, in us: 2.85 cycles if it starts
@@ -127,7 +128,46 @@ constexpr int kGemmPairWidth = 512;
 inline double gemm_copy_row_us(long long pitch) {
   return pitch % 64 == 0 ? 0.0 : pitch % 32 == 0 ? 0.00086 : pitch % 16 == 0 ? 0.00100 : 0.00146;
 }
+// The same for batched problems, most of which are a few k-blocks deep and give every CTA many tiles: the step from one tile to the next,
+// not the launch, decides. Fitted to 1600 problems of 2 .. 1024 products (M 32 .. 1024, N 64 .. 1024, K 32 .. 1024, both storage
+// orders of B, fp16 and bf16, every width forced), 7 .. 16 % root mean square by row of the table; the widths they pick take 1.012
+// times the best one's time on average, 1.41 at worst. The estimate of single products, which was used here before, took 1.06 and 2.3
+// times, and 47 of the 1600 were slower by more than 2 % than by the rule of whole waves ahead of it (now 11, the worst by 7 %):
+// 78 x [160 x 80 x 72] row-major B 11.8 us, 5.6 now (128 wide); 285 x [374 x 136 x 88] 22.4, 17.9 (256); 445 x [295 x 392 x 40] 50.9, 39.8.
+inline double gemm_batched_tile_us(const GemmProblem& g, int width, int sms) {
+  // launch and one epilogue; a k-block; a step's own cost and its share that goes by how full the tiles are; how much of the shorter one
+  // of step and main loop is not hidden by the longer; a chunk of 32 columns that the edge of N cuts, which the threads of
+  // 64-wide tiles store element by element
+  struct Cost {
+    double once, k_block, step, filled, exposed, cut;
+  };
+  static constexpr Cost whole[4] = {{2.90, 0.151, 0.10, 1.04, 0.96, 2.07},
+                                    {2.80, 0.149, 0.37, 0.56, 1.00, 0.0},
+                                    {3.31, 0.250, 0.38, 1.71, 1.00, 0.0},
+                                    {3.93, 0.219, 0.67, 1.42, 1.00, 0.0}};
+  static constexpr Cost ragged[4] = {{7.11, 0.220, 4.54, 0.56, 0.06, 0.0},
+                                     {7.64, 0.122, 4.93, 0.0, 0.20, 0.0},
+                                     {11.74, 0.348, 9.53, 0.0, 0.16, 0.0},
+                                     {11.90, 0.324, 8.94, 0.59, 0.39, 0.0}};
+  static constexpr Cost row_major[4] = {{3.10, 0.196, 0.55, 0.48, 0.91, 2.75},
+                                        {4.04, 0.300, 1.32, 0.35, 0.36, 0.0},
+                                        {5.35, 0.468, 2.30, 1.31, 0.38, 0.0},
+                                        {5.69, 0.337, 2.42, 0.73, 0.39, 0.0}};
+  const bool pair = width == kGemmPairWidth;
+  const Cost& c = (g.generic ? row_major : g.n % 8 == 0 ? whole : ragged)[width == 64 ? 0 : width == 128 ? 1 : pair ? 3 : 2];
+  const long long bm = pair ? 256 : 128, bn = pair ? 256 : width, walkers = pair ? sms / 2 : sms;
+  const long long tiles_m = (g.m + bm - 1) / bm, tiles_n = (g.n + bn - 1) / bn, tiles = tiles_m * tiles_n * g.batch;
+  const double ctas = static_cast<double>(std::min(tiles, walkers) * (pair ? 2 : 1));
+  const int rows = pair ? 256 : 128 + width;
+  const double loop = static_cast<double>((g.k + 63) / 64) * std::max({c.k_block, 128.0 * rows * ctas / 22.1e6, rows * gemm_copy_row_us(g.pitch)});
+  const double cut = g.n % 8 == 0 && g.n % 32 != 0 ? c.cut : 0.0;
+  const double filled = static_cast<double>(g.m) * static_cast<double>(g.n) / static_cast<double>(tiles_m * bm * tiles_n * bn);
+  const double step = c.step + c.filled * filled + cut / static_cast<double>(tiles_n);
+  return c.once + cut + loop +
+         static_cast<double>((tiles + walkers - 1) / walkers - 1) * (std::max(loop, step) + c.exposed * std::min(loop, step));
+}
 inline double gemm_tile_us(const GemmProblem& g, int width, int sms) {
+  if (g.batch > 1) return gemm_batched_tile_us(g, width, sms);
   // launch, k-block, and a tile's epilogue by GemmProblem::epilogue; then what an epilogue costs beyond that where the tiles
   // of a CTA follow on each other's heels
   struct Cost {
@@ -153,10 +193,13 @@ inline double gemm_tile_us(const GemmProblem& g, int width, int sms) {
   const int rows = pair ? 256 : 128 + width;  // that a CTA fetches per k-block
   const double k_block = std::max({c.k_block, 128.0 * rows * ctas / 22.1e6, rows * gemm_copy_row_us(g.pitch)});
   const double loop = static_cast<double>((g.k + 63) / 64) * k_block;
-  // 64-wide tiles are stored by the threads, 64 bytes each, which are not whole sectors where the rows are not
   constexpr double kGeneric[4] = {0.0, 1.2, 1.5, 1.0};
-  const double epilogue = c.epilogue[g.epilogue] + (g.generic ? kGeneric[at] : 0.0) + (width == 64 && g.n % 16 != 0 ? (g.n % 8 == 0 ? 1.3 : 2.1) : 0.0);
-  return c.launch + loop + epilogue + static_cast<double>(waves - 1) * std::max(loop, epilogue + c.next);
+  const double epilogue = c.epilogue[g.epilogue] + (g.generic ? kGeneric[at] : 0.0) + (width == 64 && g.n % 8 != 0 ? 2.1 : 0.0);
+  // 64-wide tiles are stored by the threads, element by element where the edge of N cuts a chunk of 32 columns (625 x 368 x 320:
+  // 5.6 us, 3.8 with 128-wide tiles, which were passed over as long as this was charged by sectors, N % 16)
+  const double cut = width == 64 && g.n % 8 == 0 && g.n % 32 != 0 ? (g.n % 16 == 0 ? 1.1 : 2.1) : 0.0;
+  return c.launch + loop + epilogue + cut +
+         static_cast<double>(waves - 1) * std::max(loop, epilogue + c.next + cut / static_cast<double>((g.n + 63) / 64));
 }
 // mx rows of X per group, K split r ways over a cluster, `resident` clusters on the GPU at once
 inline double gemm_swap_us(const GemmProblem& g, int mx, int r, int resident) {
@@ -178,7 +221,7 @@ inline bool gemm_swap_in_range(long long m, long long units, int resident) { ret
 inline int gemm_best_width(const GemmProblem& g, int sms) {
   int best = 64;
   for (int width : {128, 256, kGemmPairWidth}) {
-    if (width == kGemmPairWidth && (g.n < 256 || (g.generic && g.k < 512))) break;  // (659 x [344 x 512 x 40], row-major B: 88 us, pairs 111)
+    if (width == kGemmPairWidth && (!g.pairs || (g.batch == 1 && (g.n < 256 || (g.generic && g.k < 512))))) break;
     if (gemm_tile_us(g, width, sms) < gemm_tile_us(g, best, sms)) best = width;
   }
   return best;

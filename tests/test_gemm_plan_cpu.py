@@ -17,6 +17,12 @@ extern "C" double tile_us(long long m, long long n, long long k, int e, int widt
 extern "C" double swap_us(long long m, long long n, long long k, int e, int mx, int r) {
   return gemm_swap_us(GemmProblem{1, m, n, k, e, e, k, false}, mx, r, r == 2 ? 74 : r == 4 ? 33 : 15);
 }
+extern "C" int batched_width(long long b, long long m, long long n, long long k, int row_major, int pairs) {
+  return gemm_best_width(GemmProblem{b, m, n, k, 0, 0, row_major ? 64 : k, row_major != 0, pairs != 0}, 148);
+}
+extern "C" double batched_us(long long b, long long m, long long n, long long k, int row_major, int width) {
+  return gemm_tile_us(GemmProblem{b, m, n, k, 0, 0, row_major ? 64 : k, row_major != 0}, width, 148);
+}
 extern "C" bool swap_in_range(long long m, long long units, int resident) { return gemm_swap_in_range(m, units, resident); }
 extern "C" bool may_split(long long m, long long n, long long k) { return gemm_may_split(m, n, k); }
 extern "C" int best_width(long long b, long long m, long long n, long long k, int e) {
@@ -33,7 +39,7 @@ def plan(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I",
                     os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     lib = ctypes.CDLL(str(lib))
-    lib.tile_us.restype = lib.swap_us.restype = ctypes.c_double
+    lib.tile_us.restype = lib.swap_us.restype = lib.batched_us.restype = ctypes.c_double
     lib.swap_in_range.restype = lib.may_split.restype = ctypes.c_bool
     return lib
 
@@ -73,6 +79,7 @@ def test_weight_streaming_estimates(plan, m, n, k, e, mx, r, us):
         (1, 384, 3000, 640, 0, 128),                                  # rows that are not whole sectors
         (1, 300, 200, 512, 0, 128),                                   # (no pair tile is wider than the result)
         (1, 2048, 2048, 2040, 0, 512),                                # rows off every 32-byte boundary: as few copies as can be
+        (1, 625, 368, 320, 0, 128), (1, 458, 368, 384, 2, 128),       # a chunk of 32 columns that the edge cuts
     ])
 def test_widths(plan, batch, m, n, k, e, width):
     assert plan.best_width(*_ll(batch, m, n, k), e) == width
@@ -92,3 +99,21 @@ def test_weight_streaming_of_many_rows_is_one_wave(plan, m, n, taken):
                                           (1, 63, 4096, True), (5, 127, 4096, True), (5, 128, 4096, False), (3, 64, 1016, True)])
 def test_where_k_may_be_split(plan, m, n, k, split):
     assert plan.may_split(*_ll(m, n, k)) == split
+
+
+# times of products with every width forced (us: 64, 128, 256, 512), at which the estimate of single products chose the slowest but one
+@pytest.mark.parametrize(
+    "b,m,n,k,row_major,us",
+    [
+        (78, 160, 80, 72, 1, (11.9, 5.6, 8.2, 8.1)), (159, 131, 176, 40, 1, (17.4, 11.2, 12.0, 11.1)),
+        (285, 374, 136, 88, 0, (34.5, 22.4, 17.9, 19.8)), (445, 295, 392, 40, 0, (89.8, 50.9, 39.8, 49.8)),
+        (101, 202, 144, 328, 0, (17.4, 12.2, 9.7, 8.9)), (183, 69, 112, 352, 1, (14.3, 7.3, 10.3, 12.4)),
+        (892, 48, 216, 88, 0, (70.7, 19.6, 16.6, 22.4)), (19, 151, 624, 816, 1, (15.4, 11.6, 11.2, 10.5)),
+        (706, 133, 64, 40, 1, (13.3, 17.8, 26.1, 24.8)), (80, 1006, 632, 648, 0, (188.5, 111.7, 97.0, 81.6)),
+    ])
+def test_batched_widths(plan, b, m, n, k, row_major, us):
+    width = plan.batched_width(*_ll(b, m, n, k), row_major, 1)
+    assert us[(64, 128, 256, 512).index(width)] <= 1.1 * min(us)
+    assert plan.batched_width(*_ll(b, m, n, k), row_major, 0) != 512
+    for w, t in zip((64, 128, 256, 512), us):
+        assert abs(plan.batched_us(*_ll(b, m, n, k), row_major, w) / t - 1) < 0.45, w
