@@ -996,14 +996,14 @@ static GemmPlan plan_gemm(const GemmProblem& g, bool bf16, bool streams) {
   return plan;
 }
 
-// How many stages of its operand ring a launch uses, where that is fewer than the kernel has. One k-block per tile: the ring
-// runs ahead of the stores by as many tiles as it has stages, and operands fetched far ahead of use compete with the result
-// for DRAM. 1024 x [512 x 512 x 64], us with 2 / 3 / 4 / 6 stages of 128-wide tiles: 127 / 121 / 135 / 134; 768 x [384 x 384
-// x 64]: 56 / 52 / 59 / 61; 300 x [512 x 512 x 64]: 43 / 37 / 39 / 39. Smaller results are level, K = 32 is (103 / 102), two
-// k-blocks per tile want all six (512 x [512 x 512 x 128]: 93 / 75 / 73 / 70), other widths show nothing clear.
-int operand_ring_limit(long long out_bytes, long long k, int tile_n) {
-  return out_bytes > kStreamedBytes && k <= kBK && tile_n == 128 ? 3 : 64;
-}
+// How many stages of its operand ring a launch uses, where that is fewer than the kernel has. One or two k-blocks per tile: the ring
+// runs ahead of the stores by as many tiles, and operands fetched far ahead of use compete with the result
+// for DRAM. us with 2 / 3 / 4 / 6 stages of 128-wide tiles, 1024 x [512 x 512 x 64]: 127.5 / 120.6 / 135.8 / 135.7; 768 x [384 x 384
+// x 64]: 56 / 53 / 62 / 63; 996 x [258 x 96 x 40]: 22.0 / 22.3 / 22.4 / 24.2; 875 x [392 x 96 x 120]: 40.6 / 35.5 / 35.0 / 39.5;
+// 439 x [216 x 72 x 104], row-major B: 13.9 / 14.6 / 15.7 / 16.7; 893 x [69 x 112 x 72]: 10.7 / 10.3 / 10.6 / 11.2. Other widths gain as
+// well (621 x [300 x 920 x 80], 256 wide: 104 with three, 115 with all four) or are level, as small results are. Two whole k-blocks
+// want all six (512 x [512 x 512 x 128]: 92 / 74.5 / 72 / 70).
+int operand_ring_limit(long long k) { return k < 2 * kBK ? 3 : 64; }
 
 // Split-K plan: how many K-splits a problem gets and the fp32 workspace they need.
 // Splitting pays when the output tiles cannot fill the SMs but K is deep enough to share out.
@@ -1291,7 +1291,7 @@ void gemm_run(const GemmArgs& g_in) {
   const FastDiv by_batch(p.tiles_m * p.tiles_n), by_group(kGroupM * p.tiles_n), by_rest(std::max(1, p.tiles_m % kGroupM));
   p.batch_mul = by_batch.mul, p.batch_shr = by_batch.shr, p.group_mul = by_group.mul, p.group_shr = by_group.shr;
   p.rest_mul = by_rest.mul, p.rest_shr = by_rest.shr;
-  p.ring_limit = operand_ring_limit(g.batch * g.m * g.n * 2, g.k, pair ? 0 : bn);
+  p.ring_limit = operand_ring_limit(g.k);
   const int grid = pair ? 2 * std::min(p.num_units, sm_count() / 2) : std::min(p.num_units, sm_count());
   CUtensorMap td0 = ta;
   p.tma_d0 = 0;
