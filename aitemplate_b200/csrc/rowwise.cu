@@ -10,6 +10,7 @@
 // from cache. All math is fp32.
 #include "common.h"
 #include "epilogue.cuh"
+#include "rules.h"
 
 namespace b200ait {
 
@@ -385,7 +386,8 @@ void layernorm_launch(const LayerNormParams& p, cudaStream_t stream) {
     const int wpb = (vpl <= 4) ? 8 : 4;  // warps per block
     const unsigned grid = static_cast<unsigned>((p.m + wpb - 1) / wpb);
     const int threads = wpb * 32;
-#define B200AIT_LN(V) launch_early(&layernorm_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, true, 1, p)
+    const bool early = blocks_start_early(grid, threads, sm_count(), 2048, vpl <= 1);
+#define B200AIT_LN(V) launch_early(&layernorm_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, early, 1, p)
     if (vpl <= 1)
       B200AIT_LN(1);
     else if (vpl <= 2)
@@ -755,7 +757,8 @@ void softmax_launch(const SoftmaxParams& p, cudaStream_t stream) {
     const int wpb = (vpl <= 4) ? 8 : 4;
     const unsigned grid = static_cast<unsigned>((p.outer + wpb - 1) / wpb);
     const int threads = wpb * 32;
-#define B200AIT_SM(V) launch_early(&softmax_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, true, 1, p)
+    const bool early = blocks_start_early(grid, threads, sm_count(), 2048, vpl <= 1);
+#define B200AIT_SM(V) launch_early(&softmax_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, early, 1, p)
     if (vpl <= 1)
       B200AIT_SM(1);
     else if (vpl <= 2)

@@ -23,6 +23,9 @@ extern "C" long long attn_longest_share(long long items, int q_blocks, int kv_bl
 extern "C" bool gemm_rowdot_short(long long m, long long n, long long k, int whole, int bf16) {
   return b200ait::gemm_rowdot_short(m, n, k, whole != 0, bf16 != 0);
 }
+extern "C" bool blocks_start_early(long long blocks, int threads, int filled, int light, int sms) {
+  return b200ait::blocks_start_early(blocks, threads, sms, filled, light != 0);
+}
 extern "C" bool gemm_rows_output(int n, int tile_n, int residual) { return b200ait::gemm_rows_output(n, tile_n, residual != 0); }
 """
 
@@ -35,7 +38,7 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I",
                     os.path.join(ROOT, "aitemplate_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     lib = ctypes.CDLL(str(lib))
-    for f in (lib.attn_lone, lib.attn_item_per_cta, lib.gemm_rowdot_short, lib.gemm_rows_output):
+    for f in (lib.blocks_start_early, lib.attn_lone, lib.attn_item_per_cta, lib.gemm_rowdot_short, lib.gemm_rows_output):
         f.restype = ctypes.c_bool
     lib.attn_longest_share.restype = ctypes.c_longlong
     return lib
@@ -130,3 +133,16 @@ def test_few_rows_against_short_ones_run_where_they_were_faster(rules, m, n, k, 
     (31, 128, 0, False), (31, 256, 1, False), (33, 128, 1, True), (33, 256, 0, True), (1001, 256, 1, True)])
 def test_narrow_outputs_are_written_by_their_threads(rules, n, tile_n, residual, row_by_row):
     assert rules.gemm_rows_output(n, tile_n, residual) == row_by_row
+
+
+@pytest.mark.parametrize(
+    "blocks,threads,filled,light,early",
+    [
+        # rows: softmax of 365 x 1024, 3521 x 896, 13863 x 512, 520 x 3608 (128 threads), 1455 x 48
+        (46, 256, 2048, 0, True), (441, 256, 2048, 0, False), (1733, 256, 2048, 0, True), (130, 128, 2048, 0, False), (182, 256, 2048, 1, True),
+        # copies and transposes: 8 x [64 x 64], 172 x [112 x 56] twice, 91 x [862 x 112] twice, 11 x [112 x 758]
+        (2, 256, 1024, 0, True), (132, 256, 1024, 0, False), (1074, 256, 1024, 0, True), (264, 256, 1024, 0, False),
+        (74, 256, 2048, 0, True), (75, 256, 2048, 0, False), (592, 256, 1024, 0, True), (591, 256, 1024, 0, False),
+    ])
+def test_a_block_or_a_few_per_sm_wait_for_the_kernel_ahead(rules, blocks, threads, filled, light, early):
+    assert rules.blocks_start_early(ctypes.c_longlong(blocks), threads, filled, light, SMS) == early
