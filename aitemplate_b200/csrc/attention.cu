@@ -84,6 +84,8 @@ constexpr int kBlockN = 64;     // keys per block
 // The reference maximum of a row may lag its true maximum while the row's sum over a block stays below this: P is then at most
 // half of what float16 holds, and as exact as with the true maximum.
 constexpr float kMaxRowSum = 32768.f;
+// ... and in a masked block of narrow heads, while the block's maximum stays within this of it, in log2 units.
+constexpr float kMaskedSlackLog2 = 8.f;
 // Of every eight pairs of scores, this many get their exp2 from the FMA pipe (exp2_poly2 below) instead of the
 // special-function unit, which is the busiest unit of the kernel (64 exp2 per row and key block at 4 lanes per
 // clock and scheduler).
@@ -161,9 +163,9 @@ struct AttnCfg {
 // (attention_scaling_coefs_updater.h:85-165), up to the rounding of P at a different power-of-two-ish scale.
 // NOMASK: no causal mask and a key length that is a multiple of the block: every key block is "plain", and the
 // kernel is compiled without the masked softmax body (the lean variant is measurably faster than a run-time test).
-// SKIP: packed mode with a CTA per work item, where a tile past the end of its sequence ends its CTA before the set-up (64
-// sequences of 128 rows under a bound of 4096, 12 heads: 144 -> 134 us; 8 of 512 .. 4096 rows, 16 heads of 128: 258 -> 254).
-// Compiled apart: the test slowed fixed shares that never take it (768 causal heads x 384 rows of 64: 64.6 -> 66.7 us).
+// SKIP: packed mode with a CTA per work item, where a tile past the end of its sequence ends its CTA before the set-up (8
+// sequences of 512 .. 4096 rows, 16 heads of 128: 236.3 -> 231.6 us). Compiled apart: fixed shares never take it, and in an
+// earlier form of this kernel the test alone slowed them (768 causal heads x 384 rows of 64: 64.6 -> 66.7 us).
 template <int DCH, bool BF16, bool NOMASK, bool LONE, bool SKIP>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
@@ -238,7 +240,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
   };
   if constexpr (SKIP) {
     grid_wait();  // (this early: the sequence lengths are read)
-    // a CTA per item (8 packed causal sequences of 512 .. 4096 rows, 16 heads of 128: 231.6 us, without this end 236.3)
+    // (a CTA per item: this is its only one)
     if (decode_item(blockIdx.x).n_blocks == 0) return;
   }
   const int dsteps = (p.D + 15) / 16;  // k-steps of Q K^T
@@ -560,18 +562,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
             unpack2(lsum2, l0, l1);
             l_blk = l0 + l1;
           };
-          if (j == 0) m_ref = row_max();  // nothing has been accumulated yet
-          exponentials();
-          // A row's reference maximum is raised only when its block has outgrown it: no p exceeds the row's sum, so a sum of
-          // at most kMaxRowSum shows that every P was in range (a sum that is no number, or a score too far up for the
-          // polynomial, counts as out of range). The maximum itself is looked for only then, with the scores read again:
-          // taking it in every block cost 200 of a block's 1250 cycles. The TMEM accesses are warp-wide, so the decision is
-          // too; rows that did not move get alpha = 1.
-          if (j > 0 && __any_sync(0xffffffffu, !(l_blk <= kMaxRowSum) || poly_max > 120.f || m_ref == -INFINITY)) {
-            tmem_ld_32x32b_x32(s_addr, s0);
-            tmem_ld_32x32b_x32(s_addr + 32, s1);
-            tmem_ld_wait();
-            const float m_new = fmaxf(m_ref, row_max());
+          // raises the reference maximum: O and the row sum follow
+          auto raise_reference = [&](float m_new) {
             // O holds blocks 0 .. j-1 once P(j-1) V(j-1) is done; P(j) V(j) cannot start before this thread's arrival on
             // p_full below
             if (!mbar_wait(&kv_empty[(g - 1) % Cfg::kKvStages], ((g - 1) / Cfg::kKvStages) & 1, abort_flag, p.status,
@@ -601,7 +593,37 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_cons
               l_run *= alpha;
             }
             m_ref = m_new;
+          };
+          // The TMEM accesses of raise_reference are warp-wide, so the decision for it is too; rows that did not move get alpha = 1.
+          if constexpr (!kPlain && DCH == 1) {
+            // Narrow heads, a block with a mask: at most the last one or two of an item, and the only one where keys are few. Here the
+            // maximum comes first, in every block, and the reference follows where a row has outgrown it by 2^8; the form below,
+            // in which the exponentials stand twice, was slower by a fifth where every item is such a block (9 x 12 heads x 3326
+            // rows x 26 keys: 37.5 us, 32.5; 40 x 12 x 307 rows x up to 64 keys, 32 channels: 16.1, 14.0). Wide heads lose by it (8 packed
+            // causal sequences, 16 heads of 128: 236 -> 252).
+            const float m_blk = row_max();
+            if (__any_sync(0xffffffffu, m_blk > m_ref + kMaskedSlackLog2)) {
+              const float m_new = fmaxf(m_ref, m_blk);
+              if (j > 0)
+                raise_reference(m_new);
+              else
+                m_ref = m_new;  // nothing has been accumulated yet
+            }
             exponentials();
+          } else {
+            if (j == 0) m_ref = row_max();  // nothing has been accumulated yet
+            exponentials();
+            // A row's reference maximum is raised only when its block has outgrown it: no p exceeds the row's sum, so a sum of
+            // at most kMaxRowSum shows that every P was in range (a sum that is no number, or a score too far up for the
+            // polynomial, counts as out of range). The maximum itself is looked for only then, with the scores read again:
+            // taking it in every block cost 200 of a block's 1250 cycles.
+            if (j > 0 && __any_sync(0xffffffffu, !(l_blk <= kMaxRowSum) || poly_max > 120.f || m_ref == -INFINITY)) {
+              tmem_ld_32x32b_x32(s_addr, s0);
+              tmem_ld_32x32b_x32(s_addr + 32, s1);
+              tmem_ld_wait();
+              raise_reference(fmaxf(m_ref, row_max()));
+              exponentials();
+            }
           }
           // as pairs over the first 32 columns of this S buffer: every score of the row has been used by now
           tmem_st_32x32b_x32(s_addr, packed);

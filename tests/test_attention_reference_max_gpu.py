@@ -41,6 +41,23 @@ def test_one_key_stands_out(rise, d, dtype):
     _check(q.to(dtype), k.to(dtype), v.to(dtype))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("skv", [1, 26, 63, 65, 100, 190])
+@pytest.mark.parametrize("rise", [3.0, 5.5, 5.6, 30.0, 260.0])
+def test_last_block_has_a_mask(rise, skv, d, dtype):
+    """The last block of keys is cut; its last key scores `rise` (nats; 2^8 is 5.55) above the rest in half of the heads."""
+    heads, sq = 12, 300
+    gen = torch.Generator(device="cuda").manual_seed(int(rise * 10) + d + skv)
+    q = torch.randn(2, heads, sq, d, generator=gen, device="cuda") * 0.1
+    k = torch.randn(2, heads, skv, d, generator=gen, device="cuda") * 0.1
+    v = torch.randn(2, heads, skv, d, generator=gen, device="cuda")
+    q[..., 0] = 4.0
+    k[..., 0] = 0.0
+    k[:, ::2, skv - 1, 0] = rise * math.sqrt(d) / 4
+    _check(q.to(dtype), k.to(dtype), v.to(dtype))
+
+
 @pytest.mark.parametrize("d", [64, 96])
 def test_rising_blocks_causal(d):
     gen = torch.Generator(device="cuda").manual_seed(d)
