@@ -771,11 +771,11 @@ void launch_attn_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   opt_in_smem_once(configured, reinterpret_cast<const void*>(kernel), kSmemBytes);
   // early where a CTA walks few items, for the reason given at gemm_starts_early (rules.h): 2 x 8 heads x 4096 rows x 40, 1.7 items
   // a CTA, is worth 2 us behind its projection; in a layer of 4 x 4096 rows with 12 heads, 5.2 a CTA, it cost 11 of 534 us
-  // Where two CTAs fit an SM they pile up on the SMs that fall free first, as blocks_start_early (rules.h) has it of other kernels: 120
-  // items in a layer of 5 x 211 rows 59.3 us, plain 55.6, 96 of 1 x 900 59.7 and 55.6, 144 of 4 x 384 51.3 and 49.5; 288 of 8 x 384
-  // fill the SMs and gain (61.8, plain 62.2), as 36 of 1 x 384 do.
+  // Where two CTAs fit an SM they pile up on the SMs that fall free first, as blocks_start_early (rules.h) has it of other kernels. In
+  // graphs, 120 items in a layer of 5 x 211 rows 59.3 us, plain 55.6, 96 of 1 x 900 59.7 and 55.6, 144 of 4 x 384 51.3 and 49.5; 288 of
+  // 8 x 384 fill the SMs and gain (61.8, plain 62.2), as 36 of 1 x 384 do. (Launched one by one: 64.4, plain 66; 64.5 and 66; 57.5 and 58.5.)
   const bool piles_up = !LONE && 2 * p.num_items > sm_count() && 4ll * p.num_items < 7ll * sm_count();
-  const bool early = 2ll * p.num_items <= 5ll * grid && !piles_up;
+  const bool early = 2ll * p.num_items <= 5ll * grid && !(piles_up && in_capture(stream));
   launch_early(kernel, dim3(grid), kAttnThreads, kSmemBytes, stream, early, 1, tq, tk, tv, p);
 }
 

@@ -78,6 +78,16 @@ void launch_early(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t
   B200AIT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 
+// Is this launch being captured into a graph? (Of a stream that cannot be asked: no.)
+inline bool in_capture(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return status == cudaStreamCaptureStatusActive;
+}
+
 // Runs `fn`, converts any exception into a nonzero status + last-error text.
 template <class F>
 int guarded(const char* where, F&& fn) {

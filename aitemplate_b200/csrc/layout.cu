@@ -17,8 +17,8 @@
 namespace b200ait {
 
 // launch_early for the kernels of this file, 256 threads a block (rules.h)
-static bool starts_early(const dim3& grid) {
-  return blocks_start_early(static_cast<long long>(grid.x) * grid.y * grid.z, 256, sm_count(), 1024);
+static bool starts_early(const dim3& grid, cudaStream_t stream) {
+  return blocks_start_early(static_cast<long long>(grid.x) * grid.y * grid.z, 256, sm_count(), 1024) || !in_capture(stream);
 }
 
 // ------------------------------------------------------------------------- strided 2-D copy batch
@@ -100,7 +100,7 @@ void run_copies(const std::vector<HostCopy>& copies, long long rows, cudaStream_
     const long long per_block = 256 * 8;
     const unsigned gx = static_cast<unsigned>(std::min<long long>((max_vecs + per_block - 1) / per_block, 148 * 16));
     dim3 grid(std::max(gx, 1u), n);
-    const bool early = starts_early(grid);
+    const bool early = starts_early(grid, stream);
     switch (vec) {
       case 16: launch_early(&copy2d_kernel<uint4>, grid, 256, 0, stream, early, 1, b); break;
       case 8: launch_early(&copy2d_kernel<uint2>, grid, 256, 0, stream, early, 1, b); break;
@@ -298,12 +298,12 @@ void permute_run(const void* src, void* dst, const int64_t* in_shape, const int6
           (reinterpret_cast<uintptr_t>(src) & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
         dim3 grid64(static_cast<unsigned>((C + 63) / 64), static_cast<unsigned>((R + 63) / 64), static_cast<unsigned>(B));
         const bool vec = R % 8 == 0 && C % 8 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
-        launch_early(vec ? &transpose16_vec_kernel : &transpose16_kernel, grid64, 256, 0, stream, starts_early(grid64), 1,
+        launch_early(vec ? &transpose16_vec_kernel : &transpose16_kernel, grid64, 256, 0, stream, starts_early(grid64, stream), 1,
                      static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
       } else if (elem_size == 2)
-        launch_early(&transpose_kernel<uint16_t>, grid, 256, 0, stream, starts_early(grid), 1, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
+        launch_early(&transpose_kernel<uint16_t>, grid, 256, 0, stream, starts_early(grid, stream), 1, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, C);
       else
-        launch_early(&transpose_kernel<uint32_t>, grid, 256, 0, stream, starts_early(grid), 1, static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), R, C);
+        launch_early(&transpose_kernel<uint32_t>, grid, 256, 0, stream, starts_early(grid, stream), 1, static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), R, C);
       B200AIT_CUDA_CHECK(cudaGetLastError());
       return;
     }
@@ -334,9 +334,9 @@ void permute_run(const void* src, void* dst, const int64_t* in_shape, const int6
 #define B200AIT_GATHER(V)                                                   \
   do {                                                                      \
     if (small)                                                              \
-      launch_early(&permute_gather_kernel<V, uint32_t>, dim3(grid), 256, 0, stream, starts_early(grid), 1, p); \
+      launch_early(&permute_gather_kernel<V, uint32_t>, dim3(grid), 256, 0, stream, starts_early(grid, stream), 1, p); \
     else                                                                    \
-      launch_early(&permute_gather_kernel<V, long long>, dim3(grid), 256, 0, stream, starts_early(grid), 1, p); \
+      launch_early(&permute_gather_kernel<V, long long>, dim3(grid), 256, 0, stream, starts_early(grid, stream), 1, p); \
   } while (0)
   switch (vec) {
     case 16: B200AIT_GATHER(uint4); break;
@@ -637,9 +637,9 @@ B200AIT_EXPORT int b200ait_elementwise(void* output, const int64_t* out_shape, i
     const long long work = vec ? p.total / 8 : p.total;
     const unsigned grid = static_cast<unsigned>(std::min<long long>((work + 255) / 256, 148 * 32));
     if (dtype == kDTypeBFloat16)
-      launch_early(&elementwise_kernel<true>, dim3(grid), 256, 0, stream, starts_early(grid), 1, p);
+      launch_early(&elementwise_kernel<true>, dim3(grid), 256, 0, stream, starts_early(grid, stream), 1, p);
     else
-      launch_early(&elementwise_kernel<false>, dim3(grid), 256, 0, stream, starts_early(grid), 1, p);
+      launch_early(&elementwise_kernel<false>, dim3(grid), 256, 0, stream, starts_early(grid, stream), 1, p);
     B200AIT_CUDA_CHECK(cudaGetLastError());
   });
 }

@@ -386,7 +386,7 @@ void layernorm_launch(const LayerNormParams& p, cudaStream_t stream) {
     const int wpb = (vpl <= 4) ? 8 : 4;  // warps per block
     const unsigned grid = static_cast<unsigned>((p.m + wpb - 1) / wpb);
     const int threads = wpb * 32;
-    const bool early = blocks_start_early(grid, threads, sm_count(), 2048, vpl <= 1);
+    const bool early = blocks_start_early(grid, threads, sm_count(), 2048, vpl <= 1) || !in_capture(stream);
 #define B200AIT_LN(V) launch_early(&layernorm_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, early, 1, p)
     if (vpl <= 1)
       B200AIT_LN(1);
@@ -757,7 +757,7 @@ void softmax_launch(const SoftmaxParams& p, cudaStream_t stream) {
     const int wpb = (vpl <= 4) ? 8 : 4;
     const unsigned grid = static_cast<unsigned>((p.outer + wpb - 1) / wpb);
     const int threads = wpb * 32;
-    const bool early = blocks_start_early(grid, threads, sm_count(), 2048, vpl <= 1);
+    const bool early = blocks_start_early(grid, threads, sm_count(), 2048, vpl <= 1) || !in_capture(stream);
 #define B200AIT_SM(V) launch_early(&softmax_warp_kernel<V, BF16>, dim3(grid), threads, 0, stream, early, 1, p)
     if (vpl <= 1)
       B200AIT_SM(1);

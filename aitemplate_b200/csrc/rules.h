@@ -248,7 +248,7 @@ inline bool gemm_may_split(long long m, long long n, long long k) {
 inline bool gemm_starts_early(int units, int walkers, bool staged, int sms) {
   return staged ? 2ll * units <= 5ll * walkers : 2ll * units <= sms;  // (unstaged: at most half of the SMs get a tile)
 }
-// The same for kernels of which an SM holds many blocks (rows, copies, permutes, element-wise). They take the SMs in the order in which these
+// The same for kernels of which an SM holds many blocks (rows, copies, permutes, element-wise), in a graph. They take the SMs in the order in which these
 // fall free as well, several blocks to an SM: a grid that would put a block or a few on every SM piles up on the first ones and
 // the others stay idle. Behind one another, us, early -> plain: softmax of 3521 x 896 (441 blocks of 256 threads) 5.65 -> 3.84, layernorm of
 // 2575 x 832 (322) 5.20 -> 3.90, concatenate 2 x [172 x 112 x 56] 4.62 -> 3.38, 11 x [112 x 758] transposed (264) 2.92 -> 2.38. Fewer
@@ -256,6 +256,9 @@ inline bool gemm_starts_early(int units, int walkers, bool staged, int sms) {
 // SMs (13863 x 512: 5.54 -> 5.12; copies from half of the threads on, 1074 blocks: 8.8 -> 8.1). `light`: rows of one 16-byte
 // vector per lane at most, which gain up to four blocks an SM (1455 x 48: 1.90 -> 1.79, 634 x 40: 1.79 -> 1.40). Over 720 calls of
 // seven kinds: early always 0.92 of the plain launch's time and 105 calls slower, by this rule 0.91 and 2, by 4 and 6 %.
+// Outside of a graph a plain launch is dearer, its times come in steps of 2.05 us (4.11, 6.16), and everything starts early: softmax of
+// 1055 x 768 2.7 us, plain 4.1, 64 x [384 x 64] transposed 2.2 and 4.1, layernorm of 2575 x 832 5.6 and 6.2 (but softmax of 3521 x 896 6.5 and
+// 6.2); encoder layers of 5 x 211 and 7 x 150 rows, each run waited for, 82 and 80 us, 87 both with this rule.
 inline bool blocks_start_early(long long blocks, int threads, int sms, int filled_threads, bool light = false) {
   return 2 * blocks <= sms || blocks * threads >= static_cast<long long>(filled_threads) * sms || (light && blocks <= 4ll * sms);
 }
