@@ -1062,6 +1062,15 @@ SplitPlan plan_split_k(const GemmProblem& g, int tile_n, int planned_tile_n, int
   return sp;
 }
 
+// Does this epilogue have instantiations of its own?
+static bool has_own_epilogue(int code) {
+#define B200AIT_OWN(CODE) \
+  if (code == (CODE)) return true;
+  B200AIT_FOR_EACH_FAST_EPILOGUE(B200AIT_OWN)
+#undef B200AIT_OWN
+  return false;
+}
+
 void gemm_run(const GemmArgs& g_in) {
   GemmArgs g = g_in;
   long long c_bdiv = 0, c_bs_hi = 0;
@@ -1196,7 +1205,12 @@ void gemm_run(const GemmArgs& g_in) {
   const bool streams = tma_ok && g.batch == 1 && !g.b_mn && g.num_out == 1 && g.tile_n == 0 && g.split_k == 0;
   // (row-major B: its boxes are not rows of K, and the figures of rules.h do not hold)
   const long long pitch = g.b_mn ? kBK : gemm_copy_row_us(g.lda) > gemm_copy_row_us(g.ldb) ? g.lda : g.ldb;
-  GemmProblem problem{g.batch, g.m, g.n, g.k, 0, 0, pitch, g.b_mn || g.num_out > 1, p.c_bdiv == 0};
+  GemmProblem problem{g.batch, g.m, g.n, g.k, 0, 0, pitch, g.b_mn || g.num_out > 1};
+  // CTA pairs do not write permuted batches, and with an epilogue read from the parameters (two residuals, an activation without an
+  // instantiation of its own) they need K to hide it behind: 829 x 6824 x 216 + add + add 23.6 us, 128-wide tiles 17.9, 1234 x 4768 x 72
+  // mul_tanh 19.7 and 15.0. Over 260 problems with such epilogues, from K = 512 on none is slower than by the rule of whole waves before.
+  const bool own_epilogue = has_own_epilogue(p.epilogue) && (b1 != kBinaryNone || p.alpha == 1.f);
+  problem.pairs = p.c_bdiv == 0 && (g.batch > 1 || own_epilogue || g.k >= 512);
   GemmPlan planned{g.tile_n, nullptr};
   {
     const int code = p.epilogue;

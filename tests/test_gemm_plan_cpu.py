@@ -20,6 +20,9 @@ extern "C" double swap_us(long long m, long long n, long long k, int e, int mx, 
 extern "C" int batched_width(long long b, long long m, long long n, long long k, int row_major, int pairs) {
   return gemm_best_width(GemmProblem{b, m, n, k, 0, 0, row_major ? 64 : k, row_major != 0, pairs != 0}, 148);
 }
+extern "C" int width_of(long long m, long long n, long long k, int e, int pairs) {
+  return gemm_best_width(GemmProblem{1, m, n, k, e, e, k, false, pairs != 0}, 148);
+}
 extern "C" double batched_us(long long b, long long m, long long n, long long k, int row_major, int width) {
   return gemm_tile_us(GemmProblem{b, m, n, k, 0, 0, row_major ? 64 : k, row_major != 0}, width, 148);
 }
@@ -117,3 +120,10 @@ def test_batched_widths(plan, b, m, n, k, row_major, us):
     assert plan.batched_width(*_ll(b, m, n, k), row_major, 0) != 512
     for w, t in zip((64, 128, 256, 512), us):
         assert abs(plan.batched_us(*_ll(b, m, n, k), row_major, w) / t - 1) < 0.45, w
+
+
+@pytest.mark.parametrize("m,n,k,width", [(829, 6824, 216, 128), (2075, 2816, 160, 128), (8144, 768, 200, 128), (3572, 1808, 128, 128)])
+def test_short_k_without_pairs(plan, m, n, k, width):
+    """Epilogues without an instantiation of their own: two residuals, measured with every width forced."""
+    assert plan.width_of(*_ll(m, n, k), 1, 1) == 512
+    assert plan.width_of(*_ll(m, n, k), 1, 0) == width
