@@ -283,14 +283,16 @@ class Executor {
       const TensorInfo& b = plan.tensors[op.operands[1]];
       if (a.dims.empty() || b.dims.size() != 2 || !b.dims[0].is_static || !a.dims.back().is_static) continue;
       // Split-K demand is not monotonic in M (none once the tiles fill the SMs, little at M = 1, most
-      // around M = 128..512), so a dynamic M is sampled: both bounds, then every multiple of 128 up to 2048
-      // and powers of two above, inside [lo, hi].
+      // around M = 128..512), so a dynamic M is sampled: both bounds, 2 and 4 (the last row counts that may split at all against
+      // many columns), then every multiple of 128 up to 2048 and powers of two above, inside [lo, hi].
       int64_t m_lo = 1, m_hi = 1;
       for (size_t i = 0; i + 1 < a.dims.size(); ++i) {
         m_lo *= a.dims[i].is_static ? a.dims[i].v : plan.dims[a.dims[i].v].lo;
         m_hi *= a.dims[i].is_static ? a.dims[i].v : plan.dims[a.dims[i].v].hi;
       }
       std::vector<int64_t> ms{m_lo, m_hi};
+      for (int64_t m : {2, 4})
+        if (m > m_lo && m < m_hi) ms.push_back(m);
       for (int64_t m = 128; m < m_hi && m <= 2048; m += 128)
         if (m > m_lo) ms.push_back(m);
       for (int64_t m = 4096; m < m_hi; m *= 2)

@@ -625,6 +625,12 @@ def test_dynamic_m_reserves_split_k_workspace_for_interior_sizes(workdir):
     wide.DLL.AITemplateTrackingAllocatorGetNumBytes(wide.allocator_handle, ctypes.byref(nbytes))
     assert nbytes.value < need, (nbytes.value, need)
     wide.close()
+    deep = kernels._scratch_bytes(0, 4, 512, 24576, 0, 0)  # four rows against rows of W that shared memory does not hold
+    assert deep > 0 and kernels._scratch_bytes(0, 1, 512, 24576, 0, 0) == 0
+    few = compile_model(_relu_layer(512, 24576), detect_target(), workdir, "dyn_m_few_rows", allocator_kind=AITemplateAllocatorKind.TRACKING)
+    few.DLL.AITemplateTrackingAllocatorGetNumBytes(few.allocator_handle, ctypes.byref(nbytes))
+    assert nbytes.value >= deep, (nbytes.value, deep)
+    few.close()
     w, b = _rand((n, k), 2, 0.02), _rand((n,), 3)
     for m in (1, 256, 300, 4096):
         x = _rand((m, k), 10 + m)
