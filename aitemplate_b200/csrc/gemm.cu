@@ -963,7 +963,10 @@ int choose_tile_n(const GemmProblem& g) {
   // 4096: 141 against 125 (the wide tile fetches a quarter fewer operand rows, and TMA pays per row). So the narrow
   // tile is taken for one full k-block, and for two only on a narrow result.
   // K = 32 (whole 64-byte rows): 102 us at 1024 x [512 x 512] against 125.
-  if (g.n >= 128 && g.batch * g.m * g.n * 2 > kStreamedBytes && (g.k <= 32 || g.k == kBK || (g.k > kBK && g.k <= 2 * kBK && g.n <= 512)))
+  // Between one and two k-blocks, where the rows are not whole sectors, the estimates are ahead (us, narrow tile, 256-wide, pairs): 695 x
+  // [497 x 352 x 104] 101 / 102 / 75, 600 x [400 x 400 x 72] 98 / 83 / 64, 300 x [512 x 512 x 80] 44 / 38 / 41; 512 x [512 x 512 x 96] 66 / 66 / 71.
+  if (g.n >= 128 && g.batch * g.m * g.n * 2 > kStreamedBytes &&
+      (g.k <= 32 || g.k == kBK || (g.k > kBK && g.k <= 2 * kBK && g.k % 32 == 0 && g.n <= 512)))
     return 128;
   return gemm_best_width(g, sm_count());
 }
@@ -1001,9 +1004,10 @@ static GemmPlan plan_gemm(const GemmProblem& g, bool bf16, bool streams) {
 // for DRAM. us with 2 / 3 / 4 / 6 stages of 128-wide tiles, 1024 x [512 x 512 x 64]: 127.5 / 120.6 / 135.8 / 135.7; 768 x [384 x 384
 // x 64]: 56 / 53 / 62 / 63; 996 x [258 x 96 x 40]: 22.0 / 22.3 / 22.4 / 24.2; 875 x [392 x 96 x 120]: 40.6 / 35.5 / 35.0 / 39.5;
 // 439 x [216 x 72 x 104], row-major B: 13.9 / 14.6 / 15.7 / 16.7; 893 x [69 x 112 x 72]: 10.7 / 10.3 / 10.6 / 11.2. Other widths gain as
-// well (621 x [300 x 920 x 80], 256 wide: 104 with three, 115 with all four) or are level, as small results are. Two whole k-blocks
-// want all six (512 x [512 x 512 x 128]: 92 / 74.5 / 72 / 70).
-int operand_ring_limit(long long k) { return k < 2 * kBK ? 3 : 64; }
+// well (621 x [300 x 920 x 80], 256 wide: 104 with three, 111 with all four) or are level, as small results are. Two whole k-blocks
+// want all six (512 x [512 x 512 x 128]: 92 / 74.5 / 72 / 70), and so does K = 96, whose rows are whole sectors (512 x [512 x 512 x 96]:
+// 73 with three, 66).
+int operand_ring_limit(long long k) { return k <= kBK || (k < 2 * kBK && k % 32 != 0) ? 3 : 64; }
 
 // Split-K plan: how many K-splits a problem gets and the fp32 workspace they need.
 // Splitting pays when the output tiles cannot fill the SMs but K is deep enough to share out.
